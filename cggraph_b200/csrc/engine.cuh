@@ -116,21 +116,26 @@ struct cgb_graph {
     // PageRank layout: vertices relabelled by out-degree bucket (stable; zero
     // out-degree last), in-edge CSC over the new ids, out-degree by new id
     uint32_t* pr_rank = nullptr;     // old id -> new id
-    uint32_t* pr_off = nullptr;      // V+1
-    uint32_t* pr_src = nullptr;      // E
+    uint32_t* pr_off = nullptr;      // V+1 (while the layout is built)
+    uint32_t* pr_src = nullptr;      // E (likewise)
     uint32_t* pr_outdeg = nullptr;   // V
-    uint2* pr_chunks = nullptr;      // hub rows: (row, first edge) of each kPrChunk-edge chunk
-    uint32_t* pr_chunk_base = nullptr;  // per hub row: index of its first chunk (n_pr_huge + 1)
-    uint32_t* pr_huge_rows = nullptr;   // hub rows (new ids)
-    double* pr_part = nullptr;       // per-chunk partial sums
-    uint32_t n_pr_huge = 0, n_pr_chunks = 0;
-    // sliced ELL (32 rows per slice) of the non-hub rows: edge j of row
-    // 32*s + l at col[slice_ptr[s] + 32*j + l]; padding points at vertex V,
-    // whose contribution is kept at 0
-    uint64_t* pr_slice_ptr = nullptr;   // nslices + 1
-    uint32_t* pr_slice_len = nullptr;   // nslices
+    uint32_t n_src = 0;              // vertices with out-edges: the new ids [0, n_src)
+    // long rows (pr_long_row in-edges or more), cut into segments of at most
+    // pr_seg edges; segments are numbered row by row
+    uint32_t pr_long_row = 0, pr_seg = 0;
+    uint32_t n_pr_long = 0, n_pr_seg = 0, n_pr_hubs = 0;
+    uint32_t* pr_long_rows = nullptr;   // n_pr_long rows (new ids)
+    uint32_t* pr_seg_base = nullptr;    // first segment of each long row (n_pr_long + 1)
+    uint32_t* pr_hubs = nullptr;        // long rows (indices) of more than kPrHubSegs segments
+    uint32_t* pr_seg_id = nullptr;      // segments in slice order
+    double* pr_part = nullptr;          // sum of each segment
+    uint32_t* pr_long_bm = nullptr;     // bitmap of the long rows
+    // sliced ELL (32 rows per slice) of the segments, then of the other rows:
+    // edge j of row 32*s + l at col[slice_ptr[s] + 32*j + l]; padding points
+    // at vertex V, whose contribution is kept at 0
+    uint64_t* pr_slice_ptr = nullptr;   // slices + 1
+    uint32_t* pr_slice_len = nullptr;   // slices
     uint32_t* pr_col = nullptr;
-    uint32_t* pr_hub_bm = nullptr;      // bitmap of hub rows
     uint64_t pr_sell_size = 0;
     bool pr_ready = false;
 
@@ -159,10 +164,6 @@ struct cgb_graph {
 
     cudaEvent_t ev_start = nullptr, ev_stop = nullptr;
     cudaEvent_t ev_iter[2] = {nullptr, nullptr};
-    // PageRank hub chunks run beside the sliced pull: a second stream forked
-    // from and joined to `stream` by these events (created on first use)
-    cudaStream_t aux_stream = nullptr;
-    cudaEvent_t ev_fork = nullptr, ev_join = nullptr;
     std::vector<cudaEvent_t> kev;     // per-launch timing events (pairs)
     size_t kev_used = 0;
     std::vector<int> kev_class;
@@ -183,8 +184,7 @@ struct cgb_graph {
 
 namespace cgb {
 
-constexpr uint32_t kPrHuge = 4096;   // PageRank rows split into chunks across CTAs
-constexpr uint32_t kPrChunk = 4096;  // edges per PageRank hub chunk
+constexpr uint32_t kPrHubSegs = 128;  // PageRank: rows of more segments are added up by a CTA each
 constexpr uint32_t kHugeDeg = 16384; // push: hubs split across CTAs
 constexpr uint32_t kCtaDeg = 1024;   // push: CTA-per-vertex tier
 constexpr uint32_t kHugeChunk = 4096;

@@ -515,14 +515,6 @@ __global__ void k_sum_u32(uint32_t n, const uint32_t* __restrict__ a, unsigned l
     if (lane_id() == 0 && s) atomicAdd(out, s);
 }
 
-__global__ void k_collect_heavy_rows(uint32_t V, const uint32_t* __restrict__ in_off, uint32_t th, uint32_t* rows,
-                                     uint32_t* n)
-{
-    for (uint32_t v = blockIdx.x * blockDim.x + threadIdx.x; v < V; v += gridDim.x * blockDim.x) {
-        if (in_off[v + 1] - in_off[v] >= th) rows[atomicAdd(n, 1u)] = v;
-    }
-}
-
 __global__ void k_count_reached(uint32_t V, const uint32_t* __restrict__ value, const uint32_t* __restrict__ off,
                                 DevCounters* ctr)
 {
@@ -1121,15 +1113,24 @@ __global__ void k_pr_bucket(uint32_t V, const uint32_t* __restrict__ off, const 
     }
 }
 
-// Slice lengths of the sliced ELL: the longest non-hub row of each slice.
-__global__ void k_sell_len(uint32_t V, const uint32_t* __restrict__ off, uint32_t hub, uint32_t* len, uint64_t* width)
+// Slice lengths of the sliced ELL: the longest segment of each segment
+// slice, then the longest row of each row slice that is not a long one.
+__global__ void k_sell_len(uint32_t V, const uint32_t* __restrict__ off, uint32_t long_row, uint32_t n_seg,
+                           const uint32_t* __restrict__ seg_id, const uint2* __restrict__ seg, uint32_t* len,
+                           uint64_t* width)
 {
-    const uint32_t nslices = (V + 31) / 32;
+    const uint32_t seg_slices = (n_seg + 31) / 32, nslices = seg_slices + (V + 31) / 32;
     for (uint32_t s = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; s < nslices;
          s += (gridDim.x * blockDim.x) >> 5) {
-        const uint32_t r = s * 32 + lane_id();
-        uint32_t d = r < V ? off[r + 1] - off[r] : 0;
-        if (d >= hub) d = 0;
+        uint32_t d = 0;
+        if (s < seg_slices) {
+            const uint32_t i = s * 32 + lane_id();
+            if (i < n_seg) d = seg[seg_id[i]].y;
+        } else {
+            const uint32_t r = (s - seg_slices) * 32 + lane_id();
+            if (r < V) d = off[r + 1] - off[r];
+            if (d >= long_row) d = 0;
+        }
         d = warp_max(d);
         if (lane_id() == 0) {
             len[s] = d;
@@ -1148,12 +1149,58 @@ __global__ void k_pr_rank(uint32_t V, const uint32_t* __restrict__ order, const 
     }
 }
 
-__global__ void k_row_bounds(const uint32_t* __restrict__ rows, uint32_t n, const uint32_t* __restrict__ off,
-                             uint32_t* lohi)
+constexpr int kPrSegBits = 9;  // segment lengths are below 2^9
+
+// *n_src = number of vertices with out-edges (outdeg is zero from there on).
+__global__ void k_pr_count_src(uint32_t V, const uint32_t* __restrict__ outdeg, uint32_t* n_src)
 {
-    for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
-        lohi[i] = off[rows[i]];
-        lohi[n + i] = off[rows[i] + 1];
+    for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < V; i += gridDim.x * blockDim.x)
+        if (outdeg[i] && (i + 1 == V || !outdeg[i + 1])) *n_src = i + 1;
+}
+
+// Segments of every long row (0 for the others), and 1 for the long rows;
+// entry V of both is 0.
+__global__ void k_pr_row_segs(uint32_t V, const uint32_t* __restrict__ off, uint32_t long_row, uint32_t seg,
+                              uint32_t* n, uint32_t* is_long)
+{
+    for (uint32_t r = blockIdx.x * blockDim.x + threadIdx.x; r <= V; r += gridDim.x * blockDim.x) {
+        const uint32_t len = r < V ? off[r + 1] - off[r] : 0;
+        n[r] = len >= long_row ? (len + seg - 1) / seg : 0;
+        is_long[r] = len >= long_row ? 1u : 0u;
+    }
+}
+
+// Long-row list and segment table from the exclusive sums of k_pr_row_segs;
+// a warp takes 32 rows and writes each row's segments together.  A segment's
+// sort key is the 4096-source window of its first source, then its length
+// (longest first, so that slices hold segments of one length).
+__global__ void k_pr_fill_segs(uint32_t V, const uint32_t* __restrict__ off, const uint32_t* __restrict__ src,
+                               const uint32_t* __restrict__ base, const uint32_t* __restrict__ long_idx,
+                               uint32_t hub_segs, uint32_t* rows, uint32_t* seg_base, uint32_t* hubs, uint32_t* n_hubs,
+                               uint32_t* key, uint32_t* id, uint2* seg)
+{
+    const uint32_t lane = lane_id();
+    for (uint32_t r0 = ((blockIdx.x * blockDim.x + threadIdx.x) >> 5) * 32; r0 < V;
+         r0 += ((gridDim.x * blockDim.x) >> 5) * 32) {
+        const uint32_t r = r0 + lane;
+        const uint32_t b = r < V ? base[r] : 0, n = r < V ? base[r + 1] - b : 0;
+        if (n) {
+            const uint32_t i = long_idx[r];
+            rows[i] = r;
+            seg_base[i] = b;
+            if (n > hub_segs) hubs[atomicAdd(n_hubs, 1u)] = i;
+        }
+        for (uint32_t todo = __ballot_sync(0xffffffffu, n != 0); todo; todo &= todo - 1) {
+            const uint32_t l = __ffs(todo) - 1;
+            const uint32_t rb = __shfl_sync(0xffffffffu, b, l), rn = __shfl_sync(0xffffffffu, n, l);
+            const uint32_t beg = off[r0 + l], len = off[r0 + l + 1] - beg;
+            for (uint32_t c = lane; c < rn; c += 32) {
+                const uint32_t e0 = (uint32_t)((uint64_t)len * c / rn), e1 = (uint32_t)((uint64_t)len * (c + 1) / rn);
+                key[rb + c] = (src[beg + e0] >> 12 << kPrSegBits) | ((1u << kPrSegBits) - 1 - (e1 - e0));
+                id[rb + c] = rb + c;
+                seg[rb + c] = make_uint2(beg + e0, e1 - e0);
+            }
+        }
     }
 }
 
@@ -1183,47 +1230,55 @@ struct PrEdgesF {
     }
 };
 
-// SELL columns from the relabelled CSC, one warp per 32-row slice, lane i
-// on row 32s + i: column j of the slice is 32 consecutive words, so every
-// store is coalesced, and each lane reads its own row front to back.
-// Positions past a row's end hold the padding target V; hub rows (hub
-// in-edges or more) are summed from pr_src instead, keep only padding here
-// and are marked in hub_bm (one word per slice, written whole).
+// SELL columns from the relabelled CSC, one warp per 32-row slice, lane i on
+// segment or row 32s + i: column j of the slice is 32 consecutive words, so
+// every store is coalesced, and each lane reads its own row front to back.
+// Positions past a row's end hold the padding target V; long rows are summed
+// as segments, keep only padding in their row slices and are marked in
+// long_bm (one word per row slice, written whole).
 __global__ void k_sell_fill(uint32_t V, const uint32_t* __restrict__ pr_off, const uint32_t* __restrict__ pr_src,
                             const uint64_t* __restrict__ slice_ptr, const uint32_t* __restrict__ slice_len,
-                            uint32_t hub, uint32_t* col, uint32_t* hub_bm)
+                            uint32_t long_row, uint32_t n_seg, const uint32_t* __restrict__ seg_id,
+                            const uint2* __restrict__ seg, uint32_t* col, uint32_t* long_bm)
 {
-    const uint32_t nslices = (V + 31) / 32;
+    const uint32_t seg_slices = (n_seg + 31) / 32, nslices = seg_slices + (V + 31) / 32;
     const uint32_t lane = lane_id();
     for (uint32_t sl = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; sl < nslices;
          sl += (gridDim.x * blockDim.x) >> 5) {
-        const uint32_t r = sl * 32 + lane;
-        const uint32_t beg = r < V ? pr_off[r] : 0;
-        const uint32_t len = r < V ? pr_off[r + 1] - beg : 0;
-        const bool is_hub = len >= hub;
-        const uint32_t hubs = __ballot_sync(0xffffffffu, is_hub);
-        if (lane == 0) hub_bm[sl] = hubs;
-        const uint32_t use = is_hub ? 0 : len;
+        uint32_t beg = 0, use = 0;
+        if (sl < seg_slices) {
+            const uint32_t i = sl * 32 + lane;
+            if (i < n_seg) {
+                const uint2 g = seg[seg_id[i]];
+                beg = g.x;
+                use = g.y;
+            }
+        } else {
+            const uint32_t r = (sl - seg_slices) * 32 + lane;
+            beg = r < V ? pr_off[r] : 0;
+            const uint32_t len = r < V ? pr_off[r + 1] - beg : 0;
+            const uint32_t longs = __ballot_sync(0xffffffffu, len >= long_row);
+            if (lane == 0) long_bm[sl - seg_slices] = longs;
+            use = len >= long_row ? 0 : len;
+        }
         uint32_t* c = col + slice_ptr[sl] + lane;
         const uint32_t width = slice_len[sl];
         for (uint32_t j = 0; j < width; j++) c[32ull * j] = j < use ? pr_src[beg + j] : V;
     }
 }
 
-// Sliced ELL layout of the non-hub rows (slice lengths, offsets and the
-// column array); k_sell_fill writes the columns and their padding.
-static void build_sell(cgb_graph* g)
+// Sliced ELL layout of the segments and the rows that are not long.
+static void build_sell(cgb_graph* g, const uint2* seg)
 {
     const uint32_t V = g->V;
-    const uint32_t nslices = (V + 31) / 32;
+    const uint32_t nslices = div_up(g->n_pr_seg, 32) + div_up(V, 32);
     g->pr_slice_len = dalloc<uint32_t>(nslices, g->stream);
     g->pr_slice_ptr = dalloc<uint64_t>((size_t)nslices + 1, g->stream);
-    g->pr_hub_bm = dalloc<uint32_t>(g->words(), g->stream);
-    CGB_CUDA_TRY(cudaMemsetAsync(g->pr_hub_bm, 0, (size_t)g->words() * 4, g->stream));
+    g->pr_long_bm = dalloc<uint32_t>(g->words(), g->stream);
     uint64_t* width = dalloc<uint64_t>((size_t)nslices + 1, g->stream);
     CGB_CUDA_TRY(cudaMemsetAsync(width + nslices, 0, 8, g->stream));
     k_sell_len<<<grid_for((uint64_t)nslices * 32, kBlock, num_sms() * 8), kBlock, 0, g->stream>>>(
-        V, g->pr_off, kPrHuge, g->pr_slice_len, width);
+        V, g->pr_off, g->pr_long_row, g->n_pr_seg, g->pr_seg_id, seg, g->pr_slice_len, width);
     size_t tb = 0;
     CGB_CUDA_TRY(cub::DeviceScan::ExclusiveSum(nullptr, tb, width, g->pr_slice_ptr, (uint64_t)nslices + 1, g->stream));
     void* temp = dalloc<char>(tb, g->stream);
@@ -1238,6 +1293,25 @@ static void build_sell(cgb_graph* g)
     CGB_CUDA_TRY(err);
     g->pr_sell_size = total;
     g->pr_col = dalloc<uint32_t>(total, g->stream);
+    k_sell_fill<<<grid_for((uint64_t)nslices * 32, kBlock, num_sms() * 16), kBlock, 0, g->stream>>>(
+        V, g->pr_off, g->pr_src, g->pr_slice_ptr, g->pr_slice_len, g->pr_long_row, g->n_pr_seg, g->pr_seg_id, seg,
+        g->pr_col, g->pr_long_bm);
+}
+
+// In-edges from which a PageRank row is long, and edges per segment, by the
+// graph's edges (a rule of the graph alone, so that results do not depend on
+// the device).  A row's lane is a chain of up to long_row gathers; a small
+// graph's iteration lasts as long as its longest chain, a large one pays 8
+// bytes written and read per segment.  20 iterations, ms, (long_row, seg):
+//                      (64, 32)  (128, 64)  (256, 128)
+//   RMAT-16              0.23      0.29       0.29
+//   RMAT-24             14.2      13.6       13.8
+//   Chung-Lu 126 M       6.4       6.3        6.5
+static void pr_row_sizes(uint32_t E, uint32_t& long_row, uint32_t& seg)
+{
+    const bool small = E < (1u << 22);
+    long_row = small ? 64 : 128;
+    seg = small ? 32 : 64;
 }
 
 // Builds the PageRank layout (see cgb_graph): the relabel keeps every
@@ -1316,58 +1390,69 @@ void ensure_pr(cgb_graph* g)
             CGB_CUDA_TRY(cudaMemsetAsync(g->pr_off, 0, ((size_t)V + 1) * 4, g->stream));
         }
         dfree(src_off, g->stream);
-        build_sell(g);
-        if (E)
-            k_sell_fill<<<grid_for((uint64_t)(V + 31) / 32 * 32, kBlock, num_sms() * 16), kBlock, 0, g->stream>>>(
-                V, g->pr_off, g->pr_src, g->pr_slice_ptr, g->pr_slice_len, kPrHuge, g->pr_col, g->pr_hub_bm);
         CGB_CUDA_TRY(cudaStreamSynchronize(g->stream));
         dfree(order, g->stream);
     }
-    // 3. hub rows and their chunk table (host-built; few rows)
+    // 3. the long rows' segments, and the sliced ELL
     {
-        uint32_t* n = dalloc<uint32_t>(1, g->stream);
-        uint32_t* rows = dalloc<uint32_t>(V, g->stream);
-        CGB_CUDA_TRY(cudaMemsetAsync(n, 0, sizeof(uint32_t), g->stream));
-        k_collect_heavy_rows<<<grid_for(V, kBlock, num_sms() * 8), kBlock, 0, g->stream>>>(V, g->pr_off, kPrHuge, rows,
-                                                                                        n);
-        PinnedArray<uint32_t> hn(1);
-        CGB_CUDA_TRY(cudaMemcpyAsync(hn.data(), n, 4, cudaMemcpyDeviceToHost, g->stream));
+        pr_row_sizes(E, g->pr_long_row, g->pr_seg);
+        uint32_t* n = dalloc<uint32_t>((size_t)V + 1, g->stream);
+        uint32_t* is_long = dalloc<uint32_t>((size_t)V + 1, g->stream);
+        uint32_t* base = dalloc<uint32_t>((size_t)V + 1, g->stream);
+        uint32_t* long_idx = dalloc<uint32_t>((size_t)V + 1, g->stream);
+        uint32_t* cnt = dalloc<uint32_t>(2, g->stream);  // vertices with out-edges, hub rows
+        CGB_CUDA_TRY(cudaMemsetAsync(cnt, 0, 2 * sizeof(uint32_t), g->stream));
+        k_pr_count_src<<<grid_for(V, kBlock, num_sms() * 8), kBlock, 0, g->stream>>>(V, g->pr_outdeg, cnt);
+        k_pr_row_segs<<<grid_for((uint64_t)V + 1, kBlock, num_sms() * 8), kBlock, 0, g->stream>>>(
+            V, g->pr_off, g->pr_long_row, g->pr_seg, n, is_long);
+        exclusive_sum_u32(g, n, base, (uint64_t)V + 1);
+        exclusive_sum_u32(g, is_long, long_idx, (uint64_t)V + 1);
+        PinnedArray<uint32_t> h(4);
+        CGB_CUDA_TRY(cudaMemcpyAsync(h.data(), cnt, 4, cudaMemcpyDeviceToHost, g->stream));
+        CGB_CUDA_TRY(cudaMemcpyAsync(h.data() + 1, base + V, 4, cudaMemcpyDeviceToHost, g->stream));
+        CGB_CUDA_TRY(cudaMemcpyAsync(h.data() + 2, long_idx + V, 4, cudaMemcpyDeviceToHost, g->stream));
         CGB_CUDA_TRY(cudaStreamSynchronize(g->stream));
-        const uint32_t h = hn[0];
         dfree(n, g->stream);
-        // pinned staging for every transfer here (see pinned_acquire, h2d_small)
-        PinnedArray<uint32_t> hrows(std::max<uint32_t>(h, 1)), lohi_h(2 * (size_t)std::max<uint32_t>(h, 1));
-        if (h) {
-            CGB_CUDA_TRY(cudaMemcpyAsync(hrows.data(), rows, h * 4ull, cudaMemcpyDeviceToHost, g->stream));
-            CGB_CUDA_TRY(cudaStreamSynchronize(g->stream));
-            std::sort(hrows.data(), hrows.data() + h);
-            h2d_small(rows, hrows.data(), h * 4ull, g->stream);
-            uint32_t* lohi = dalloc<uint32_t>(2ull * h, g->stream);
-            k_row_bounds<<<grid_for(h, kBlock, num_sms() * 8), kBlock, 0, g->stream>>>(rows, h, g->pr_off, lohi);
-            CGB_CUDA_TRY(cudaMemcpyAsync(lohi_h.data(), lohi, 2ull * h * 4, cudaMemcpyDeviceToHost, g->stream));
-            CGB_CUDA_TRY(cudaStreamSynchronize(g->stream));
-            dfree(lohi, g->stream);
+        dfree(is_long, g->stream);
+        g->n_src = h[0];
+        g->n_pr_seg = h[1];
+        g->n_pr_long = h[2];
+        uint2* seg = nullptr;
+        h[3] = 0;
+        if (g->n_pr_seg) {
+            const uint32_t ns = g->n_pr_seg;
+            g->pr_long_rows = dalloc<uint32_t>(g->n_pr_long, g->stream);
+            g->pr_seg_base = dalloc<uint32_t>((size_t)g->n_pr_long + 1, g->stream);
+            g->pr_hubs = dalloc<uint32_t>(ns / kPrHubSegs + 1, g->stream);
+            g->pr_seg_id = dalloc<uint32_t>(ns, g->stream);
+            g->pr_part = dalloc<double>(ns, g->stream);
+            seg = dalloc<uint2>(ns, g->stream);
+            uint32_t* key = dalloc<uint32_t>(ns, g->stream);
+            uint32_t* key2 = dalloc<uint32_t>(ns, g->stream);
+            uint32_t* id = dalloc<uint32_t>(ns, g->stream);
+            k_pr_fill_segs<<<grid_for(V, kBlock, num_sms() * 8), kBlock, 0, g->stream>>>(
+                V, g->pr_off, g->pr_src, base, long_idx, kPrHubSegs, g->pr_long_rows, g->pr_seg_base, g->pr_hubs,
+                cnt + 1, key, id, seg);
+            CGB_CUDA_TRY(cudaMemcpyAsync(g->pr_seg_base + g->n_pr_long, base + V, 4, cudaMemcpyDeviceToDevice,
+                                         g->stream));
+            CGB_CUDA_TRY(cudaMemcpyAsync(h.data() + 3, cnt + 1, 4, cudaMemcpyDeviceToHost, g->stream));
+            stable_sort_u32(g, key, key2, id, g->pr_seg_id, ns,
+                            std::min<int>(32, (int)bits_for((V >> 12) + 1) + kPrSegBits));
+            dfree(key, g->stream);
+            dfree(key2, g->stream);
+            dfree(id, g->stream);
         }
-        uint64_t nch = 0;
-        for (uint32_t i = 0; i < h; i++) nch += (lohi_h[h + i] - lohi_h[i] + kPrChunk - 1) / kPrChunk;
-        PinnedArray<uint2> chunks(std::max<uint64_t>(nch, 1));
-        PinnedArray<uint32_t> base(h + 1);
-        uint32_t c = 0;
-        for (uint32_t i = 0; i < h; i++) {
-            base[i] = c;
-            for (uint32_t e = lohi_h[i]; e < lohi_h[h + i]; e += kPrChunk) chunks[c++] = make_uint2(hrows[i], e);
-        }
-        base[h] = c;
-        g->n_pr_huge = h;
-        g->n_pr_chunks = c;
-        g->pr_huge_rows = rows;
-        g->pr_chunk_base = dalloc<uint32_t>(h + 1, g->stream);
-        h2d_small(g->pr_chunk_base, base.data(), (h + 1) * 4ull, g->stream);
-        g->pr_chunks = dalloc<uint2>(c, g->stream);
-        if (c)
-            h2d_small(g->pr_chunks, chunks.data(), (size_t)c * sizeof(uint2), g->stream);
-        CGB_CUDA_TRY(cudaStreamSynchronize(g->stream));  // the pinned tables go out of scope
-        g->pr_part = dalloc<double>(c, g->stream);
+        build_sell(g, seg);
+        CGB_CUDA_TRY(cudaStreamSynchronize(g->stream));
+        g->n_pr_hubs = h[3];
+        // the columns hold every source: the relabelled CSC is not read again
+        dfree(g->pr_src, g->stream);
+        dfree(g->pr_off, g->stream);
+        g->pr_src = g->pr_off = nullptr;
+        dfree(base, g->stream);
+        dfree(long_idx, g->stream);
+        dfree(cnt, g->stream);
+        dfree(seg, g->stream);
     }
     g->pr_ready = true;
 }
@@ -1510,19 +1595,18 @@ void graph_free(cgb_graph* g)
     if (g->pending_w) dfree(g->pending_w, g->stream);
     free_msbfs(g);
     free_mssp(g);
-    void* ptrs[] = {g->off, g->dst, g->w, g->pr_huge_rows, g->pr_rank, g->pr_off, g->pr_src, g->pr_outdeg,
-                    g->pr_chunks, g->pr_chunk_base, g->pr_part, g->pr_slice_ptr, g->pr_slice_len, g->pr_col,
-                    g->pr_hub_bm, g->value, g->pr[0], g->pr[1], g->contrib[0],
+    void* ptrs[] = {g->off, g->dst, g->w, g->pr_rank, g->pr_off, g->pr_src, g->pr_outdeg,
+                    g->pr_long_rows, g->pr_seg_base, g->pr_hubs, g->pr_seg_id, g->pr_part, g->pr_slice_ptr,
+                    g->pr_slice_len, g->pr_col, g->pr_long_bm, g->value, g->pr[0], g->pr[1], g->contrib[0],
                     g->contrib[1], g->q[0], g->q[1], g->chunk_q, g->visited, g->front_bm, g->stamp, g->sample,
                     g->aux_bm, g->persist, g->ctr};
     for (void* p : ptrs) dfree(p, g->stream);
     pinned_small_free(g->h_ctr);
     pinned_release(g->h_persist, g->h_persist_bytes);
     for (cudaEvent_t e : g->kev) cudaEventDestroy(e);
-    cudaEvent_t evs[] = {g->ev_start, g->ev_stop, g->ev_iter[0], g->ev_iter[1], g->ev_fork, g->ev_join};
+    cudaEvent_t evs[] = {g->ev_start, g->ev_stop, g->ev_iter[0], g->ev_iter[1]};
     for (cudaEvent_t e : evs)
         if (e) cudaEventDestroy(e);
-    if (g->aux_stream) cudaStreamDestroy(g->aux_stream);
     if (g->own_stream) cudaStreamDestroy(g->own_stream);
     delete g;
 }
