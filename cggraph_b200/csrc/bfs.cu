@@ -112,18 +112,12 @@ struct BfsTdOp {
     }
 };
 
-__global__ void k_bfs_init(uint32_t V, uint32_t* level, uint32_t* visited, uint32_t words)
+__global__ void k_bfs_init(uint32_t V, uint32_t* level, uint32_t* visited, uint32_t words, uint32_t root, uint32_t* q0)
 {
-    const uint32_t stride = gridDim.x * blockDim.x;
-    for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < V; i += stride) level[i] = kValueMax;
-    for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < words; i += stride) visited[i] = 0;
-}
-
-__global__ void k_bfs_root(uint32_t* level, uint32_t* visited, uint32_t root, uint32_t* q0)
-{
-    level[root] = 0;
-    visited[root >> 5] = 1u << (root & 31u);
-    q0[0] = root;
+    const uint32_t stride = gridDim.x * blockDim.x, i0 = blockIdx.x * blockDim.x + threadIdx.x;
+    for (uint32_t i = i0; i < V; i += stride) level[i] = i == root ? 0 : kValueMax;
+    for (uint32_t i = i0; i < words; i += stride) visited[i] = i == root >> 5 ? 1u << (root & 31u) : 0;
+    if (i0 == 0) q0[0] = root;
 }
 
 // Queue -> frontier bitmap (bitmap cleared beforehand).
@@ -215,6 +209,10 @@ static void reset_level_counters(cgb_graph* g, int out)
     k_level_reset<<<1, 1, 0, g->stream>>>(g->ctr, out);
 }
 
+// A graph of at most this many edges runs in the cluster from start to end,
+// all levels pushed.
+constexpr uint32_t kClusterWholeEdges = 1u << 20;
+
 void run_bfs(cgb_graph* g, uint32_t root, const cgb_options& o)
 {
     ensure_frontier(g);
@@ -230,22 +228,30 @@ void run_bfs(cgb_graph* g, uint32_t root, const cgb_options& o)
     PolicySamples* collect = want_pull && !force_pull ? g->collect : nullptr;
     Policy* pol = (o.schedule == CGB_SCHED_LEARNED && want_pull && !force_pull) ? policy_for(g) : nullptr;
 
-    PinnedArray<uint32_t> host_root_deg(2);  // pinned: see pinned_acquire
-    CGB_CUDA_TRY(cudaMemcpyAsync(host_root_deg.data(), g->off + root, 2 * sizeof(uint32_t), cudaMemcpyDeviceToHost,
-                                 g->stream));
-    CGB_CUDA_TRY(cudaStreamSynchronize(g->stream));
+    // device-resident levels for small frontiers (not while collecting
+    // samples, which time each level's variants on the host)
+    const bool persist_ok = !tracing && !collect && o.schedule != CGB_SCHED_FIXED;
+    const bool cluster_ok =
+        persist_ok && g->tune.persist_enter > 0 && g->tune.cluster_enter > 0 && cluster_loop_ctas() > 0;
+    // the root's out-degree, which the cluster loop finds out for itself
+    uint64_t scout = 0;
+    if (!cluster_ok) {
+        PinnedArray<uint32_t> host_root_deg(2);  // pinned: see pinned_acquire
+        CGB_CUDA_TRY(cudaMemcpyAsync(host_root_deg.data(), g->off + root, 2 * sizeof(uint32_t),
+                                     cudaMemcpyDeviceToHost, g->stream));
+        CGB_CUDA_TRY(cudaStreamSynchronize(g->stream));
+        scout = host_root_deg[1] - host_root_deg[0];
+    }
     CGB_CUDA_TRY(cudaEventRecord(g->ev_start, g->stream));
     if (timing) ktimer_begin(g, CGB_K_INIT);
     ++g->stats.launches;
-    k_bfs_init<<<num_sms() * 4, kBlock, 0, g->stream>>>(V, g->value, g->visited, words);
-    ++g->stats.launches;
-    k_bfs_root<<<1, 1, 0, g->stream>>>(g->value, g->visited, root, g->q[0]);
+    k_bfs_init<<<grid_for(V, kBlock, num_sms() * 4), kBlock, 0, g->stream>>>(V, g->value, g->visited, words, root,
+                                                                          g->q[0]);
     if (timing) ktimer_end(g);
 
     uint32_t cur = 0;  // queue holding the current frontier
     uint64_t nf = (root < g->nz) ? 1 : 0;
     uint64_t prev_nf = 0;
-    uint64_t scout = host_root_deg[1] - host_root_deg[0];
     int64_t edges_to_check = (int64_t)g->E;
     uint32_t maxdeg = (uint32_t)scout;
     uint64_t visited_cnt = 1;
@@ -303,33 +309,43 @@ void run_bfs(cgb_graph* g, uint32_t root, const cgb_options& o)
         return in;
     };
 
-    // device-resident levels for small frontiers (not while collecting
-    // samples, which time each level's variants on the host)
-    const bool persist_ok = !tracing && !collect && o.schedule != CGB_SCHED_FIXED;
     while (nf > 0) {
         CGB_REQUIRE(iters < max_iters, CGB_ETIMEOUT, "BFS iteration budget exhausted");
         // ----- direction decision
         const bool heur = bottom_up ? (awake >= old_awake) || ((double)awake > (double)V / beta)
                                     : (double)scout > (double)edges_to_check / alpha;
-        // small frontiers far from the switch point: run levels on the device
-        if (persist_ok && !heur && nf <= g->tune.persist_enter && maxdeg < g->tune.persist_deg &&
-            (double)scout * alpha * 4.0 <= (double)edges_to_check) {
+        // small frontiers far from the switch point: run levels on the device;
+        // a small graph's whole run, in the cluster
+        const bool whole = g->E <= kClusterWholeEdges && !bottom_up;
+        const bool far_off = !heur && (double)scout * alpha * 4.0 <= (double)edges_to_check;
+        const uint64_t scout_exit = (uint64_t)std::max(0.0, (double)edges_to_check / alpha / 4.0);
+        const uint32_t max_levels = (uint32_t)std::min<uint64_t>(max_iters - iters, 1u << 20);
+        const bool use_cluster = cluster_ok && nf <= std::min(g->tune.cluster_enter, g->tune.persist_enter) &&
+                                 (whole || (far_off && scout <= kClusterEnterEdges));
+        const bool use_grid = persist_ok && !use_cluster && far_off && nf <= g->tune.persist_enter &&
+                              maxdeg < g->tune.persist_deg && scout > 0;
+        if (use_cluster || use_grid) {
             if (timing) ktimer_begin(g, CGB_K_PUSH);
-            const unsigned long long scout_exit = (unsigned long long)((double)edges_to_check / alpha / 4.0);
             const PersistResult r =
-                bfs_persistent(g, cur, (uint32_t)nf, scout, maxdeg, level, g->tune.persist_enter, scout_exit, g->tune.persist_deg,
-                               (uint32_t)std::min<uint64_t>(max_iters - iters, 1u << 20));
+                use_cluster ? bfs_cluster(g, cur, (uint32_t)nf, level,
+                                          whole ? 0xFFFFFFFFu
+                                                : std::min(g->tune.persist_enter, 2 * g->tune.cluster_enter),
+                                          whole ? 0xFFFFFFFFu
+                                                : (uint32_t)std::min<uint64_t>(scout_exit, kClusterExitEdges),
+                                          max_levels)
+                            : bfs_persistent(g, cur, (uint32_t)nf, scout, maxdeg, level, g->tune.persist_enter,
+                                             scout_exit, g->tune.persist_deg, max_levels);
             if (timing) ktimer_end(g);
+            scout = r.scout;
+            maxdeg = r.max_deg;
             if (r.levels > 0) {
-                visited_cnt += r.added - nf + r.nf;
+                visited_cnt += r.found;
                 edges_to_check -= (int64_t)r.scouts;
                 iters += r.levels;
                 level += r.levels;
                 g->stats.pushes_td += r.levels;
                 prev_nf = nf;
                 nf = r.nf;
-                scout = r.scout;
-                maxdeg = r.max_deg;
                 cur = r.cur;
                 bottom_up = false;
                 have_policy_out = false;

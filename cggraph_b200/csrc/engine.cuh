@@ -156,6 +156,7 @@ struct cgb_graph {
     uint32_t* sample = nullptr;           // CC sampling buffer
     uint32_t* aux_bm = nullptr;           // 3 bitmaps: device-resident SSSP near dedup
     void* persist = nullptr;              // state of the device-resident loops
+    void* cluster = nullptr;              // state of the cluster loops
     cgb::MsBuffers* ms = nullptr;         // multi-root BFS masks
     cgb::MsspBuffers* mssp = nullptr;     // multi-root SSSP distances and masks
 

@@ -1599,7 +1599,7 @@ void graph_free(cgb_graph* g)
                     g->pr_long_rows, g->pr_seg_base, g->pr_hubs, g->pr_seg_id, g->pr_part, g->pr_slice_ptr,
                     g->pr_slice_len, g->pr_col, g->pr_long_bm, g->value, g->pr[0], g->pr[1], g->contrib[0],
                     g->contrib[1], g->q[0], g->q[1], g->chunk_q, g->visited, g->front_bm, g->stamp, g->sample,
-                    g->aux_bm, g->persist, g->ctr};
+                    g->aux_bm, g->persist, g->cluster, g->ctr};
     for (void* p : ptrs) dfree(p, g->stream);
     pinned_small_free(g->h_ctr);
     pinned_release(g->h_persist, g->h_persist_bytes);

@@ -22,7 +22,12 @@
 namespace cgb {
 
 constexpr uint32_t kBarrierSpins = 1u << 22;  // mostly x ~64 ns: gives up after ~0.3 s
-constexpr int kClusterThreads = 1024;          // threads per CTA of the cluster level loop
+
+// The cluster loops (cluster.cu) take frontiers of at most
+// cgb_tuning.cluster_enter vertices and kClusterEnterEdges out-edges, and
+// return once a frontier exceeds twice the entry size or kClusterExitEdges:
+// beyond, 16 SMs take longer than a host round trip over all of them.
+constexpr uint32_t kClusterEnterEdges = 1u << 17, kClusterExitEdges = 1u << 18;
 
 // Host-visible state of a device-resident loop.
 struct PersistState {
@@ -60,12 +65,26 @@ struct PersistBlock {
     PersistSssp sx;
 };
 
+// What a cluster loop reports on exit.
+struct ClusterState {
+    uint32_t qlen;      // frontier vertices left in the global queue
+    uint32_t status;    // 1 = a barrier gave up, 2 = queue overflow
+    uint32_t levels;    // levels (rounds) run
+    uint32_t max_deg;   // longest list of the frontier
+    uint32_t found;     // BFS: vertices reached; SSSP: list pieces expanded
+    uint32_t far_left;  // SSSP: vertices left in the far bitmap
+    unsigned long long scout;   // out-edges of the frontier
+    unsigned long long scouts;  // BFS: sum of the out-edges of the levels run
+    unsigned long long thr, bucket_lo;
+};
+
 struct PersistResult {
     uint32_t levels = 0;       // levels (rounds) run
     uint32_t cur = 0;          // queue index holding the frontier on exit
     uint32_t nf = 0;           // frontier size on exit
-    uint32_t max_deg = 0;      // its max out-degree (BFS)
-    unsigned long long scout = 0;   // its out-edges (BFS)
+    uint32_t max_deg = 0;      // its max out-degree
+    uint32_t found = 0;        // vertices reached (BFS)
+    unsigned long long scout = 0;   // its out-edges (BFS, cluster loops)
     unsigned long long added = 0;   // sum of the frontier sizes run
     unsigned long long scouts = 0;  // sum of their out-edges (BFS)
 };
@@ -81,6 +100,14 @@ struct PersistResult {
 PersistResult bfs_persistent(cgb_graph* g, uint32_t cur, uint32_t nf, unsigned long long scout, uint32_t max_deg,
                              uint32_t level, uint32_t nf_exit, unsigned long long scout_exit, uint32_t deg_exit,
                              uint32_t max_levels);
+
+// The cluster loops.  CTAs of a cluster on the current device (0: the device
+// schedules none, and the loops must not be called).
+uint32_t cluster_loop_ctas();
+// BFS levels from q[cur][0, nf) (level `level`): bounds as bfs_persistent.
+// Vertices without out-edges are reached but not part of a frontier.
+PersistResult bfs_cluster(cgb_graph* g, uint32_t cur, uint32_t nf, uint32_t level, uint32_t nf_exit,
+                          uint32_t scout_exit, uint32_t max_levels);
 
 // One cooperative launch of k_bfs_persistent with no exit threshold, from
 // the state's qlen[0] roots in q[0] (graph batches).
@@ -105,6 +132,12 @@ struct SsspTail {
 SsspTail sssp_device_tail(cgb_graph* g, uint32_t cur, uint32_t nf, uint32_t max_deg, uint64_t thr, uint32_t nfar,
                           uint64_t bucket_lo, uint32_t* far_bm, uint32_t delta, uint32_t nf_exit, uint32_t deg_exit,
                           uint32_t max_rounds);
+
+// The same in a cluster loop, which leaves when a frontier exceeds nf_exit
+// vertices or scout_exit out-edges (r.scout: the out-edges of the frontier it
+// returns).
+SsspTail sssp_cluster(cgb_graph* g, uint32_t cur, uint32_t nf, uint64_t thr, uint32_t nfar, uint64_t bucket_lo,
+                      uint32_t* far_bm, uint32_t delta, uint32_t nf_exit, uint32_t scout_exit, uint32_t max_rounds);
 
 // Warp-aggregated append into a device-resident loop's queue (every lane
 // calls it); past `cap` the loop's status records an overflow.

@@ -306,17 +306,12 @@ __global__ void k_sssp_split_reset(DevCounters* ctr, int out)
     ctr->max_deg = 0;
 }
 
-__global__ void k_sssp_init(uint32_t V, uint32_t* dist, uint32_t* far_bm, uint32_t words)
+__global__ void k_sssp_init(uint32_t V, uint32_t* dist, uint32_t* far_bm, uint32_t words, uint32_t root, uint32_t* q0)
 {
-    const uint32_t stride = gridDim.x * blockDim.x;
-    for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < V; i += stride) dist[i] = kValueMax;
-    for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < words; i += stride) far_bm[i] = 0;
-}
-
-__global__ void k_sssp_root(uint32_t* dist, uint32_t root, uint32_t* q0)
-{
-    dist[root] = 0;
-    q0[0] = root;
+    const uint32_t stride = gridDim.x * blockDim.x, i0 = blockIdx.x * blockDim.x + threadIdx.x;
+    for (uint32_t i = i0; i < V; i += stride) dist[i] = i == root ? 0 : kValueMax;
+    for (uint32_t i = i0; i < words; i += stride) far_bm[i] = 0;
+    if (i0 == 0) q0[0] = root;
 }
 
 // Splits the far bitmap at [lo, hi) (see file comment).  A warp takes 32
@@ -410,9 +405,8 @@ static void sssp_loop(cgb_graph* g, uint32_t root, uint32_t delta, const cgb_opt
     CGB_CUDA_TRY(cudaEventRecord(g->ev_start, g->stream));
     if (timing) ktimer_begin(g, CGB_K_INIT);
     ++g->stats.launches;
-    k_sssp_init<<<num_sms() * 4, kBlock, 0, g->stream>>>(V, g->value, far_bm, words);
-    ++g->stats.launches;
-    k_sssp_root<<<1, 1, 0, g->stream>>>(g->value, root, g->q[0]);
+    k_sssp_init<<<grid_for(V, kBlock, num_sms() * 4), kBlock, 0, g->stream>>>(V, g->value, far_bm, words, root,
+                                                                           g->q[0]);
     if (timing) ktimer_end(g);
 
     int cur = 0;
@@ -429,27 +423,43 @@ static void sssp_loop(cgb_graph* g, uint32_t root, uint32_t delta, const cgb_opt
     uint64_t iters = 0;
     uint64_t expanded = 0;
 
-    // The device-resident tail (persist.cuh): once the near queue holds at
-    // most persist_enter vertices whose lists are all shorter than
-    // persist_deg edges, near rounds and bucket splits run in one cooperative
-    // launch until the run ends or a frontier outgrows those bounds (then
-    // the host loop's binned kernels take over again).  It keeps the current
-    // delta for the buckets it splits.  Graphs with lists of persist_deg
-    // edges or more (power-law graphs) stay on the host loop: their tail
-    // rounds hold medium-degree lists that the tail's one-warp-per-list
-    // expansion walks slowly, and their frontiers outgrow the tail's bounds
-    // bucket after bucket (measured on RMAT-24: 6.9 against 5.2 ms a run).
-    // Under the learned schedule the tail waits for the first bucket
-    // boundary, so that the network picks the delta it keeps.
-    const bool tail_fits = !tracing && o.schedule != CGB_SCHED_FIXED && g->tune.persist_enter > 0 &&
-                           g->max_degree < g->tune.persist_deg;
-    const bool tail_ok = tail_fits && !collect;
+    // Device-resident rounds (persist.cuh).  The cluster loop takes near
+    // queues of at most cluster_enter vertices and kClusterEnterEdges
+    // out-edges on any graph (a hub's list is spread over the cluster).  The
+    // grid loop takes up to persist_enter vertices on graphs whose lists are
+    // all shorter than persist_deg edges; on others (power-law graphs) its
+    // one-warp-per-list expansion walks medium lists slowly, and frontiers
+    // outgrow its bounds bucket after bucket (RMAT-24: 6.9 against 5.2 ms a
+    // run).  Both run near rounds and bucket splits until the run ends or a
+    // frontier outgrows their bounds (then the rounds below take over again),
+    // and keep the current delta for the buckets they split.  Under the
+    // learned schedule they wait for the first bucket boundary, so that the
+    // network picks that delta.
+    const bool tail_allowed = !tracing && o.schedule != CGB_SCHED_FIXED && g->tune.persist_enter > 0;
+    const bool grid_fits = tail_allowed && g->max_degree < g->tune.persist_deg;
+    const bool cluster_fits = tail_allowed && g->tune.cluster_enter > 0 && cluster_loop_ctas() > 0;
     bool tail_delta_chosen = pol == nullptr;
+    enum { kNoTail, kClusterTail, kGridTail };
+    auto tail_kind = [&]() {
+        if (cluster_fits && nnear <= std::min(g->tune.cluster_enter, g->tune.persist_enter) &&
+            near_edges <= kClusterEnterEdges)
+            return kClusterTail;
+        if (grid_fits && nnear <= g->tune.persist_enter && near_maxdeg < g->tune.persist_deg) return kGridTail;
+        return kNoTail;
+    };
+    // Runs the loop that takes the near queue (or, when it is empty, the next
+    // split); false if none does or it ran no round.
     auto device_tail = [&]() -> bool {
+        const int kind = tail_kind();
+        if (kind == kNoTail) return false;
+        const uint32_t max_rounds = (uint32_t)std::min<uint64_t>(max_iters - iters, 1u << 30);
         if (timing) ktimer_begin(g, CGB_K_PUSH);
-        const SsspTail t = sssp_device_tail(g, cur, (uint32_t)nnear, near_maxdeg, thr, (uint32_t)nfar, bucket_lo,
-                                            far_bm, delta, g->tune.persist_enter, g->tune.persist_deg,
-                                            (uint32_t)std::min<uint64_t>(max_iters - iters, 1u << 30));
+        const SsspTail t =
+            kind == kClusterTail
+                ? sssp_cluster(g, cur, (uint32_t)nnear, thr, (uint32_t)nfar, bucket_lo, far_bm, delta,
+                               std::min(g->tune.persist_enter, 2 * g->tune.cluster_enter), kClusterExitEdges, max_rounds)
+                : sssp_device_tail(g, cur, (uint32_t)nnear, near_maxdeg, thr, (uint32_t)nfar, bucket_lo, far_bm, delta,
+                                   g->tune.persist_enter, g->tune.persist_deg, max_rounds);
         if (timing) ktimer_end(g);
         iters += t.r.levels;
         expanded += t.r.added;
@@ -458,7 +468,7 @@ static void sssp_loop(cgb_graph* g, uint32_t root, uint32_t delta, const cgb_opt
         nfar = t.nfar;
         thr = t.thr;
         bucket_lo = t.bucket_lo;
-        near_edges = 0;  // not counted by the device-resident rounds: push next
+        near_edges = t.r.scout;  // 0 (unknown) from the grid loop: push next
         cur = (int)t.r.cur;
         return t.r.levels > 0;
     };
@@ -523,9 +533,9 @@ static void sssp_loop(cgb_graph* g, uint32_t root, uint32_t delta, const cgb_opt
     auto near_rounds = [&]() {
         while (nnear > 0) {
             CGB_REQUIRE(iters < max_iters, CGB_ETIMEOUT, "SSSP iteration budget exhausted");
-            if (tail_ok && tail_delta_chosen && nnear <= g->tune.persist_enter && near_maxdeg < g->tune.persist_deg) {
+            if (!collect && tail_delta_chosen && device_tail()) {
                 have_round_out = false;
-                if (device_tail()) continue;
+                continue;
             }
             const int out = cur ^ 1;
             // heuristic: pull when the near set's out-edges times alpha exceed the graph's
@@ -705,12 +715,11 @@ static void sssp_loop(cgb_graph* g, uint32_t root, uint32_t delta, const cgb_opt
                 // device-resident tail included (it changes what a round costs)
                 delta = dk;
                 do {
-                    if (tail_fits) {
-                        near_maxdeg = 0;
-                        if (device_tail()) {
-                            near_rounds();
-                            continue;
-                        }
+                    near_maxdeg = 0;
+                    near_edges = 0;
+                    if (device_tail()) {
+                        near_rounds();
+                        continue;
                     }
                     advance(dk);
                     near_rounds();
@@ -747,9 +756,10 @@ static void sssp_loop(cgb_graph* g, uint32_t root, uint32_t delta, const cgb_opt
         }
         delta = d;
         tail_delta_chosen = true;
-        if (tail_ok) {
+        if (!collect) {
             // the next bucket's split, and what follows, on the device
             near_maxdeg = 0;
+            near_edges = 0;
             if (device_tail()) {
                 near_rounds();
                 continue;

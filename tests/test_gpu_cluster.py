@@ -1,0 +1,63 @@
+"""The cluster frontier loops: pieces of long lists, queues that spill, small and large exits."""
+import numpy as np
+import pytest
+
+import cggraph_b200 as cg
+from oracle import oracle as O
+
+BFS, SSSP = int(cg.Algorithm_type.BFS), int(cg.Algorithm_type.SSSP)
+
+
+def csr(V, src, dst, seed, wmax):
+    key = np.unique(src.astype(np.int64) * V + dst)
+    src, dst = key // V, (key % V).astype(np.uint32)
+    off = np.zeros(V + 1, np.uint32)
+    off[1:] = np.cumsum(np.bincount(src, minlength=V))
+    w = np.random.default_rng(seed).integers(1, wmax + 1, dst.size).astype(np.uint32)
+    return off, dst, w
+
+
+def star(leaves, degree):
+    """Vertex 0 to every leaf, each leaf to `degree` others: the second frontier has leaves * ceil(degree / 8) pieces."""
+    V = leaves + 1
+    i = np.repeat(np.arange(1, V), degree)
+    j = (i * 7 + 13 * np.tile(np.arange(degree), leaves)) % V
+    return V, np.concatenate([np.zeros(leaves, np.int64), i]), np.concatenate([np.arange(1, V), j])
+
+
+def ladder(degrees):
+    """A chain whose i-th vertex also points at degrees[i] leaves: lists around the piece size, thin frontiers."""
+    n = len(degrees)
+    src, dst, nxt = [], [], n
+    for i, d in enumerate(degrees):
+        if i + 1 < n:
+            src.append(i), dst.append(i + 1)
+        src += [i] * d
+        dst += range(nxt, nxt + d)
+        nxt += d
+    return nxt, np.array(src), np.array(dst)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("graph", [
+    lambda: star(100_000, 9),     # the queues spill
+    lambda: star(65_000, 8),      # one piece a leaf, a queue nearly full
+    lambda: star(3, 2),
+    lambda: ladder([0, 1, 6, 7, 8, 9, 14, 15, 16, 17, 30, 31, 32, 33, 255, 256, 257, 5000] * 3),
+])
+@pytest.mark.parametrize("wmax,delta", [(1, 0), (1000, 0), (1000, 50)])
+def test_cluster_loops(graph, wmax, delta):
+    V, src, dst = graph()
+    keep = src != dst
+    off, dst, w = csr(V, src[keep], dst[keep], 5, wmax)
+    # the tail without out-edges is left out of the frontiers
+    nz = int(np.nonzero(np.diff(off.astype(np.int64)))[0].max()) + 1
+    with cg.Graph.from_csr(off, dst, w, noZeroOutDegreeNum=nz) as g:
+        np.testing.assert_array_equal(g.run(BFS, 0)[0], O.bfs(off, dst, 0))
+        opts = cg.make_options(sssp_delta=delta)
+        np.testing.assert_array_equal(g.run(SSSP, 0, opts)[0], O.sssp(off, dst, w, 0))
+        # again after the other algorithm used the shared scratch, from a vertex inside
+        np.testing.assert_array_equal(g.run(BFS, 1)[0], O.bfs(off, dst, 1))
+        np.testing.assert_array_equal(g.run(SSSP, 1, opts)[0], O.sssp(off, dst, w, 1))
+    with cg.Graph.from_csr(off, dst) as g:  # unit weights
+        np.testing.assert_array_equal(g.run(SSSP, 0)[0], O.bfs(off, dst, 0))
