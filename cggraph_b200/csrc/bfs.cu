@@ -37,6 +37,7 @@ struct BfsTdOp {
     uint32_t* qlen;
     uint32_t cap;
     DevCounters* ctr;
+    uint32_t t_edges = 0, t_maxdeg = 0;  // of the vertices this thread claimed
     static constexpr int kBatch = 4;  // edge slots per lane visited together (push.cuh)
 
     __device__ __forceinline__ bool load(uint32_t v, uint32_t& s, uint32_t& d, uint32_t& m) const
@@ -47,7 +48,7 @@ struct BfsTdOp {
         return true;
     }
     template <int N>
-    __device__ __forceinline__ void edges(const bool (&valid)[N], const uint32_t (&e)[N], const uint32_t (&)[N]) const
+    __device__ __forceinline__ void edges(const bool (&valid)[N], const uint32_t (&e)[N], const uint32_t (&)[N])
     {
         uint32_t d[N], word[N], bit[N], lo[N], hi[N];
         bool win[N], enq[N];
@@ -70,27 +71,14 @@ struct BfsTdOp {
             lo[i] = enq[i] ? off[d[i]] : 0u;
             hi[i] = enq[i] ? off[d[i] + 1] : 0u;
         }
-        warp_append_n<N>(enq, d, qout, qlen, cap, &ctr->overflow);
-        bool any = false;
+        stage_append_n<N>(enq, d, qout, qlen, cap, &ctr->overflow);
 #pragma unroll
-        for (int i = 0; i < N; i++) any |= enq[i];
-        if (__any_sync(0xffffffffu, any)) {
-            unsigned long long sum = 0;
-            uint32_t mx = 0;
-#pragma unroll
-            for (int i = 0; i < N; i++) {
-                sum += hi[i] - lo[i];
-                mx = max(mx, hi[i] - lo[i]);
-            }
-            sum = warp_sum(sum);
-            mx = warp_max(mx);
-            if (lane_id() == 0) {
-                atomicAdd(&s_td_medges, sum);
-                atomicMax(&s_td_maxdeg, mx);
-            }
+        for (int i = 0; i < N; i++) {
+            t_edges += hi[i] - lo[i];
+            t_maxdeg = max(t_maxdeg, hi[i] - lo[i]);
         }
     }
-    __device__ __forceinline__ void edge(bool valid, uint32_t e, uint32_t m) const
+    __device__ __forceinline__ void edge(bool valid, uint32_t e, uint32_t m)
     {
         const bool v[1] = {valid};
         const uint32_t ee[1] = {e}, mm[1] = {m};
@@ -98,6 +86,7 @@ struct BfsTdOp {
     }
     __device__ __forceinline__ void block_begin() const
     {
+        stage_begin();
         if (threadIdx.x == 0) {
             s_td_medges = 0;
             s_td_maxdeg = 0;
@@ -105,6 +94,13 @@ struct BfsTdOp {
     }
     __device__ __forceinline__ void block_end() const
     {
+        const uint32_t sum = __reduce_add_sync(0xffffffffu, t_edges);  // at most E < 2^32
+        const uint32_t mx = __reduce_max_sync(0xffffffffu, t_maxdeg);
+        if (lane_id() == 0 && sum) {
+            atomicAdd(&s_td_medges, (unsigned long long)sum);
+            atomicMax(&s_td_maxdeg, mx);
+        }
+        stage_end(qout, qlen, cap, &ctr->overflow);  // a CTA barrier is inside
         if (threadIdx.x == 0 && s_td_medges) {
             atomicAdd(&ctr->medges, s_td_medges);
             atomicMax(&ctr->max_deg, s_td_maxdeg);
@@ -130,12 +126,13 @@ __global__ void k_q2bm(const uint32_t* __restrict__ q, uint32_t n, uint32_t* bm)
 }
 
 // One bottom-up level.  Reads front (current frontier bitmap), writes
-// next (all words, so it needs no clearing) and the next queue.  Each lane
-// scans its vertex's in-list four entries at a time: four source loads,
-// then their four frontier words, are in flight together, and the scan
-// stops after the group that holds a parent.  A CTA takes kBlock / 32
-// consecutive bitmap words per step (one per warp) and appends the step's
-// found vertices with one atomic.
+// next (all words, so it needs no clearing) and the next queue.  A warp takes
+// one bitmap word per step, and warps share nothing between steps (finds are
+// staged, push.cuh): what bounds the level is each warp's chain of dependent
+// loads, so no warp waits for another's.  Each lane scans its vertex's
+// in-list four entries at a time: four source loads, then their four
+// frontier words, are in flight together, and the scan stops after the group
+// that holds a parent.
 __global__ void __launch_bounds__(kBlock) k_bfs_bu(uint32_t V, const uint32_t* __restrict__ in_off,
                                                    const uint32_t* __restrict__ in_src,
                                                    const uint32_t* __restrict__ off, uint32_t* level,
@@ -143,18 +140,18 @@ __global__ void __launch_bounds__(kBlock) k_bfs_bu(uint32_t V, const uint32_t* _
                                                    uint32_t* next, uint32_t next_level, uint32_t nz, uint32_t* qout,
                                                    uint32_t* qlen, uint32_t cap, DevCounters* ctr)
 {
-    const uint32_t words = (V + 31) / 32;
-    constexpr uint32_t kWarps = kBlock / 32;
-    unsigned long long medges = 0;
-    uint32_t found_cnt = 0, mx = 0;
-    for (uint32_t base = blockIdx.x * kWarps; base < words; base += gridDim.x * kWarps) {
-        const uint32_t wi = base + (threadIdx.x >> 5);
-        const uint32_t v = wi * 32 + lane_id();
-        bool enq = false;
-        if (wi < words) {  // uniform across the warp
-            const uint32_t vis = visited[wi];
+    const uint32_t words = (V + 31) / 32, lane = lane_id();
+    const uint32_t warps = gridDim.x * (kBlock / 32);
+    uint32_t medges = 0, found_cnt = 0, mx = 0;
+    stage_begin();
+    __syncthreads();
+    for (uint32_t wi = blockIdx.x * (kBlock / 32) + (threadIdx.x >> 5); wi < words; wi += warps) {
+        const uint32_t v = wi * 32 + lane;
+        const uint32_t vis = visited[wi];
+        uint32_t fm = 0;
+        if (vis != 0xFFFFFFFFu) {
             bool found = false;
-            if (v < V && !((vis >> lane_id()) & 1u)) {
+            if (v < V && !((vis >> lane) & 1u)) {
                 const uint32_t e1 = in_off[v + 1];
                 for (uint32_t e = in_off[v]; e < e1 && !found; e += 4) {
                     uint32_t u[4], f[4];
@@ -166,28 +163,30 @@ __global__ void __launch_bounds__(kBlock) k_bfs_bu(uint32_t V, const uint32_t* _
                     for (int k = 0; k < 4; k++) found |= (f[k] & 1u) != 0;
                 }
             }
-            const uint32_t fm = __ballot_sync(0xffffffffu, found);
-            if (found) level[v] = next_level;
-            if (lane_id() == 0) {
-                next[wi] = fm;
-                if (fm) visited[wi] = vis | fm;
+            fm = __ballot_sync(0xffffffffu, found);
+            if (fm) {
+                if (found) level[v] = next_level;
+                const bool enq[1] = {found && v < nz};
+                const uint32_t deg = enq[0] ? off[v + 1] - off[v] : 0;
+                medges += deg;
+                found_cnt += enq[0];
+                mx = max(mx, deg);
+                const uint32_t it[1] = {v};
+                stage_append_n<1>(enq, it, qout, qlen, cap, &ctr->overflow);
             }
-            enq = found && v < nz;
-            uint32_t deg = 0;
-            if (enq) deg = off[v + 1] - off[v];
-            medges += deg;
-            found_cnt += enq;
-            mx = max(mx, deg);
         }
-        const bool p[1] = {enq};
-        const uint32_t it[1] = {v};
-        block_append_n<1>(p, it, qout, qlen, cap, &ctr->overflow);
+        if (lane == 0) {
+            next[wi] = fm;
+            if (fm) visited[wi] = vis | fm;
+        }
     }
-    medges = warp_sum(medges);
-    found_cnt = warp_sum(found_cnt);
-    mx = warp_max(mx);
-    if (lane_id() == 0 && found_cnt) {
-        atomicAdd(&ctr->medges, medges);
+    __syncthreads();
+    stage_end(qout, qlen, cap, &ctr->overflow);
+    const uint32_t warp_edges = __reduce_add_sync(0xffffffffu, medges);  // at most E < 2^32
+    found_cnt = __reduce_add_sync(0xffffffffu, found_cnt);
+    mx = __reduce_max_sync(0xffffffffu, mx);
+    if (lane == 0 && found_cnt) {
+        atomicAdd(&ctr->medges, (unsigned long long)warp_edges);
         atomicAdd(&ctr->found, found_cnt);
         atomicMax(&ctr->max_deg, mx);
     }

@@ -147,7 +147,8 @@ __device__ __forceinline__ void cl_push(ClShared& s, uint32_t buf, const bool (&
             const uint32_t bn = __shfl_sync(0xffffffffu, n[i], l), bp = __shfl_sync(0xffffffffu, pos, l);
             const uint32_t bv = __shfl_sync(0xffffffffu, v[i], l), bs = __shfl_sync(0xffffffffu, start[i], l);
             const uint32_t bd = __shfl_sync(0xffffffffu, deg[i], l);
-            for (uint32_t k = lane; k < bn; k += 32) put(bp + k, k, bv, bs, bd, bp + bn <= kClQueue);
+            const uint32_t room = bp < kClQueue ? min(bn, kClQueue - bp) : 0;
+            for (uint32_t k = lane; k < room; k += 32) put(bp + k, k, bv, bs, bd, bp + bn <= kClQueue);
         }
         pos += n[i];
     }

@@ -515,22 +515,51 @@ __global__ void k_sum_u32(uint32_t n, const uint32_t* __restrict__ a, unsigned l
     if (lane_id() == 0 && s) atomicAdd(out, s);
 }
 
-__global__ void k_count_reached(uint32_t V, const uint32_t* __restrict__ value, const uint32_t* __restrict__ off,
-                                DevCounters* ctr)
+// Vertices with a value and their out-edges; a thread takes 4 vertices with
+// one 16-byte load of each array (and the offset that follows).
+__global__ void __launch_bounds__(kBlock) k_count_reached(uint32_t V, const uint32_t* __restrict__ value,
+                                                          const uint32_t* __restrict__ off, DevCounters* ctr)
 {
     unsigned long long edges = 0;
     uint32_t cnt = 0;
-    for (uint32_t v = blockIdx.x * blockDim.x + threadIdx.x; v < V; v += gridDim.x * blockDim.x) {
-        if (value[v] != kValueMax) {
-            cnt++;
-            edges += off[v + 1] - off[v];
+    for (uint64_t v0 = ((uint64_t)blockIdx.x * blockDim.x + threadIdx.x) * 4; v0 < V;
+         v0 += (uint64_t)gridDim.x * blockDim.x * 4) {
+        uint32_t x[4], o[5];
+        if (v0 + 3 < V) {
+            const uint4 a = *reinterpret_cast<const uint4*>(value + v0);
+            const uint4 b = *reinterpret_cast<const uint4*>(off + v0);
+            x[0] = a.x, x[1] = a.y, x[2] = a.z, x[3] = a.w;
+            o[0] = b.x, o[1] = b.y, o[2] = b.z, o[3] = b.w, o[4] = off[v0 + 4];
+        } else {
+#pragma unroll
+            for (int k = 0; k < 4; k++) x[k] = v0 + k < V ? value[v0 + k] : kValueMax;
+#pragma unroll
+            for (int k = 0; k < 5; k++) o[k] = off[v0 + k < V ? v0 + k : V];
+        }
+#pragma unroll
+        for (int k = 0; k < 4; k++) {
+            if (x[k] != kValueMax) {
+                cnt++;
+                edges += o[k + 1] - o[k];
+            }
         }
     }
     edges = warp_sum(edges);
-    cnt = warp_sum(cnt);
-    if (lane_id() == 0 && cnt) {
-        atomicAdd(&ctr->reached_edges, edges);
-        atomicAdd(&ctr->reached, cnt);
+    cnt = __reduce_add_sync(0xffffffffu, cnt);
+    __shared__ unsigned long long s_edges[kBlock / 32];
+    __shared__ uint32_t s_cnt[kBlock / 32];
+    if (lane_id() == 0) {
+        s_edges[threadIdx.x >> 5] = edges;
+        s_cnt[threadIdx.x >> 5] = cnt;
+    }
+    __syncthreads();
+    if (threadIdx.x < 32) {
+        edges = warp_sum(threadIdx.x < kBlock / 32 ? s_edges[threadIdx.x] : 0ull);
+        cnt = __reduce_add_sync(0xffffffffu, threadIdx.x < kBlock / 32 ? s_cnt[threadIdx.x] : 0u);
+        if (threadIdx.x == 0 && cnt) {
+            atomicAdd(&ctr->reached_edges, edges);
+            atomicAdd(&ctr->reached, cnt);
+        }
     }
 }
 
@@ -1461,7 +1490,7 @@ void count_reached(cgb_graph* g)
 {
     CGB_CUDA_TRY(cudaMemsetAsync(&g->ctr->reached_edges, 0, sizeof(unsigned long long), g->stream));
     CGB_CUDA_TRY(cudaMemsetAsync(&g->ctr->reached, 0, sizeof(uint32_t), g->stream));
-    k_count_reached<<<grid_for(g->V, kBlock, num_sms() * 8), kBlock, 0, g->stream>>>(g->V, g->value, g->off, g->ctr);
+    k_count_reached<<<grid_for(div_up(g->V, 4), kBlock, num_sms() * 8), kBlock, 0, g->stream>>>(g->V, g->value, g->off, g->ctr);
     sync_counters(g);
     g->stats.reached = g->h_ctr->reached;
     g->stats.traversed_edges = g->h_ctr->reached_edges;

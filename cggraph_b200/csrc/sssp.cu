@@ -49,6 +49,7 @@ struct SsspOp {
     uint32_t cap;
     uint32_t* far_bm;
     DevCounters* ctr;
+    uint32_t t_newfar = 0, t_touched = 0, t_edges = 0, t_maxdeg = 0;  // this thread's counts
     static constexpr int kBatch = 4;
 
     __device__ __forceinline__ bool load(uint32_t v, uint32_t& s, uint32_t& d, uint32_t& m) const
@@ -60,7 +61,7 @@ struct SsspOp {
     }
     template <int N>
     __device__ __forceinline__ void edges(const bool (&valid)[N], const uint32_t (&e)[N],
-                                          const uint32_t (&du)[N]) const
+                                          const uint32_t (&du)[N])
     {
         uint32_t d[N], nd[N], cur[N], old[N], word[N], bit[N];
         bool ok[N], near_c[N], far_c[N], first[N], to_near[N], new_far[N];
@@ -95,41 +96,23 @@ struct SsspOp {
             to_near[i] = fresh && near_c[i];
             new_far[i] = fresh && far_c[i];
         }
-        warp_append_n<N>(to_near, d, near_out, near_len, cap, &ctr->overflow);
-        uint32_t nf = 0, nt = 0;
-        bool any_near = false;
+        stage_append_n<N>(to_near, d, near_out, near_len, cap, &ctr->overflow);
+        // out-edges of the next near queue: the next round's push / pull choice
+        uint32_t lo[N], hi[N];
 #pragma unroll
         for (int i = 0; i < N; i++) {
-            nf += __popc(__ballot_sync(0xffffffffu, new_far[i]));
-            nt += __popc(__ballot_sync(0xffffffffu, first[i]));
-            any_near |= to_near[i];
+            lo[i] = to_near[i] ? off[d[i]] : 0u;
+            hi[i] = to_near[i] ? off[d[i] + 1] : 0u;
         }
-        if (nf && lane_id() == 0) atomicAdd(&s_sssp_newfar, nf);
-        if (nt && lane_id() == 0) atomicAdd(&s_sssp_touched, nt);
-        if (__any_sync(0xffffffffu, any_near)) {
-            // out-edges of the next near queue: the next round's push / pull choice
-            uint32_t lo[N], hi[N];
 #pragma unroll
-            for (int i = 0; i < N; i++) {
-                lo[i] = to_near[i] ? off[d[i]] : 0u;
-                hi[i] = to_near[i] ? off[d[i] + 1] : 0u;
-            }
-            unsigned long long dg = 0;
-            uint32_t mx = 0;
-#pragma unroll
-            for (int i = 0; i < N; i++) {
-                dg += hi[i] - lo[i];
-                mx = max(mx, hi[i] - lo[i]);
-            }
-            dg = warp_sum(dg);
-            mx = warp_max(mx);
-            if (dg && lane_id() == 0) {
-                atomicAdd(&s_sssp_medges, dg);
-                atomicMax(&s_sssp_maxdeg, mx);
-            }
+        for (int i = 0; i < N; i++) {
+            t_newfar += new_far[i] ? 1u : 0u;
+            t_touched += first[i] ? 1u : 0u;
+            t_edges += hi[i] - lo[i];
+            t_maxdeg = max(t_maxdeg, hi[i] - lo[i]);
         }
     }
-    __device__ __forceinline__ void edge(bool valid, uint32_t e, uint32_t du) const
+    __device__ __forceinline__ void edge(bool valid, uint32_t e, uint32_t du)
     {
         const bool v[1] = {valid};
         const uint32_t ee[1] = {e}, m[1] = {du};
@@ -137,6 +120,7 @@ struct SsspOp {
     }
     __device__ __forceinline__ void block_begin() const
     {
+        stage_begin();
         if (threadIdx.x == 0) {
             s_sssp_newfar = 0;
             s_sssp_medges = 0;
@@ -146,6 +130,16 @@ struct SsspOp {
     }
     __device__ __forceinline__ void block_end() const
     {
+        const uint32_t nf = __reduce_add_sync(0xffffffffu, t_newfar), nt = __reduce_add_sync(0xffffffffu, t_touched);
+        const uint32_t dg = __reduce_add_sync(0xffffffffu, t_edges);  // at most E < 2^32
+        const uint32_t mx = __reduce_max_sync(0xffffffffu, t_maxdeg);
+        if (lane_id() == 0) {
+            if (nf) atomicAdd(&s_sssp_newfar, nf);
+            if (nt) atomicAdd(&s_sssp_touched, nt);
+            if (dg) atomicAdd(&s_sssp_medges, (unsigned long long)dg);
+            if (mx) atomicMax(&s_sssp_maxdeg, mx);
+        }
+        stage_end(near_out, near_len, cap, &ctr->overflow);  // a CTA barrier is inside
         if (threadIdx.x == 0 && s_sssp_newfar) atomicAdd(&ctr->far_len[0], s_sssp_newfar);
         if (threadIdx.x == 0 && s_sssp_medges) atomicAdd(&ctr->medges, s_sssp_medges);
         if (threadIdx.x == 0 && s_sssp_touched) atomicAdd(&ctr->touched, s_sssp_touched);
