@@ -197,25 +197,36 @@ __global__ void k_cc_link_round(uint32_t V, const uint32_t* __restrict__ off, co
     }
 }
 
-// Points every vertex at its root (path halving on the way, which shortens
-// the chains that other threads are still walking).  Each thread walks the
-// paths of kN vertices, kN x (grid threads) apart, in one loop.  No hooking
-// runs during this pass, so the set of roots is fixed and weak loads are
-// exact about which vertex is a root (L1 holds nothing from before the
-// launch).
+// Points every vertex at its root.  Each thread walks the paths of kN
+// vertices, kN x (grid threads) apart, in one loop, and writes only its own
+// vertices: a walk that halved the paths it passed could store an older
+// ancestor into a vertex after that vertex's own thread had stored its root,
+// and leave it one step short.  No hooking runs during this pass, so the set
+// of roots is fixed and weak loads are exact about which vertex is a root (L1
+// holds nothing from before the launch).
 template <int kN>
 __global__ void k_cc_compress(uint32_t V, uint32_t* comp)
 {
     const uint64_t T = (uint64_t)gridDim.x * blockDim.x;
     for (uint64_t v0 = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; v0 < V; v0 += kN * T) {
-        uint32_t x[kN];
+        uint32_t first[kN], x[kN];
 #pragma unroll
-        for (int i = 0; i < kN; i++) x[i] = (uint32_t)(v0 + i * T < V ? v0 + i * T : v0);
-        find_roots<false, kN>(x, comp);
+        for (int i = 0; i < kN; i++) x[i] = first[i] = ld_comp<false>(comp, (uint32_t)(v0 + i * T < V ? v0 + i * T : v0));
+        for (bool more = true; more;) {
+            uint32_t p[kN];
+#pragma unroll
+            for (int i = 0; i < kN; i++) p[i] = ld_comp<false>(comp, x[i]);
+            more = false;
+#pragma unroll
+            for (int i = 0; i < kN; i++) {
+                more |= p[i] != x[i];  // pointers only go to smaller vertices: every walk ends
+                x[i] = p[i];
+            }
+        }
 #pragma unroll
         for (int i = 0; i < kN; i++) {
             const uint64_t v = v0 + i * T;
-            if (v < V && ld_comp<false>(comp, (uint32_t)v) != x[i]) comp[v] = x[i];
+            if (v < V && first[i] != x[i]) comp[v] = x[i];
         }
     }
 }

@@ -1,0 +1,53 @@
+"""Components where the sampled link rounds find one giant tree, many equal ones, or none."""
+import numpy as np
+import pytest
+
+import cggraph_b200 as cg
+from oracle import oracle as O
+
+CC = int(cg.Algorithm_type.CC)
+WEAK = 0x8
+
+
+def blocks(sizes, extra, seed):
+    """Disjoint random trees of the given sizes over shuffled ids (parents skewed to a hub), plus `extra` lone vertices."""
+    rng = np.random.default_rng(seed)
+    V = int(sum(sizes)) + extra
+    ids = rng.permutation(V)
+    src, dst, base = [], [], 0
+    for n in sizes:
+        child = np.arange(1, n)
+        parent = np.where(rng.random(n - 1) < 0.5, 0, (rng.random(n - 1) * child).astype(np.int64))
+        a, b = ids[base + child], ids[base + parent]
+        flip = rng.random(n - 1) < 0.5  # edges point either way
+        src.append(np.where(flip, a, b))
+        dst.append(np.where(flip, b, a))
+        base += n
+    return V, np.concatenate(src), np.concatenate(dst)
+
+
+def csr(V, src, dst):
+    key = np.unique(src.astype(np.int64) * V + dst)
+    src, dst = key // V, (key % V).astype(np.uint32)
+    off = np.zeros(V + 1, np.uint32)
+    off[1:] = np.cumsum(np.bincount(src, minlength=V))
+    return off, dst
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("sizes,extra", [
+    ([200_000, 3, 2], 5_000),
+    ([300] * 400, 1),
+    ([130, 2, 2, 2], 0),            # fewer vertices than one sample step
+    ([70_000, 70_000, 70_001], 33),
+    ([5_000_000, 1_000], 100_000),  # rounds above 2^22 vertices
+])
+def test_components(sizes, extra):
+    V, src, dst = blocks(sizes, extra, seed=len(sizes) + extra)
+    off, dd = csr(V, src, dst)
+    soff, sdst = csr(V, np.concatenate([src, dst]), np.concatenate([dst, src]))
+    exp = O.cc(soff, sdst)
+    with cg.Graph.from_csr(off, dd) as g:
+        np.testing.assert_array_equal(g.run(CC, 0, cg.make_options(flags=WEAK))[0], exp)
+    with cg.Graph.from_csr(soff, sdst) as g:
+        np.testing.assert_array_equal(g.run(CC, 0)[0], exp)
