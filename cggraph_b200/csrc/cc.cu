@@ -14,8 +14,10 @@
 //      initialisation of ECL-CC, Jaiganesh and Burtscher 2018);
 //   2. one round that links v with its second neighbour, and with its first
 //      one where step 1 left it pointing at itself (first neighbour larger);
-//      every find halves the path it walks, so no separate compress pass
-//      runs before step 5;
+//      on graphs with hubs it runs on a sample of the vertices first, and the
+//      full round skips the giant component that step 3 finds after that
+//      sample and a compress; every find halves the path it walks, so no
+//      other compress pass runs before step 5;
 //   3. find the roots of 1024 hashed vertices and take the most frequent
 //      one as the giant component c;
 //   4. link every remaining edge of each vertex whose root is not c (the
@@ -166,35 +168,109 @@ __global__ void k_cc_init_min_nbr_weak(uint32_t V, const uint32_t* __restrict__ 
     }
 }
 
+// The vertex of position i when one vertex of every `stride` is taken, at a
+// hashed place (1: all of them).
+__device__ __forceinline__ uint32_t strided_vertex(uint32_t i, uint32_t stride)
+{
+    return stride == 1 ? i : i * stride + (uint32_t)(mix64(i) % stride);
+}
+
+// Links v with n of its neighbours x (v itself stands for a neighbour that is
+// not there).  Their parents are loaded together, and a neighbour with v's
+// parent needs nothing.
+template <int N>
+__device__ __forceinline__ void link_neighbours(uint32_t v, uint32_t cv, const uint32_t (&x)[N], uint32_t* comp,
+                                                DevCounters* ctr)
+{
+    uint32_t c[N];
+#pragma unroll
+    for (int i = 0; i < N; i++) c[i] = ld_comp<false>(comp, x[i]);
+#pragma unroll
+    for (int i = 0; i < N; i++)
+        if (c[i] != cv && x[i] != v) link(v, x[i], comp, ctr);
+}
+
+// The link rounds take one vertex of every `stride`, and skip those whose
+// parent is `giant` (their edges are seen from the other end) and those
+// without edges.  A thread looks at kScan vertices at once and the CTA
+// gathers the ones with work, so that the long chain of a link (lists,
+// parents, walks, CAS) runs in full warps: with a thread per vertex, most of
+// them idle, the full round took 331 us at RMAT-24, gathered 171 us.  Rounds
+// of at most kScanWide vertices take one per thread, which spreads them over
+// more CTAs (RMAT-20 CC 0.16 against 0.21 ms).
+constexpr uint32_t kScanWide = 1u << 22;
+
+template <int kScan, class Want, class Work>
+__device__ __forceinline__ void cc_scan(uint32_t n, uint32_t stride, uint32_t giant, const uint32_t* comp,
+                                        const Want& want, const Work& work)
+{
+    __shared__ uint32_t s_v[kBlock * kScan];
+    __shared__ uint32_t s_n;
+    for (uint64_t b = (uint64_t)blockIdx.x * kBlock * kScan; b < n; b += (uint64_t)gridDim.x * kBlock * kScan) {
+        if (threadIdx.x == 0) s_n = 0;
+        __syncthreads();
+        uint32_t v[kScan], cv[kScan];
+        bool go[kScan];
+#pragma unroll
+        for (int k = 0; k < kScan; k++) {
+            const uint64_t i = b + (uint64_t)k * kBlock + threadIdx.x;
+            go[k] = i < n;
+            v[k] = go[k] ? strided_vertex((uint32_t)i, stride) : 0;
+            cv[k] = go[k] ? ld_comp<false>(comp, v[k]) : giant;
+        }
+#pragma unroll
+        for (int k = 0; k < kScan; k++) go[k] = go[k] && cv[k] != giant && want(v[k]);
+#pragma unroll
+        for (int k = 0; k < kScan; k++) {
+            const uint32_t m = __ballot_sync(0xffffffffu, go[k]);
+            uint32_t at = 0;
+            if (lane_id() == 0 && m) at = atomicAdd(&s_n, (uint32_t)__popc(m));
+            at = __shfl_sync(0xffffffffu, at, 0) + __popc(m & lanemask_lt());
+            if (go[k]) s_v[at] = v[k];
+        }
+        __syncthreads();
+        for (uint32_t i = threadIdx.x; i < s_n; i += kBlock) work(s_v[i]);
+        __syncthreads();
+    }
+}
+
 // Weak components: links v with the first two entries of its out- and
 // in-list, except the one k_cc_init_min_nbr_weak already pointed it at.
-__global__ void k_cc_link_round_weak(uint32_t V, const uint32_t* __restrict__ off, const uint32_t* __restrict__ dst,
-                                     const uint32_t* __restrict__ in_off, const uint32_t* __restrict__ in_src,
-                                     uint32_t* comp, DevCounters* ctr)
+template <int kScan>
+__global__ void __launch_bounds__(kBlock)
+    k_cc_link_round_weak(uint32_t V, const uint32_t* __restrict__ off, const uint32_t* __restrict__ dst,
+                         const uint32_t* __restrict__ in_off, const uint32_t* __restrict__ in_src, uint32_t* comp,
+                         uint32_t stride, uint32_t giant, DevCounters* ctr)
 {
-    for (uint32_t v = blockIdx.x * blockDim.x + threadIdx.x; v < V; v += gridDim.x * blockDim.x) {
-        const uint32_t s = off[v], d = off[v + 1] - s;
-        const uint32_t is = in_off[v], id = in_off[v + 1] - is;
-        const uint32_t o0 = d > 0 ? dst[s] : v, i0 = id > 0 ? in_src[is] : v;
-        const uint32_t init = min(v, min(o0, i0));
-        if (o0 != init) link(v, o0, comp, ctr);
-        if (i0 != init && i0 != o0) link(v, i0, comp, ctr);
-        if (d > 1) link(v, dst[s + 1], comp, ctr);
-        if (id > 1) link(v, in_src[is + 1], comp, ctr);
-    }
+    cc_scan<kScan>(
+        V / stride, stride, giant, comp,
+        [&](uint32_t v) { return (off[v + 1] - off[v]) + (in_off[v + 1] - in_off[v]) != 0; },
+        [&](uint32_t v) {
+            const uint32_t s = off[v], d = off[v + 1] - s;
+            const uint32_t is = in_off[v], id = in_off[v + 1] - is, cv = ld_comp<false>(comp, v);
+            const uint32_t o0 = d > 0 ? dst[s] : v, i0 = id > 0 ? in_src[is] : v;
+            const uint32_t init = min(v, min(o0, i0));
+            const uint32_t x[4] = {o0 != init ? o0 : v, i0 != init && i0 != o0 ? i0 : v, d > 1 ? dst[s + 1] : v,
+                                   id > 1 ? in_src[is + 1] : v};
+            link_neighbours<4>(v, cv, x, comp, ctr);
+        });
 }
 
 // Links v with its r-th neighbour; with `first_up` also with its first
 // neighbour when that one is larger than v (the min-neighbour
 // initialisation only covered edge 0 when it pointed down).
-__global__ void k_cc_link_round(uint32_t V, const uint32_t* __restrict__ off, const uint32_t* __restrict__ dst,
-                                uint32_t* comp, uint32_t r, int first_up, DevCounters* ctr)
+template <int kScan>
+__global__ void __launch_bounds__(kBlock)
+    k_cc_link_round(uint32_t V, const uint32_t* __restrict__ off, const uint32_t* __restrict__ dst, uint32_t* comp,
+                    uint32_t r, int first_up, uint32_t stride, uint32_t giant, DevCounters* ctr)
 {
-    for (uint32_t v = blockIdx.x * blockDim.x + threadIdx.x; v < V; v += gridDim.x * blockDim.x) {
-        const uint32_t s = off[v], d = off[v + 1] - s;
-        if (first_up && d > 0 && dst[s] > v) link(v, dst[s], comp, ctr);
-        if (d > r) link(v, dst[s + r], comp, ctr);
-    }
+    cc_scan<kScan>(
+        V / stride, stride, giant, comp, [&](uint32_t v) { return off[v + 1] != off[v]; },
+        [&](uint32_t v) {
+            const uint32_t s = off[v], d = off[v + 1] - s, cv = ld_comp<false>(comp, v);
+            const uint32_t x[2] = {first_up && d > 0 ? max(v, dst[s]) : v, d > r ? dst[s + r] : v};
+            link_neighbours<2>(v, cv, x, comp, ctr);
+        });
 }
 
 // Points every vertex at its root.  Each thread walks the paths of kN
@@ -288,7 +364,8 @@ struct CcLinkOp {
         s = off[v];
         d = off[v + 1] - s;
         m = v;
-        if (d <= skip || find_halve<false>(v, comp) == giant) return false;
+        // (the giant component's root may have moved since it was sampled)
+        if (d <= skip || find_halve<false>(v, comp) == find_halve<false>(giant, comp)) return false;
         s += skip;
         d -= skip;
         return true;
@@ -397,35 +474,71 @@ static void cc_afforest(cgb_graph* g, bool weak)
         CGB_CUDA_TRY(cudaMemsetAsync(g->ctr, 0, sizeof(DevCounters), g->stream));
         if (timing) ktimer_end(g);
     }
-    for (uint32_t r = 1; r < kRounds; r++) {
-        if (timing) ktimer_begin(g, CGB_K_HOOK);
+    // The link round, first on a few vertices.  The init forest of a skewed
+    // graph has a few thousand large trees, and with every vertex linking at
+    // once, hundreds of thousands of threads try to hook the same roots: the
+    // CASes on one address run at 1.5 G a second, and all but one fail and
+    // walk again (RMAT-20 took as long as RMAT-23).  A hashed sample of the
+    // vertices merges the large trees first, a compress points everyone at
+    // the merged roots, and the full round then finds equal parents.
+    // (RMAT-20 weak: 0.46 -> 0.16 ms, RMAT-24: 1.0 -> 0.75 ms.)  Meshes have
+    // no such trees.
+    constexpr uint32_t kNoGiant = 0xFFFFFFFFu;
+    auto link_round = [&](uint32_t stride, uint32_t skip_giant) {
         ++g->stats.launches;
+        const uint32_t n = std::max(1u, V / stride);
+        const bool wide = n > kScanWide;
+        const uint32_t lgrid = div_up(n, wide ? kBlock * 4 : kBlock);
         if (weak)
-            k_cc_link_round_weak<<<grid, kBlock, 0, g->stream>>>(V, g->off, g->dst, g->in_off, g->in_src, g->value,
-                                                                 g->ctr);
+            (wide ? k_cc_link_round_weak<4> : k_cc_link_round_weak<1>)<<<lgrid, kBlock, 0, g->stream>>>(
+                V, g->off, g->dst, g->in_off, g->in_src, g->value, stride, skip_giant, g->ctr);
         else
-            k_cc_link_round<<<grid, kBlock, 0, g->stream>>>(V, g->off, g->dst, g->value, r, r == 1, g->ctr);
+            (wide ? k_cc_link_round<4> : k_cc_link_round<1>)<<<lgrid, kBlock, 0, g->stream>>>(
+                V, g->off, g->dst, g->value, 1, 1, stride, skip_giant, g->ctr);
+    };
+    auto compress = [&]() {
+        ++g->stats.launches;
+        k_cc_compress<kCompressVerts><<<div_up(V, kBlock * kCompressVerts), kBlock, 0, g->stream>>>(V, g->value);
+    };
+    // the most frequent root of kSamples hashed vertices
+    auto sample_giant = [&]() {
+        if (timing) ktimer_begin(g, CGB_K_OTHER);
+        ++g->stats.launches;
+        k_cc_sample<<<4, kBlock, 0, g->stream>>>(V, g->value, g->sample, kSamples, 0xAFF0E57ull);
         if (timing) ktimer_end(g);
-    }
-    // no compress here either: sampling and the final link find roots themselves
-    if (timing) ktimer_begin(g, CGB_K_OTHER);
-    ++g->stats.launches;
-    k_cc_sample<<<4, kBlock, 0, g->stream>>>(V, g->value, g->sample, kSamples, 0xAFF0E57ull);
-    if (timing) ktimer_end(g);
-    PinnedArray<uint32_t> h(kSamples);  // pinned: a pageable copy would wait on other threads' copies
-    CGB_CUDA_TRY(cudaMemcpyAsync(h.data(), g->sample, kSamples * sizeof(uint32_t), cudaMemcpyDeviceToHost, g->stream));
-    CGB_CUDA_TRY(cudaStreamSynchronize(g->stream));
-    std::sort(h.data(), h.data() + kSamples);
-    uint32_t giant = h[0], best = 0;
-    for (uint32_t i = 0; i < kSamples;) {
-        uint32_t j = i;
-        while (j < kSamples && h[j] == h[i]) j++;
-        if (j - i > best) {
-            best = j - i;
-            giant = h[i];
+        PinnedArray<uint32_t> h(kSamples);  // pinned: a pageable copy would wait on other threads' copies
+        CGB_CUDA_TRY(cudaMemcpyAsync(h.data(), g->sample, kSamples * sizeof(uint32_t), cudaMemcpyDeviceToHost,
+                                     g->stream));
+        CGB_CUDA_TRY(cudaStreamSynchronize(g->stream));
+        std::sort(h.data(), h.data() + kSamples);
+        uint32_t giant = h[0], best = 0;
+        for (uint32_t i = 0; i < kSamples;) {
+            uint32_t j = i;
+            while (j < kSamples && h[j] == h[i]) j++;
+            if (j - i > best) {
+                best = j - i;
+                giant = h[i];
+            }
+            i = j;
         }
-        i = j;
+        return giant;
+    };
+    uint32_t giant = kNoGiant;
+    if (g->max_degree >= kProbeMaxDeg) {
+        if (timing) ktimer_begin(g, CGB_K_HOOK);
+        link_round(1024, kNoGiant);
+        link_round(32, kNoGiant);
+        if (timing) ktimer_end(g);
+        if (timing) ktimer_begin(g, CGB_K_COMPRESS);
+        compress();
+        if (timing) ktimer_end(g);
+        giant = sample_giant();
     }
+    if (timing) ktimer_begin(g, CGB_K_HOOK);
+    link_round(1, giant);
+    if (timing) ktimer_end(g);
+    // no compress here either: sampling and the final link find roots themselves
+    if (giant == kNoGiant) giant = sample_giant();
     CGB_CUDA_TRY(cudaMemsetAsync(&g->ctr->chunk_len, 0, sizeof(uint32_t), g->stream));
     if (timing) ktimer_begin(g, CGB_K_HOOK);
     CcLinkOp op{g->off, g->dst, g->value, giant, kRounds, g->ctr};
@@ -437,8 +550,7 @@ static void cc_afforest(cgb_graph* g, bool weak)
     }
     if (timing) ktimer_end(g);
     if (timing) ktimer_begin(g, CGB_K_COMPRESS);
-    ++g->stats.launches;
-    k_cc_compress<kCompressVerts><<<div_up(V, kBlock * kCompressVerts), kBlock, 0, g->stream>>>(V, g->value);
+    compress();
     if (timing) ktimer_end(g);
     sync_counters(g);
     CGB_REQUIRE(!g->h_ctr->link_giveup, CGB_ETIMEOUT, "CC link retry bound exceeded");
