@@ -367,21 +367,6 @@ cgb_status cgb_run(cgb_graph* g, int algorithm, uint32_t root_or_iters, const cg
     });
 }
 
-// Sum of out-degrees of the reached vertices of n root-major level arrays.
-__global__ void k_batch_reached(uint64_t n, uint32_t V, const uint32_t* __restrict__ val,
-                                const uint32_t* __restrict__ off, DevCounters* ctr)
-{
-    unsigned long long edges = 0;
-    for (uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (uint64_t)gridDim.x * blockDim.x) {
-        if (val[i] != kValueMax) {
-            const uint32_t v = (uint32_t)(i % V);
-            edges += off[v + 1] - off[v];
-        }
-    }
-    edges = warp_sum(edges);
-    if (lane_id() == 0 && edges) atomicAdd(&ctr->reached_edges, edges);
-}
-
 static bool is_device_ptr(const void* p)
 {
     cudaPointerAttributes a;
@@ -453,10 +438,13 @@ cgb_status cgb_run_batch(cgb_graph* g, int algorithm, const uint32_t* roots, uin
                 total += ms;
                 iters += g->stats.iterations;
                 launches += g->stats.launches;
-                CGB_CUDA_TRY(cudaMemsetAsync(&g->ctr->reached_edges, 0, 8, g->stream));
-                k_batch_reached<<<num_sms() * 8, kBlock, 0, g->stream>>>((uint64_t)n * V, (uint32_t)V, lv, g->off, g->ctr);
-                sync_counters(g);
-                edges += g->h_ctr->reached_edges;
+                if (algorithm == CGB_BFS) {
+                    count_reached_ms(g);
+                } else {
+                    sync_counters(g);  // counted while the distances were written
+                    g->stats.traversed_edges = g->h_ctr->reached_edges;
+                }
+                edges += g->stats.traversed_edges;
                 if (out_u32 && !dev_out)
                     CGB_CUDA_TRY(cudaMemcpyAsync(out_u32 + (size_t)s0 * V, lv, (size_t)n * V * 4, cudaMemcpyDeviceToHost,
                                                  g->stream));

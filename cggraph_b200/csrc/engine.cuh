@@ -227,6 +227,7 @@ void count_reached(cgb_graph* g);  // fills stats.reached / traversed_edges for 
 // Multi-root BFS of n <= 64 roots; a level pulls (bottom-up) when the
 // frontier's out-edges times alpha exceed the graph's edges.
 void run_msbfs(cgb_graph* g, const uint32_t* d_roots, uint32_t n, uint32_t* level_out, double alpha);
+void count_reached_ms(cgb_graph* g);  // fills stats.traversed_edges after run_msbfs
 constexpr double kMsAlpha = 15.0;  // default alpha of multi-root passes
 void free_msbfs(cgb_graph* g);
 // Multi-root SSSP of n <= 64 roots (device array); out (device) receives

@@ -36,22 +36,21 @@ __global__ void k_ms_fill(uint64_t n, uint32_t* a, uint32_t value)
 }
 
 // Roots: seen/frontier bits, level 0, and the first active queue (a root
-// listed twice still gets one queue entry).
+// listed twice still gets one queue entry); one thread per root.
 __global__ void k_ms_roots(const uint32_t* roots, uint32_t n, uint32_t V, unsigned long long* seen,
                            unsigned long long* f0, uint32_t* level_out, uint32_t* q, uint32_t* qlen, uint32_t nz,
                            unsigned long long* alive)
 {
-    if (threadIdx.x != 0 || blockIdx.x != 0) return;
-    for (uint32_t k = 0; k < n; k++) {
-        const uint32_t r = roots[k];
-        if (!seen[r] && r < nz) q[(*qlen)++] = r;
-        seen[r] |= 1ull << k;
-        if (r < nz) {
-            f0[r] |= 1ull << k;  // only vertices with out-edges are ever read as frontier
-            *alive |= 1ull << k;
-        }
-        level_out[(size_t)k * V + r] = 0;
+    const uint32_t k = threadIdx.x;
+    if (k >= n) return;
+    const uint32_t r = roots[k];
+    const unsigned long long bit = 1ull << k;
+    if (atomicOr(seen + r, bit) == 0ull && r < nz) q[atomicAdd(qlen, 1u)] = r;
+    if (r < nz) {  // only vertices with out-edges are ever read as frontier
+        atomicOr(f0 + r, bit);
+        atomicOr(alive, bit);
     }
+    level_out[(size_t)k * V + r] = 0;
 }
 
 // Moves next into seen / the new frontier for the queued vertices, writes
@@ -106,18 +105,25 @@ __global__ void k_ms_clear(const uint32_t* __restrict__ q, uint32_t n, unsigned 
 // different depths, so lists are often walked to the end.  Walking a hub's
 // list on one thread would make the hub the whole kernel's time, so:
 //   k_ms_bu_light  -- the first kMsLight in-edges of every vertex, packed
-//                     edge-parallel per CTA;
+//                     edge-parallel per warp;
 //                     vertices left unfinished go to a warp list (or, with
-//                     at least kMsBlockDeg edges left, a CTA list) with the
+//                     at least kMsBlockDeg edges left, a hub list, with a
+//                     descriptor for each kMsHubChunk edges) with the
 //                     roots found so far parked in `acc` (the top-down
 //                     scratch mask, zero between levels);
 //   k_ms_bu_warp   -- a warp per listed vertex, lanes striding the list;
-//   k_ms_bu_chunks -- hub lists cut into chunks over all CTAs, merged into
-//                     acc by atomicOr; k_ms_bu_settle then finishes them.
+//   k_ms_bu_chunks -- a warp per hub chunk, merged into acc by atomicOr;
+//                     k_ms_bu_settle then finishes the hubs.
 // Each vertex has one owner at a time, so its masks and levels are written
 // without atomics; new vertices with out-edges join the next queue.
+// RMAT-22, 64 roots, the level after the roots' (31 k vertices, 22.8 M
+// out-edges; most vertices find few of their roots and walk whole lists):
+// walking the hub list in every CTA took 1.27 ms, descriptors take 0.05 ms;
+// in the next level (levels written one root's run at a time) the light
+// kernel went from 1.09 to 0.51 ms.
 constexpr uint32_t kMsLight = 32;
 constexpr uint32_t kMsBlockDeg = 4096;
+constexpr uint32_t kMsHubChunk = 512;
 
 __device__ __forceinline__ unsigned long long warp_or64(unsigned long long v)
 {
@@ -126,36 +132,34 @@ __device__ __forceinline__ unsigned long long warp_or64(unsigned long long v)
     return ((unsigned long long)hi << 32) | lo;
 }
 
-// Records the roots `got` newly found for vertex u (its owner only).
-__device__ __forceinline__ bool ms_bu_settle(uint32_t u, unsigned long long s, unsigned long long got,
-                                             unsigned long long* seen, unsigned long long* fnext,
-                                             uint32_t* level_out, uint32_t V, uint32_t lvl, uint32_t nz,
-                                             const uint32_t* start)
+// Levels of the roots `got` newly found for vertex u, the warp's lanes
+// holding consecutive vertices: one root at a time, so that a warp's stores
+// are one run of the root's row (a lane writing its own roots one after the
+// other touches a sector per root and vertex).
+__device__ __forceinline__ void ms_write_levels(uint32_t u, unsigned long long got, uint32_t* level_out, uint32_t V,
+                                                uint32_t lvl, const uint32_t* start)
 {
-    seen[u] = s | got;
-    for (unsigned long long m = got; m; m &= m - 1) {
+    for (unsigned long long m = warp_or64(got); m; m &= m - 1) {
         const uint32_t k = __ffsll(m) - 1;
-        level_out[(size_t)k * V + u] = start ? lvl - start[k] : lvl;
+        if ((got >> k) & 1ull) level_out[(size_t)k * V + u] = start ? lvl - start[k] : lvl;
     }
-    if (u < nz) fnext[u] = got;
-    return u < nz;
 }
 
 __global__ void __launch_bounds__(kBlock) k_ms_bu_light(MsBuArgs a)
 {
-    // A CTA takes kBlock consecutive vertices; a CTA-wide exclusive scan
-    // packs the first kMsLight in-edges of each into shared memory, one edge
-    // per thread (coalesced reads of in_src), and the finds are ORed into
-    // the owner's shared mask.
-    __shared__ uint32_t s_scan[kBlock / 32 + 1];
-    __shared__ uint32_t s_edge[kBlock];
-    __shared__ uint32_t s_owner[kBlock];
-    __shared__ unsigned long long s_acc[kBlock];
-    __shared__ unsigned long long s_pend[kBlock];
-    const uint32_t V = a.V, tid = threadIdx.x;
+    // A warp takes 32 consecutive vertices; a warp scan packs the first
+    // kMsLight in-edges of each, kN edges per lane at a time (sources, then
+    // masks, in flight together), and the finds are ORed into the owner's
+    // shared mask.  Warps share nothing between steps.
+    constexpr int kN = 4;
+    __shared__ uint32_t s_acc[kBlock / 32][2][32];
+    const uint32_t V = a.V, lane = lane_id(), warp = threadIdx.x >> 5;
     unsigned long long live = 0;
-    for (uint32_t base = blockIdx.x * kBlock; base < V; base += gridDim.x * kBlock) {
-        const uint32_t u = base + tid;
+    const uint32_t warps = gridDim.x * (kBlock / 32);
+    stage_begin();
+    __syncthreads();
+    for (uint32_t base = (blockIdx.x * (kBlock / 32) + warp) * 32; base < V; base += warps * 32) {
+        const uint32_t u = base + lane;
         unsigned long long s = 0, pending = 0;
         uint32_t e0 = 0, deg = 0, cnt = 0;
         if (u < V) {
@@ -167,42 +171,64 @@ __global__ void __launch_bounds__(kBlock) k_ms_bu_light(MsBuArgs a)
                 cnt = min(deg, kMsLight);
             }
         }
-        s_acc[tid] = 0;
-        s_pend[tid] = pending;
-        uint32_t total;
-        const uint32_t rank = block_excl_scan(cnt, total, s_scan);
-        uint32_t consumed = 0;
-        for (uint32_t done = 0; done < total; done += kBlock) {
-            while (consumed < cnt && rank + consumed < done + kBlock) {
-                s_edge[rank + consumed - done] = e0 + consumed;
-                s_owner[rank + consumed - done] = tid;
-                consumed++;
+        const uint32_t incl = warp_incl_scan(cnt), total = __shfl_sync(0xffffffffu, incl, 31);
+        if (total == 0) continue;
+        const uint32_t excl = incl - cnt;
+        s_acc[warp][0][lane] = s_acc[warp][1][lane] = 0;
+        __syncwarp();
+        for (uint32_t b = 0; b < total; b += 32 * kN) {
+            uint32_t o[kN], src[kN];
+            unsigned long long x[kN];
+#pragma unroll
+            for (int i = 0; i < kN; i++) {
+                const uint32_t p = b + 32 * i + lane;
+                o[i] = 0;
+#pragma unroll
+                for (uint32_t step = 16; step >= 1; step >>= 1) {
+                    const uint32_t ex = __shfl_sync(0xffffffffu, excl, o[i] + step);
+                    if (ex <= p) o[i] += step;
+                }
+                const uint32_t e = __shfl_sync(0xffffffffu, e0, o[i]) + p - __shfl_sync(0xffffffffu, excl, o[i]);
+                src[i] = p < total ? a.in_src[e] : 0xFFFFFFFFu;
             }
-            __syncthreads();
-            if (tid < min((uint32_t)kBlock, total - done)) {
-                const uint32_t o = s_owner[tid];
-                const unsigned long long x = a.front[a.in_src[s_edge[tid]]] & s_pend[o];
-                if (x) atomicOr(&s_acc[o], x);
-            }
-            __syncthreads();
-        }
-        bool act = false, to_warp = false, to_block = false;
-        if (pending) {
-            const unsigned long long got = s_acc[tid];
-            if (got != pending && deg > kMsLight) {
-                a.acc[u] = got;  // finish on a warp or on hub chunks
-                to_block = deg - kMsLight >= kMsBlockDeg;
-                to_warp = !to_block;
-            } else if (got) {
-                act = ms_bu_settle(u, s, got, a.seen, a.fnext, a.level_out, V, a.lvl, a.nz, a.start);
-                if (act) live |= got;
+#pragma unroll
+            for (int i = 0; i < kN; i++) x[i] = src[i] != 0xFFFFFFFFu ? a.front[src[i]] : 0ull;
+#pragma unroll
+            for (int i = 0; i < kN; i++) {
+                const uint32_t lo = (uint32_t)x[i], hi = (uint32_t)(x[i] >> 32);
+                if (lo) atomicOr(&s_acc[warp][0][o[i]], lo);
+                if (hi) atomicOr(&s_acc[warp][1][o[i]], hi);
             }
         }
-        warp_append(act, u, a.qact, a.qact_len, a.cap, &a.ctr->overflow);
+        __syncwarp();
+        unsigned long long got =
+            pending & (((unsigned long long)s_acc[warp][1][lane] << 32) | s_acc[warp][0][lane]);
+        __syncwarp();
+        bool act[1] = {false}, to_warp = false, to_hub = false;
+        if (got != pending && deg > kMsLight) {
+            a.acc[u] = got;  // finish on a warp or in hub chunks
+            got = 0;
+            to_hub = deg - kMsLight >= kMsBlockDeg;
+            to_warp = !to_hub;
+        }
+        ms_write_levels(u, got, a.level_out, V, a.lvl, a.start);
+        if (got) {
+            a.seen[u] = s | got;
+            if (u < a.nz) {
+                a.fnext[u] = got;
+                live |= got;
+                act[0] = true;
+            }
+        }
+        const uint32_t ua[1] = {u};
+        stage_append_n<1>(act, ua, a.qact, a.qact_len, a.cap, &a.ctr->overflow);
         warp_append(to_warp, u, a.heavy_w, a.heavy_len, a.cap, &a.ctr->overflow);
-        warp_append(to_block, u, a.heavy_b, a.heavy_len + 1, a.cap_b, &a.ctr->overflow);
-        __syncthreads();  // s_acc / s_pend are rewritten by the next batch
+        warp_append(to_hub, u, a.heavy_b, a.heavy_len + 1, a.cap_b, &a.ctr->overflow);
+        warp_append_chunks(u, to_hub ? (deg - kMsLight + kMsHubChunk - 1) / kMsHubChunk : 0, a.hub_chunks,
+                           a.heavy_len + 2, a.cap_c, &a.ctr->overflow);
     }
+    __syncthreads();
+    stage_end(a.qact, a.qact_len, a.cap, &a.ctr->overflow);
     if (a.alive) {
         live = warp_or(live);
         if (lane_id() == 0 && live) atomicOr(a.alive, live);
@@ -256,47 +282,49 @@ __global__ void __launch_bounds__(kBlock) k_ms_bu_warp(MsBuArgs a)
     }
 }
 
-// Hub lists: the rest of every listed vertex's list is cut into
-// kMsBlockDeg-edge chunks dealt round-robin over the CTAs (a hub's chunks
-// run on different SMs); each CTA ORs its chunk's finds into acc[u] and
-// skips chunks of vertices already complete.
+// Hub chunks, one warp each: the chunk's finds are ORed into acc[u]; chunks
+// of vertices already complete are skipped.
 __global__ void __launch_bounds__(kBlock) k_ms_bu_chunks(MsBuArgs a)
 {
-    __shared__ unsigned long long s_got;
-    const uint32_t n = min(a.heavy_len[1], a.cap_b);
-    uint64_t chunk_base = 0;
-    for (uint32_t i = 0; i < n; i++) {
-        const uint32_t u = a.heavy_b[i];
-        const uint32_t b0 = a.in_off[u] + kMsLight, e1 = a.in_off[u + 1];
-        const uint32_t nch = (e1 - b0 + kMsBlockDeg - 1) / kMsBlockDeg;
-        const unsigned long long pending = a.full & ~a.seen[u];
-        const uint32_t first = (uint32_t)((blockIdx.x + gridDim.x - (chunk_base % gridDim.x)) % gridDim.x);
-        chunk_base += nch;
-        for (uint32_t c = first; c < nch; c += gridDim.x) {
-            // complete already?  (one read, shared, so the whole CTA takes the same branch)
-            __syncthreads();
-            if (threadIdx.x == 0) s_got = *(volatile unsigned long long*)(a.acc + u);
-            __syncthreads();
-            if (s_got == pending) break;
-            const uint32_t cs = b0 + c * kMsBlockDeg, ce = min(e1, cs + kMsBlockDeg);
-            unsigned long long got = 0;
-            for (uint32_t e = cs + threadIdx.x; e < ce; e += 4 * kBlock) {
-                uint32_t src[4];
+    constexpr int kN = 8;
+    const uint32_t n = min(a.heavy_len[2], a.cap_c), lane = lane_id();
+    const uint32_t warps = gridDim.x * (kBlock / 32);
+    for (uint32_t c = (threadIdx.x >> 5) * gridDim.x + blockIdx.x; c < n; c += warps) {
+        const uint2 d = a.hub_chunks[c];
+        const unsigned long long pending = a.full & ~a.seen[d.x];
+        // one read for the warp: other warps are ORing into it
+        const unsigned long long have =
+            __shfl_sync(0xffffffffu, *(volatile unsigned long long*)(a.acc + d.x), 0);
+        if (have == pending) continue;
+        const uint32_t b0 = a.in_off[d.x] + kMsLight + d.y * kMsHubChunk;
+        const uint32_t e1 = min(a.in_off[d.x + 1], b0 + kMsHubChunk);
+        unsigned long long got = 0;
+        for (uint32_t e = b0 + lane; e < e1; e += 32 * kN) {
+            uint32_t src[kN];
 #pragma unroll
-                for (int j = 0; j < 4; j++) src[j] = e + j * kBlock < ce ? a.in_src[e + j * kBlock] : 0xFFFFFFFFu;
+            for (int j = 0; j < kN; j++) src[j] = e + 32 * j < e1 ? a.in_src[e + 32 * j] : 0xFFFFFFFFu;
 #pragma unroll
-                for (int j = 0; j < 4; j++)
-                    if (src[j] != 0xFFFFFFFFu) got |= a.front[src[j]];
-            }
-            got = warp_or64(got & pending);
-            if (threadIdx.x == 0) s_got = 0;
-            __syncthreads();
-            if (lane_id() == 0 && got) atomicOr(&s_got, got);
-            __syncthreads();
-            if (threadIdx.x == 0 && (s_got & ~*(volatile unsigned long long*)(a.acc + u))) atomicOr(a.acc + u, s_got);
-            __syncthreads();
+            for (int j = 0; j < kN; j++)
+                if (src[j] != 0xFFFFFFFFu) got |= a.front[src[j]];
         }
+        got = warp_or64(got) & pending;
+        if (lane == 0 && (got & ~have)) atomicOr(a.acc + d.x, got);
     }
+}
+
+// Records the roots `got` newly found for vertex u (its owner only).
+__device__ __forceinline__ bool ms_bu_settle(uint32_t u, unsigned long long s, unsigned long long got,
+                                             unsigned long long* seen, unsigned long long* fnext,
+                                             uint32_t* level_out, uint32_t V, uint32_t lvl, uint32_t nz,
+                                             const uint32_t* start)
+{
+    seen[u] = s | got;
+    for (unsigned long long m = got; m; m &= m - 1) {
+        const uint32_t k = __ffsll(m) - 1;
+        level_out[(size_t)k * V + u] = start ? lvl - start[k] : lvl;
+    }
+    if (u < nz) fnext[u] = got;
+    return u < nz;
 }
 
 // Settles the listed hub vertices from their merged masks.
@@ -328,11 +356,11 @@ __global__ void __launch_bounds__(kBlock) k_ms_bu_settle(MsBuArgs a)
 
 void ms_bottom_up(const MsBuArgs& a, cudaStream_t st, uint64_t* launches)
 {
-    CGB_CUDA_TRY(cudaMemsetAsync(a.heavy_len, 0, 8, st));
+    CGB_CUDA_TRY(cudaMemsetAsync(a.heavy_len, 0, 12, st));
     k_ms_bu_light<<<grid_for(a.V, kBlock, num_sms() * 8), kBlock, 0, st>>>(a);
     k_ms_bu_warp<<<num_sms() * 8, kBlock, 0, st>>>(a);
-    k_ms_bu_chunks<<<num_sms() * 4, kBlock, 0, st>>>(a);
-    k_ms_bu_settle<<<num_sms(), kBlock, 0, st>>>(a);
+    k_ms_bu_chunks<<<num_sms() * 8, kBlock, 0, st>>>(a);
+    k_ms_bu_settle<<<num_sms() * 4, kBlock, 0, st>>>(a);
     if (launches) *launches += 4;
 }
 
@@ -347,6 +375,25 @@ __global__ void k_ms_degree_sum(const uint32_t* __restrict__ q, uint32_t n, cons
     }
     s = warp_sum(s);
     if (lane_id() == 0 && s) atomicAdd(&ctr->medges, s);
+}
+
+// Out-edges of the reached (root, vertex) pairs, from the seen masks.
+__global__ void k_ms_reached(uint32_t V, const unsigned long long* __restrict__ seen, const uint32_t* __restrict__ off,
+                             DevCounters* ctr)
+{
+    unsigned long long edges = 0;
+    for (uint32_t v = blockIdx.x * blockDim.x + threadIdx.x; v < V; v += gridDim.x * blockDim.x)
+        edges += (unsigned long long)__popcll(seen[v]) * (off[v + 1] - off[v]);
+    edges = warp_sum(edges);
+    if (lane_id() == 0 && edges) atomicAdd(&ctr->reached_edges, edges);
+}
+
+void count_reached_ms(cgb_graph* g)
+{
+    CGB_CUDA_TRY(cudaMemsetAsync(&g->ctr->reached_edges, 0, 8, g->stream));
+    k_ms_reached<<<grid_for(g->V, kBlock, num_sms() * 8), kBlock, 0, g->stream>>>(g->V, g->ms->seen, g->off, g->ctr);
+    sync_counters(g);
+    g->stats.traversed_edges = g->h_ctr->reached_edges;
 }
 
 unsigned long long* ms_alloc(size_t n)
@@ -376,7 +423,7 @@ void run_msbfs(cgb_graph* g, const uint32_t* d_roots, uint32_t n, uint32_t* leve
     k_ms_fill<<<num_sms() * 8, kBlock, 0, g->stream>>>((uint64_t)n * V, level_out, kValueMax);
     CGB_CUDA_TRY(cudaMemsetAsync(g->ctr, 0, sizeof(DevCounters), g->stream));
     ++g->stats.launches;
-    k_ms_roots<<<1, 1, 0, g->stream>>>(d_roots, n, V, b.seen, b.front[0], level_out, g->q[0], &g->ctr->qlen[0], g->nz,
+    k_ms_roots<<<1, 64, 0, g->stream>>>(d_roots, n, V, b.seen, b.front[0], level_out, g->q[0], &g->ctr->qlen[0], g->nz,
                                        &g->ctr->alive);
     sync_counters(g);
     uint64_t nact = g->h_ctr->qlen[0];
@@ -406,7 +453,7 @@ void run_msbfs(cgb_graph* g, const uint32_t* d_roots, uint32_t n, uint32_t* leve
         if (pull) {
             MsBuArgs ba{V, g->in_off, g->in_src, fcur, b.seen, fnxt, b.next, live, level_out, lvl + 1, g->nz,
                         g->q[nxt], &g->ctr->qlen[nxt], V, g->ctr, nullptr, &g->ctr->alive, b.heavy_w, b.heavy_b,
-                        b.heavy_len, b.cap_b};
+                        b.heavy_len, b.cap_b, b.hub_chunks, b.cap_c};
             ms_bottom_up(ba, g->stream, &g->stats.launches);
             g->stats.pulls_bu++;
         } else {
@@ -462,7 +509,10 @@ MsBuffers* ms_buffers_alloc(uint32_t V, uint64_t E)
         CGB_CUDA_TRY(cudaMalloc((void**)&b->heavy_w, (size_t)V * 4));
         b->cap_b = (uint32_t)std::min<uint64_t>(E / kMsBlockDeg + 2, V);
         CGB_CUDA_TRY(cudaMalloc((void**)&b->heavy_b, (size_t)b->cap_b * 4));
-        CGB_CUDA_TRY(cudaMalloc((void**)&b->heavy_len, 8));
+        // every hub's list past kMsLight in chunks: sum of ceil(deg / kMsHubChunk) <= E / kMsHubChunk + hubs
+        b->cap_c = (uint32_t)(E / kMsHubChunk + b->cap_b + 1);
+        CGB_CUDA_TRY(cudaMalloc((void**)&b->hub_chunks, (size_t)b->cap_c * sizeof(uint2)));
+        CGB_CUDA_TRY(cudaMalloc((void**)&b->heavy_len, 12));
     } catch (...) {
         ms_buffers_free(b);
         throw;
@@ -479,6 +529,7 @@ void ms_buffers_free(MsBuffers* b)
     cudaFree(b->next);
     cudaFree(b->heavy_w);
     cudaFree(b->heavy_b);
+    cudaFree(b->hub_chunks);
     cudaFree(b->heavy_len);
     delete b;
 }

@@ -3,6 +3,7 @@
 #pragma once
 
 #include "engine.cuh"
+#include "push.cuh"
 
 namespace cgb {
 
@@ -11,9 +12,10 @@ struct MsBuffers {
     unsigned long long* front[2] = {nullptr, nullptr};
     unsigned long long* next = nullptr;     // top-down scratch; bottom-up partial masks; zero between levels
     uint32_t* heavy_w = nullptr;            // bottom-up: vertices finished by a warp (V)
-    uint32_t* heavy_b = nullptr;            // ... by a CTA (cap_b)
-    uint32_t* heavy_len = nullptr;          // [2] lengths of the two lists
-    uint32_t cap_b = 0;
+    uint32_t* heavy_b = nullptr;            // ... in chunks (cap_b)
+    uint2* hub_chunks = nullptr;            // their chunks: (vertex, chunk) (cap_c)
+    uint32_t* heavy_len = nullptr;          // [3] lengths of the three lists
+    uint32_t cap_b = 0, cap_c = 0;
 };
 
 MsBuffers* ms_buffers_alloc(uint32_t V, uint64_t E);
@@ -42,6 +44,8 @@ struct MsBuArgs {
     uint32_t* heavy_b;
     uint32_t* heavy_len;
     uint32_t cap_b;
+    uint2* hub_chunks;
+    uint32_t cap_c;
 };
 void ms_bottom_up(const MsBuArgs& a, cudaStream_t st, uint64_t* launches);
 
@@ -56,6 +60,8 @@ struct MsTdOp {
     uint32_t cap;
     DevCounters* ctr;
 
+    static constexpr int kBatch = 4;  // edge slots per lane visited together (push.cuh)
+
     __device__ __forceinline__ bool load(uint32_t v, uint32_t& s, uint32_t& d, uint32_t& m) const
     {
         s = off[v];
@@ -63,19 +69,30 @@ struct MsTdOp {
         m = v;
         return true;
     }
+    template <int N>
+    __device__ __forceinline__ void edges(const bool (&valid)[N], const uint32_t (&e)[N], const uint32_t (&v)[N]) const
+    {
+        uint32_t u[N];
+        unsigned long long add[N], have[N];
+        bool first[N];
+#pragma unroll
+        for (int i = 0; i < N; i++) u[i] = valid[i] ? __ldcs(dst + e[i]) : 0u;
+#pragma unroll
+        for (int i = 0; i < N; i++) add[i] = valid[i] ? front[v[i]] & ~seen[u[i]] : 0ull;
+#pragma unroll
+        for (int i = 0; i < N; i++) have[i] = add[i] ? next[u[i]] : 0ull;
+#pragma unroll
+        for (int i = 0; i < N; i++) first[i] = (add[i] & ~have[i]) && atomicOr(next + u[i], add[i]) == 0ull;
+        stage_append_n<N>(first, u, qout, qlen, cap, &ctr->overflow);
+    }
     __device__ __forceinline__ void edge(bool valid, uint32_t e, uint32_t v) const
     {
-        bool first = false;
-        uint32_t u = 0;
-        if (valid) {
-            u = dst[e];
-            const unsigned long long add = front[v] & ~seen[u];
-            if (add && (next[u] & add) != add) first = atomicOr(next + u, add) == 0ull;
-        }
-        warp_append(first, u, qout, qlen, cap, &ctr->overflow);
+        const bool va[1] = {valid};
+        const uint32_t ea[1] = {e}, ma[1] = {v};
+        edges<1>(va, ea, ma);
     }
-    __device__ __forceinline__ void block_begin() const {}
-    __device__ __forceinline__ void block_end() const {}
+    __device__ __forceinline__ void block_begin() const { stage_begin(); }
+    __device__ __forceinline__ void block_end() const { stage_end(qout, qlen, cap, &ctr->overflow); }
 };
 
 // n_ptr (optional) replaces n by a device-resident count.

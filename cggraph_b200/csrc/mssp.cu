@@ -36,19 +36,15 @@ __global__ void k_mssp_init(uint32_t V, uint4* dist4, unsigned long long* pend, 
     }
 }
 
-// Roots at distance 0 and queued once each (one thread).
+// Roots at distance 0 and queued once each; one thread per root.
 __global__ void k_mssp_roots(const uint32_t* roots, uint32_t n, uint32_t* dist, unsigned long long* pend, uint32_t* q,
                              MsspCounters* c)
 {
-    if (threadIdx.x != 0 || blockIdx.x != 0) return;
-    uint32_t len = 0;
-    for (uint32_t k = 0; k < n; k++) {
-        const uint32_t r = roots[k];
-        dist[(size_t)r * kMsRoots + k] = 0;
-        if (pend[r] == 0) q[len++] = r;
-        pend[r] |= 1ull << k;
-    }
-    c->nq_out = len;
+    const uint32_t k = threadIdx.x;
+    if (k >= n) return;
+    const uint32_t r = roots[k];
+    dist[(size_t)r * kMsRoots + k] = 0;
+    if (atomicOr(pend + r, 1ull << k) == 0ull) q[atomicAdd(&c->nq_out, 1u)] = r;
 }
 
 __global__ void __launch_bounds__(kBlock) k_mssp_desc(const uint32_t* __restrict__ q, const uint32_t* nq_ptr,
@@ -88,17 +84,23 @@ __global__ void __launch_bounds__(kBlock) k_mssp_split(const uint32_t* __restric
 }
 
 // dist (vertex-major, 64 slots) -> out[k * V + v] for k < n, through a
-// 32-vertex x 64-root shared tile.
+// 32-vertex x 64-root shared tile; the out-edges of the reached (root,
+// vertex) pairs are added to ctr->reached_edges.
 __global__ void __launch_bounds__(kBlock) k_mssp_out(const uint32_t* __restrict__ dist, uint32_t V, uint32_t n,
-                                                     uint32_t* out)
+                                                     uint32_t* out, const uint32_t* __restrict__ off, DevCounters* ctr)
 {
+    unsigned long long edges = 0;  // lane 0's
     __shared__ uint32_t tile[32][kMsRoots + 1];
     const uint32_t tiles = (V + 31) / 32;
     for (uint32_t t = blockIdx.x; t < tiles; t += gridDim.x) {
         const uint32_t v0 = t * 32;
         for (uint32_t i = threadIdx.x; i < 32 * kMsRoots; i += blockDim.x) {
             const uint32_t r = i / kMsRoots, k = i % kMsRoots;
-            if (v0 + r < V) tile[r][k] = dist[(size_t)(v0 + r) * kMsRoots + k];
+            const uint32_t d = v0 + r < V ? dist[(size_t)(v0 + r) * kMsRoots + k] : kValueMax;
+            tile[r][k] = d;
+            // a warp holds 32 roots of one vertex
+            const uint32_t reached = __popc(__ballot_sync(0xffffffffu, k < n && d != kValueMax));
+            if (lane_id() == 0 && reached) edges += (unsigned long long)reached * (off[v0 + r + 1] - off[v0 + r]);
         }
         __syncthreads();
         for (uint32_t i = threadIdx.x; i < 32 * n; i += blockDim.x) {
@@ -107,6 +109,7 @@ __global__ void __launch_bounds__(kBlock) k_mssp_out(const uint32_t* __restrict_
         }
         __syncthreads();
     }
+    if (lane_id() == 0 && edges) atomicAdd(&ctr->reached_edges, edges);
 }
 
 void mssp_expand(bool weighted, uint32_t grid, cudaStream_t st, const uint4* desc, const MsspCounters* cc,
@@ -203,7 +206,7 @@ void run_mssp(cgb_graph* g, const uint32_t* d_roots, uint32_t n, uint32_t* out, 
     ++g->stats.launches;
     k_mssp_init<<<num_sms() * 8, kBlock, 0, g->stream>>>(V, reinterpret_cast<uint4*>(b.dist), b.pend, b.farm);
     ++g->stats.launches;
-    k_mssp_roots<<<1, 1, 0, g->stream>>>(d_roots, n, b.dist, b.pend, g->q[0], b.c);
+    k_mssp_roots<<<1, kMsRoots, 0, g->stream>>>(d_roots, n, b.dist, b.pend, g->q[0], b.c);
     uint32_t nq = mssp_sync(g).nq_out, nfar = 0;
     CGB_CUDA_TRY(cudaMemcpyAsync(&b.c->nq_in, &b.c->nq_out, 4, cudaMemcpyDeviceToDevice, g->stream));
     int cur = 0, fcur = 0;  // near queue / far list holding the live entries
@@ -259,7 +262,8 @@ void run_mssp(cgb_graph* g, const uint32_t* d_roots, uint32_t n, uint32_t* out, 
         CGB_CUDA_TRY(cudaMemcpyAsync(&b.c->nq_in, &b.c->nq_out, 4, cudaMemcpyDeviceToDevice, g->stream));
     }
     ++g->stats.launches;
-    k_mssp_out<<<num_sms() * 16, kBlock, 0, g->stream>>>(b.dist, V, n, out);
+    CGB_CUDA_TRY(cudaMemsetAsync(&g->ctr->reached_edges, 0, 8, g->stream));
+    k_mssp_out<<<num_sms() * 16, kBlock, 0, g->stream>>>(b.dist, V, n, out, g->off, g->ctr);
     g->stats.iterations = rounds;
     g->stats.sssp_delta = delta;
 }

@@ -7,6 +7,7 @@
 namespace cgb {
 
 constexpr uint32_t kMsRoots = 64;   // distance slots per vertex
+constexpr int kMsspBatch = 4;       // edges whose targets' distances are in flight together
 
 struct MsspCounters {
     uint32_t nq_in;        // entries of the near queue being expanded
@@ -16,7 +17,7 @@ struct MsspCounters {
     uint32_t ndesc;        // descriptors of the round
     uint32_t min_far;      // smallest far distance >= hi seen by a split
     uint32_t overflow;
-    unsigned long long relax;  // successful relaxations
+    unsigned long long relax;  // relaxations (root, edge) that lowered the distance read
 };
 
 struct MsspBuffers {
@@ -118,43 +119,40 @@ __device__ __forceinline__ void mssp_expand_body(const uint4* __restrict__ desc,
             // lane t collects the root masks improved through edge t, then
             // every lane publishes its own edge's masks (32 atomics at once)
             unsigned long long my_nb = 0, my_fb = 0;
-            for (uint32_t t0 = 0; t0 < cnt; t0 += 4) {
-                uint32_t u[4], wt[4], x0[4], x1[4];
+            for (uint32_t t0 = 0; t0 < cnt; t0 += kMsspBatch) {
+                uint32_t u[kMsspBatch], x0[kMsspBatch], x1[kMsspBatch];
 #pragma unroll
-                for (int i = 0; i < 4; i++) {  // loads first: four targets in flight
-                    const uint32_t t = min(t0 + i, cnt - 1);
-                    u[i] = __shfl_sync(0xffffffffu, my_u, t);
-                    wt[i] = __shfl_sync(0xffffffffu, my_w, t);
+                for (int i = 0; i < kMsspBatch; i++) {  // loads first: kMsspBatch targets in flight
+                    u[i] = __shfl_sync(0xffffffffu, my_u, min(t0 + i, cnt - 1));
                     const uint32_t* du = dist + (size_t)u[i] * kMsRoots;
                     x0[i] = s0 ? du[lane] : 0u;
                     x1[i] = s1 ? du[lane + 32] : 0u;
                 }
 #pragma unroll
-                for (int i = 0; i < 4; i++) {
+                for (int i = 0; i < kMsspBatch; i++) {
                     const uint32_t t = t0 + i;
                     if (t >= cnt) break;  // warp-uniform
+                    const uint32_t wt = __shfl_sync(0xffffffffu, my_w, t);
+                    // a candidate counts when it lowers the distance (at most
+                    // kValueMax) and the 32-bit sum did not wrap
+                    const uint32_t c0 = dv0 + wt, c1 = dv1 + wt;
+                    const bool m0 = c0 < x0[i] && c0 >= wt, m1 = c1 < x1[i] && c1 >= wt;
+                    if (!__any_sync(0xffffffffu, m0 || m1)) continue;
+                    // lowered without waiting for the old value: where another
+                    // warp lowers the pair further at the same time, both mark
+                    // it, and the later round finds the smaller distance
                     uint32_t* du = dist + (size_t)u[i] * kMsRoots;
-                    bool m0 = false, m1 = false, n0 = false, n1 = false;
-                    const uint64_t c0 = (uint64_t)dv0 + wt[i], c1 = (uint64_t)dv1 + wt[i];
-                    if (s0 && c0 < kValueMax && (uint32_t)c0 < x0[i]) {
-                        m0 = (uint32_t)c0 < atomicMin(du + lane, (uint32_t)c0);
-                        n0 = m0 && (uint32_t)c0 < thr0;
-                    }
-                    if (s1 && c1 < kValueMax && (uint32_t)c1 < x1[i]) {
-                        m1 = (uint32_t)c1 < atomicMin(du + lane + 32, (uint32_t)c1);
-                        n1 = m1 && (uint32_t)c1 < thr1;
-                    }
-                    // improved roots; their near / far split only when there are any
+                    if (m0) atomicMin(du + lane, c0);
+                    if (m1) atomicMin(du + lane + 32, c1);
                     const unsigned long long mb = (unsigned long long)__ballot_sync(0xffffffffu, m0) |
                                                   ((unsigned long long)__ballot_sync(0xffffffffu, m1) << 32);
-                    if (mb) {
-                        relax += (m0 ? 1 : 0) + (m1 ? 1 : 0);
-                        const unsigned long long nb = (unsigned long long)__ballot_sync(0xffffffffu, n0) |
-                                                      ((unsigned long long)__ballot_sync(0xffffffffu, n1) << 32);
-                        if (lane == t) {
-                            my_nb = nb;
-                            my_fb = mb & ~nb;
-                        }
+                    const unsigned long long nb =
+                        (unsigned long long)__ballot_sync(0xffffffffu, m0 && c0 < thr0) |
+                        ((unsigned long long)__ballot_sync(0xffffffffu, m1 && c1 < thr1) << 32);
+                    relax += __popcll(mb);
+                    if (lane == t) {
+                        my_nb = nb;
+                        my_fb = mb & ~nb;
                     }
                 }
             }
@@ -166,7 +164,6 @@ __device__ __forceinline__ void mssp_expand_body(const uint4* __restrict__ desc,
             warp_append(qf, my_u, far_out, far_len, cap, &c->overflow);
         }
     }
-    relax = warp_sum(relax);
     if (lane == 0 && relax) atomicAdd(&c->relax, relax);
     if (alive) {
         near_live = warp_or(near_live);

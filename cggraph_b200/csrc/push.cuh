@@ -207,6 +207,34 @@ __device__ __forceinline__ void block_append_n(const bool (&pred)[N], const uint
     __syncthreads();  // s_base is rewritten by the next call
 }
 
+// Chunk descriptors (v, 0 .. nch - 1) of every lane's vertex, written by the
+// warp together with one atomic for all of them; position p belongs to the
+// last lane whose first position is <= p (a 5-step shuffle search).
+__device__ __forceinline__ void warp_append_chunks(uint32_t v, uint32_t nch, uint2* q, uint32_t* len, uint32_t cap,
+                                                   uint32_t* overflow)
+{
+    if (!__any_sync(0xffffffffu, nch != 0)) return;
+    const uint32_t incl = warp_incl_scan(nch), total = __shfl_sync(0xffffffffu, incl, 31);
+    const uint32_t excl = incl - nch;
+    uint32_t slot = 0;
+    if (lane_id() == 0) slot = atomicAdd(len, total);
+    slot = __shfl_sync(0xffffffffu, slot, 0);
+    for (uint32_t p0 = 0; p0 < total; p0 += 32) {
+        const uint32_t p = p0 + lane_id();
+        uint32_t o = 0;
+#pragma unroll
+        for (uint32_t step = 16; step >= 1; step >>= 1) {
+            const uint32_t ex = __shfl_sync(0xffffffffu, excl, o + step);
+            if (ex <= p) o += step;
+        }
+        const uint32_t bv = __shfl_sync(0xffffffffu, v, o), ex = __shfl_sync(0xffffffffu, excl, o);
+        if (p < total) {
+            if (slot + p < cap) q[slot + p] = make_uint2(bv, p - ex);
+            else atomicOr(overflow, 1u);
+        }
+    }
+}
+
 // Fine-grained tier: a CTA-wide exclusive scan of the (small) remaining
 // degrees packs the lists into shared memory, one edge per thread per round.
 // Every thread of the CTA must call it.
@@ -380,33 +408,10 @@ __global__ void __launch_bounds__(kBlk) k_push_binned(const uint32_t* __restrict
             v = kIdentity ? i : qin[i];
             if (!op.load(v, start, deg, msg)) deg = 0;
         }
-        // big lists: the warp writes their chunk descriptors together, one
-        // atomic for all of them; position p belongs to the last lane whose
-        // first position is <= p (a 5-step shuffle search)
+        // big lists go to the chunk queue
         const bool is_big = deg >= big_deg;
-        if (__any_sync(0xffffffffu, is_big)) {
-            const uint32_t nch = is_big ? (deg + chunk - 1) / chunk : 0;
-            const uint32_t incl = warp_incl_scan(nch), total = __shfl_sync(0xffffffffu, incl, 31);
-            const uint32_t excl = incl - nch;
-            uint32_t slot = 0;
-            if (lane_id() == 0) slot = atomicAdd(chunk_len, total);
-            slot = __shfl_sync(0xffffffffu, slot, 0);
-            for (uint32_t p0 = 0; p0 < total; p0 += 32) {
-                const uint32_t p = p0 + lane_id();
-                uint32_t o = 0;
-#pragma unroll
-                for (uint32_t step = 16; step >= 1; step >>= 1) {
-                    const uint32_t ex = __shfl_sync(0xffffffffu, excl, o + step);
-                    if (ex <= p) o += step;
-                }
-                const uint32_t bv = __shfl_sync(0xffffffffu, v, o), ex = __shfl_sync(0xffffffffu, excl, o);
-                if (p < total) {
-                    if (slot + p < chunk_cap) chunk_q[slot + p] = make_uint2(bv, p - ex);
-                    else atomicOr(overflow, 1u);
-                }
-            }
-            if (is_big) deg = 0;
-        }
+        warp_append_chunks(v, is_big ? (deg + chunk - 1) / chunk : 0, chunk_q, chunk_len, chunk_cap, overflow);
+        if (is_big) deg = 0;
         // warp tier
         uint32_t wmask;
         while ((wmask = __ballot_sync(0xffffffffu, deg >= 32)) != 0) {

@@ -763,7 +763,8 @@ static void bfs_issue(cgb_server* s, Group& G)
     if (pull) {
         MsBuArgs ba{V, g->in_off, g->in_src, G.mb->front[cur], G.mb->seen, G.mb->front[nxt], G.mb->next, G.live,
                     G.region, lvl, g->nz, G.q[nxt], &g->ctr->qlen[nxt], V, g->ctr, G.d_up->start,
-                    &G.d_stats->alive[0], G.mb->heavy_w, G.mb->heavy_b, G.mb->heavy_len, G.mb->cap_b};
+                    &G.d_stats->alive[0], G.mb->heavy_w, G.mb->heavy_b, G.mb->heavy_len, G.mb->cap_b,
+                    G.mb->hub_chunks, G.mb->cap_c};
         ms_bottom_up(ba, st, nullptr);
     } else {
         CGB_CUDA_TRY(cudaMemsetAsync(&g->ctr->found, 0, 4, st));
