@@ -319,6 +319,7 @@ cgb_status cgb_batch_run(cgb_batch* b, int algorithm, const uint32_t* roots, uin
         CGB_CUDA_TRY(cudaEventElapsedTime(&ms, g->ev_start, g->ev_stop));
         g->stats.ms = ms;
         if (algorithm != CGB_CC) {
+            CGB_CUDA_TRY(cudaMemsetAsync(g->ctr, 0, sizeof(DevCounters), g->stream));
             count_reached(g);
             const uint64_t per_edge = algorithm == CGB_BFS ? 8 : (g->w ? 12 : 8);
             g->stats.alg_bytes = per_edge * g->stats.traversed_edges + 12ull * g->V;

@@ -292,9 +292,11 @@ cgb_status cgb_graph_result_download(const cgb_graph* g, void* values)
 
 }  // extern "C"
 
-// One run of the single-root engine; the caller holds the graph's lock.
+// One run of the single-root engine; the caller holds the graph's lock.  With
+// `out`, the result is also copied there, before the run's one last
+// synchronisation.
 namespace cgb {
-void run_one(cgb_graph* g, int alg, uint32_t root_or_iters, const cgb_options& o)
+void run_one(cgb_graph* g, int alg, uint32_t root_or_iters, const cgb_options& o, void* out)
 {
     g->tune = g->tune_alg[alg];
     g->stats = cgb_run_stats{};
@@ -318,15 +320,17 @@ void run_one(cgb_graph* g, int alg, uint32_t root_or_iters, const cgb_options& o
         run_pr(g, root_or_iters, o);
         break;
     }
-    CGB_CUDA_TRY(cudaEventSynchronize(g->ev_stop));
+    const uint64_t V = g->V, E = g->E;
+    if (alg != CGB_PR) g->result = g->value;
+    if (out) copy_any(out, g->result, (size_t)V * (alg == CGB_PR ? 8 : 4), g->stream);
+    if (alg == CGB_BFS || alg == CGB_SSSP) count_reached(g);
+    else CGB_CUDA_TRY(cudaStreamSynchronize(g->stream));
     CGB_CUDA_TRY(cudaGetLastError());
     float ms = 0.f;
     CGB_CUDA_TRY(cudaEventElapsedTime(&ms, g->ev_start, g->ev_stop));
     g->stats.ms = ms;
     if (o.flags & CGB_FLAG_KERNEL_TIMING) ktimer_collect(g);
-    const uint64_t V = g->V, E = g->E;
     if (alg == CGB_BFS || alg == CGB_SSSP) {
-        count_reached(g);
         const uint64_t per_edge = alg == CGB_BFS ? 8 : (g->w ? 12 : 8);
         g->stats.alg_bytes = per_edge * g->stats.traversed_edges + 12 * V;
     } else if (alg == CGB_CC) {
@@ -338,7 +342,6 @@ void run_one(cgb_graph* g, int alg, uint32_t root_or_iters, const cgb_options& o
         g->stats.reached = V;
         g->stats.alg_bytes = (12 * E + 20 * V + 4) * g->stats.iterations;
     }
-    if (alg != CGB_PR) g->result = g->value;
     g->result_alg = alg;
 }
 }  // namespace cgb
@@ -356,13 +359,7 @@ cgb_status cgb_run(cgb_graph* g, int algorithm, uint32_t root_or_iters, const cg
         const cgb_options o = effective_options(opt);
         std::lock_guard<GraphMutex> lock(g->mu);
         CGB_CUDA_TRY(cudaSetDevice(g->device));
-        run_one(g, algorithm, root_or_iters, o);
-        if (algorithm == CGB_PR) {
-            if (out_f64) copy_any(out_f64, g->result, (size_t)g->V * 8, g->stream);
-        } else if (out_u32) {
-            copy_any(out_u32, g->result, (size_t)g->V * 4, g->stream);
-        }
-        CGB_CUDA_TRY(cudaStreamSynchronize(g->stream));
+        run_one(g, algorithm, root_or_iters, o, algorithm == CGB_PR ? (void*)out_f64 : (void*)out_u32);
         if (out_ms) *out_ms = g->stats.ms;
     });
 }
@@ -392,13 +389,11 @@ cgb_status cgb_run_batch(cgb_graph* g, int algorithm, const uint32_t* roots, uin
             double total = 0;
             uint64_t edges = 0, launches = 0;
             for (uint32_t i = 0; i < nroots; i++) {
-                run_one(g, algorithm, roots[i], o);
+                run_one(g, algorithm, roots[i], o, out_u32 ? out_u32 + (size_t)i * V : nullptr);
                 total += g->stats.ms;
                 edges += g->stats.traversed_edges;
                 launches += g->stats.launches;
-                if (out_u32) copy_any(out_u32 + (size_t)i * V, g->result, (size_t)V * 4, g->stream);
             }
-            CGB_CUDA_TRY(cudaStreamSynchronize(g->stream));
             g->stats.ms = total;
             g->stats.traversed_edges = edges;
             g->stats.launches = launches;
@@ -485,7 +480,7 @@ cgb_status cgb_policy_collect(cgb_graph* g, int algorithm, uint32_t root, const 
         CGB_CUDA_TRY(cudaMalloc((void**)&ps.save_ctr, sizeof(DevCounters)));
         g->collect = &ps;
         try {
-            run_one(g, algorithm, root, o);
+            run_one(g, algorithm, root, o, nullptr);
         } catch (...) {
             g->collect = nullptr;
             throw;

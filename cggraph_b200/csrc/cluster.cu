@@ -84,11 +84,9 @@ __device__ __forceinline__ void cl_push(ClShared& s, uint32_t buf, const bool (&
         big |= pred[i] && deg[i] > kClPiece;
         edges += pred[i] ? deg[i] : 0;
     }
-    auto spill = [&](uint32_t vv) {
-        if (!take(vv)) return;
-        const uint32_t p = atomicAdd(&st->qlen, 1u);
-        if (p < cap) spill_q[p] = vv;
-        else atomicOr(&st->status, 2u);
+    auto spill = [&](bool pred, uint32_t vv) {  // warp-collective
+        if (!__any_sync(0xffffffffu, pred)) return;
+        warp_append(pred && take(vv), vv, spill_q, &st->qlen, cap, &st->status);
     };
     if (!__any_sync(0xffffffffu, big)) {
         // one entry per vertex
@@ -104,16 +102,14 @@ __device__ __forceinline__ void cl_push(ClShared& s, uint32_t buf, const bool (&
         pos = __shfl_sync(0xffffffffu, pos, 0);
 #pragma unroll
         for (int i = 0; i < N; i++) {
-            if ((m[i] >> lane) & 1u) {
-                const uint32_t at = pos + __popc(m[i] & lanemask_lt());
-                if (at < kClQueue) {
-                    s.list[buf][at] = start[i] | (uint64_t)(deg[i] | kClFirst | kClSingle) << 32;
-                    s.v[buf][at] = v[i];
-                } else {
-                    spill(v[i]);
-                }
+            const uint32_t at = pos + __popc(m[i] & lanemask_lt());
+            const bool mine = (m[i] >> lane) & 1u;
+            if (mine && at < kClQueue) {
+                s.list[buf][at] = start[i] | (uint64_t)(deg[i] | kClFirst | kClSingle) << 32;
+                s.v[buf][at] = v[i];
             }
             pos += __popc(m[i]);
+            if (pos > kClQueue) spill(mine && at >= kClQueue, v[i]);
         }
         return;
     }
@@ -139,7 +135,7 @@ __device__ __forceinline__ void cl_push(ClShared& s, uint32_t buf, const bool (&
             s.v[buf][at] = vv;
         };
         const bool fits = pos + n[i] <= kClQueue;
-        if (n[i] && !fits) spill(v[i]);
+        spill(n[i] && !fits, v[i]);
         if (n[i] <= 4)
             for (uint32_t k = 0; k < n[i]; k++) put(pos + k, k, v[i], start[i], deg[i], fits);
         for (uint32_t todo = __ballot_sync(0xffffffffu, n[i] > 4); todo; todo &= todo - 1) {
@@ -218,7 +214,7 @@ __device__ __forceinline__ bool cl_next_level(cooperative_groups::cluster_group&
             : "memory");
     if (!done) {
         s.gave_up = 1;
-        atomicOr(&st->status, 1u);
+        atomicOr(&st->status, 2u);
     }
     __syncthreads();  // the counts were reset, and all threads agree on gave_up
     return !s.gave_up;
@@ -637,7 +633,7 @@ static ClusterState run_cluster(cgb_graph* g, void (*kern)(P...), A... args)
     ++g->stats.launches;
     CGB_CUDA_TRY(cudaLaunchKernelEx(&cfg, kern, args..., (ClusterState*)g->cluster, h.data()));
     CGB_CUDA_TRY(cudaStreamSynchronize(g->stream));
-    CGB_REQUIRE(!(h[0].status & 1u), CGB_ETIMEOUT, "cluster loop: a level's barrier gave up");
+    CGB_REQUIRE(!(h[0].status & 2u), CGB_ETIMEOUT, "cluster loop: a level's barrier gave up");
     CGB_REQUIRE(!h[0].status, CGB_EOVERFLOW, "cluster loop: queue overflow");
     return h[0];
 }

@@ -1488,8 +1488,7 @@ void ensure_pr(cgb_graph* g)
 
 void count_reached(cgb_graph* g)
 {
-    CGB_CUDA_TRY(cudaMemsetAsync(&g->ctr->reached_edges, 0, sizeof(unsigned long long), g->stream));
-    CGB_CUDA_TRY(cudaMemsetAsync(&g->ctr->reached, 0, sizeof(uint32_t), g->stream));
+    // (its two counters are zero: a run clears them, and nothing else of BFS or SSSP counts in them)
     k_count_reached<<<grid_for(div_up(g->V, 4), kBlock, num_sms() * 8), kBlock, 0, g->stream>>>(g->V, g->value, g->off, g->ctr);
     sync_counters(g);
     g->stats.reached = g->h_ctr->reached;

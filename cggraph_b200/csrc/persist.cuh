@@ -26,8 +26,12 @@ constexpr uint32_t kBarrierSpins = 1u << 22;  // mostly x ~64 ns: gives up after
 // The cluster loops (cluster.cu) take frontiers of at most
 // cgb_tuning.cluster_enter vertices and kClusterEnterEdges out-edges, and
 // return once a frontier exceeds twice the entry size or kClusterExitEdges:
-// beyond, 16 SMs take longer than a host round trip over all of them.
-constexpr uint32_t kClusterEnterEdges = 1u << 17, kClusterExitEdges = 1u << 18;
+// beyond, 16 SMs take longer than a host round trip over all of them.  Entry
+// bounds of 8 k / 16 k / 32 k / 64 k / 128 k edges: SSSP RMAT-18 0.42 / 0.41
+// / 0.41 / 0.43 / 0.43 ms, RMAT-15 0.30 / 0.28 / 0.29 / 0.27 / 0.26, Chung-Lu
+// 5 M edges 0.70 / 0.68 / 0.64 / 0.66 / 0.65, 3000 x 4000 grid 114 / 111 /
+// 102 / 102 / 102; BFS on that grid 33 / 24 / 24 / 24 / 24 ms.
+constexpr uint32_t kClusterEnterEdges = 1u << 15, kClusterExitEdges = 1u << 16;
 
 // Host-visible state of a device-resident loop.
 struct PersistState {
@@ -68,7 +72,7 @@ struct PersistBlock {
 // What a cluster loop reports on exit.
 struct ClusterState {
     uint32_t qlen;      // frontier vertices left in the global queue
-    uint32_t status;    // 1 = a barrier gave up, 2 = queue overflow
+    uint32_t status;    // 1 = queue overflow, 2 = a barrier gave up
     uint32_t levels;    // levels (rounds) run
     uint32_t max_deg;   // longest list of the frontier
     uint32_t found;     // BFS: vertices reached; SSSP: list pieces expanded

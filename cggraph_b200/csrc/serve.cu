@@ -40,7 +40,7 @@
 namespace cgb {
 
 // One run of the single-root engine (capi.cu), with the graph's lock held.
-void run_one(cgb_graph* g, int alg, uint32_t root_or_iters, const cgb_options& o);
+void run_one(cgb_graph* g, int alg, uint32_t root_or_iters, const cgb_options& o, void* out);
 
 constexpr uint32_t kSrvSlots = 64;
 
@@ -1163,7 +1163,7 @@ static void lone_run(cgb_server* s, Group& G, int a, uint32_t k)
         cgb_options o;
         memset(&o, 0, sizeof(o));
         o.struct_size = sizeof(o);
-        run_one(g, G.alg, G.root[k], o);
+        run_one(g, G.alg, G.root[k], o, nullptr);
         CGB_CUDA_TRY(cudaMemcpyAsync(G.region + (size_t)k * g->V, g->value, (size_t)g->V * 4,
                                      cudaMemcpyDeviceToDevice, g->stream));
         CGB_CUDA_TRY(cudaStreamSynchronize(g->stream));

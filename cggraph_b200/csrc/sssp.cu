@@ -204,11 +204,12 @@ struct SsspDenseOp {
 // vertices with one 16-byte load of each array, so a warp covers 128
 // vertices = 4 bitmap words per step; the 8 lanes of a word OR their far
 // bits together, and the first of them writes the word (no atomics: only
-// this warp touches it).  A CTA takes kBlock * 4 consecutive vertices per
-// step and appends the step's next-queue vertices with one atomic.  The next
-// queue's out-edges and the new far bits are counted.
+// this warp touches it).  Next-queue vertices are staged (push.cuh), so warps
+// do not wait for one another.  The next queue's out-edges and the new far
+// bits are counted, and the snapshot is brought up to date where it changed,
+// so that a dense round that follows needs no copy.
 __global__ void __launch_bounds__(kBlock) k_sssp_dense_scan(uint32_t V, const uint32_t* __restrict__ dist,
-                                                            const uint32_t* __restrict__ snap, uint32_t thr,
+                                                            uint32_t* __restrict__ snap, uint32_t thr,
                                                             uint32_t nz, const uint32_t* __restrict__ off,
                                                             uint32_t* far_bm, uint32_t* near_out, uint32_t* near_len,
                                                             uint32_t cap, DevCounters* ctr)
@@ -216,10 +217,13 @@ __global__ void __launch_bounds__(kBlock) k_sssp_dense_scan(uint32_t V, const ui
     const uint32_t lane = lane_id();
     unsigned long long deg_sum = 0;
     uint32_t new_far = 0, touched = 0, max_deg = 0;
+    stage_begin();
+    __syncthreads();
     for (uint64_t b0 = (uint64_t)blockIdx.x * kBlock * 4; b0 < V; b0 += (uint64_t)gridDim.x * kBlock * 4) {
         const uint32_t v0 = (uint32_t)b0 + 4 * threadIdx.x;
         uint32_t dv[4], sv[4], v[4];
-        if (v0 + 3 < V) {
+        const bool whole = (uint64_t)v0 + 3 < V;
+        if (whole) {
             const uint4 a = *reinterpret_cast<const uint4*>(dist + v0);
             const uint4 b = *reinterpret_cast<const uint4*>(snap + v0);
             dv[0] = a.x, dv[1] = a.y, dv[2] = a.z, dv[3] = a.w;
@@ -229,6 +233,15 @@ __global__ void __launch_bounds__(kBlock) k_sssp_dense_scan(uint32_t V, const ui
             for (int k = 0; k < 4; k++) {
                 dv[k] = v0 + k < V ? dist[v0 + k] : kValueMax;
                 sv[k] = v0 + k < V ? snap[v0 + k] : kValueMax;
+            }
+        }
+        if (dv[0] != sv[0] || dv[1] != sv[1] || dv[2] != sv[2] || dv[3] != sv[3]) {
+            if (whole) {
+                *reinterpret_cast<uint4*>(snap + v0) = make_uint4(dv[0], dv[1], dv[2], dv[3]);
+            } else {
+#pragma unroll
+                for (int k = 0; k < 4; k++)
+                    if (v0 + k < V) snap[v0 + k] = dv[k];
             }
         }
         bool to_near[4];
@@ -261,8 +274,10 @@ __global__ void __launch_bounds__(kBlock) k_sssp_dense_scan(uint32_t V, const ui
             deg_sum += hi[k] - lo[k];
             max_deg = max(max_deg, hi[k] - lo[k]);
         }
-        block_append_n<4>(to_near, v, near_out, near_len, cap, &ctr->overflow);
+        stage_append_n<4>(to_near, v, near_out, near_len, cap, &ctr->overflow);
     }
+    __syncthreads();
+    stage_end(near_out, near_len, cap, &ctr->overflow);
     deg_sum = warp_sum(deg_sum);
     touched = warp_sum(touched);
     new_far = warp_sum(new_far);
@@ -433,6 +448,7 @@ static void sssp_loop(cgb_graph* g, uint32_t root, uint32_t delta, const cgb_opt
     const bool grid_fits = tail_allowed && g->max_degree < g->tune.persist_deg;
     const bool cluster_fits = tail_allowed && g->tune.cluster_enter > 0 && cluster_loop_ctas() > 0;
     bool tail_delta_chosen = pol == nullptr;
+    bool snapshot_ok = false;  // stamp[] holds the distances (dense rounds)
     enum { kNoTail, kClusterTail, kGridTail };
     auto tail_kind = [&]() {
         if (cluster_fits && nnear <= std::min(g->tune.cluster_enter, g->tune.persist_enter) &&
@@ -446,6 +462,7 @@ static void sssp_loop(cgb_graph* g, uint32_t root, uint32_t delta, const cgb_opt
     auto device_tail = [&]() -> bool {
         const int kind = tail_kind();
         if (kind == kNoTail) return false;
+        snapshot_ok = false;
         const uint32_t max_rounds = (uint32_t)std::min<uint64_t>(max_iters - iters, 1u << 30);
         if (timing) ktimer_begin(g, CGB_K_PUSH);
         const SsspTail t =
@@ -482,7 +499,9 @@ static void sssp_loop(cgb_graph* g, uint32_t root, uint32_t delta, const cgb_opt
                             (uint32_t)std::min<uint64_t>(thr, kValueMax), g->q[out], &g->ctr->qlen[out], far_bm,
                             g->aux_bm);
         } else if (dense) {
-            CGB_CUDA_TRY(cudaMemcpyAsync(g->stamp, g->value, (size_t)V * 4, cudaMemcpyDeviceToDevice, g->stream));
+            // the scan of a dense round leaves the snapshot up to date for the next one
+            if (!snapshot_ok)
+                CGB_CUDA_TRY(cudaMemcpyAsync(g->stamp, g->value, (size_t)V * 4, cudaMemcpyDeviceToDevice, g->stream));
             SsspDenseOp<kHasW> op{g->off, g->dst, g->w, g->value};
             launch_push(g, g->q[cur], (uint32_t)nnear, op, false);
             ++g->stats.launches;
@@ -497,6 +516,7 @@ static void sssp_loop(cgb_graph* g, uint32_t root, uint32_t delta, const cgb_opt
                         variant == kRoundPushChunked ? kExpandChunked : kExpandBinned);
         }
         if (timing) ktimer_end(g);
+        snapshot_ok = dense && !collect;  // (the trials of a sample restore the distances)
     };
     int last_variant = kRoundPush;
     bool have_round_out = false;  // the policy's outputs for the next round were read back
