@@ -60,11 +60,11 @@ __global__ void __launch_bounds__(kBlock) k_ms_finalize(const uint32_t* __restri
                                                         unsigned long long* fnext, uint32_t* level_out, uint32_t V,
                                                         uint32_t lvl, uint32_t nz, uint32_t* qact, uint32_t* qact_len,
                                                         uint32_t cap, DevCounters* ctr, const uint32_t* start,
-                                                        unsigned long long* alive)
+                                                        unsigned long long* alive, const uint32_t* __restrict__ off)
 {
     if (n_ptr) n = *n_ptr;
     const uint32_t n_round = (n + 31u) & ~31u;
-    unsigned long long live = 0;
+    unsigned long long live = 0, edges = 0;
     for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n_round; i += gridDim.x * blockDim.x) {
         bool act = false;
         uint32_t u = 0;
@@ -82,15 +82,30 @@ __global__ void __launch_bounds__(kBlock) k_ms_finalize(const uint32_t* __restri
                 if (act) {
                     fnext[u] = x;
                     live |= x;
+                    if (off) edges += off[u + 1] - off[u];
                 }
             }
         }
         warp_append(act, u, qact, qact_len, cap, &ctr->overflow);
     }
+    if (off) {
+        edges = warp_sum(edges);
+        if (lane_id() == 0 && edges) atomicAdd(&ctr->medges, edges);
+    }
     if (alive) {
         live = warp_or(live);
         if (lane_id() == 0 && live) atomicOr(alive, live);
     }
+}
+
+// The counters of the next level: one launch, not a memset each.
+__global__ void k_ms_level_reset(DevCounters* ctr, int nxt)
+{
+    ctr->qlen[nxt] = 0;
+    ctr->alive = 0;
+    ctr->found = 0;
+    ctr->chunk_len = 0;
+    ctr->medges = 0;
 }
 
 // Clears the frontier masks of the vertices of a queue.
@@ -425,52 +440,49 @@ void run_msbfs(cgb_graph* g, const uint32_t* d_roots, uint32_t n, uint32_t* leve
     ++g->stats.launches;
     k_ms_roots<<<1, 64, 0, g->stream>>>(d_roots, n, V, b.seen, b.front[0], level_out, g->q[0], &g->ctr->qlen[0], g->nz,
                                        &g->ctr->alive);
+    // Each level is queued whole -- its kernels read the counts of the ones
+    // before them on the device, and the next frontier's out-edges (the next
+    // direction choice) are counted on the way -- and ends with one read-back.
+    k_ms_degree_sum<<<1, kBlock, 0, g->stream>>>(g->q[0], 0, &g->ctr->qlen[0], g->off, g->ctr);
+    ++g->stats.launches;
     sync_counters(g);
     uint64_t nact = g->h_ctr->qlen[0];
     // Roots with vertices in the current frontier.  Bottom-up looks only
     // for these: a root whose traversal has ended (a small component) would
     // otherwise keep every vertex scanning its whole in-list.
     unsigned long long live = g->h_ctr->alive & full;
+    uint64_t level_edges = g->h_ctr->medges;
     int cur = 0;
     uint32_t lvl = 0;
     while (nact > 0) {
         CGB_REQUIRE(lvl <= V, CGB_ETIMEOUT, "multi-root BFS level bound exceeded");
         // direction: out-edges of the active vertices against the graph's edges
-        CGB_CUDA_TRY(cudaMemsetAsync(&g->ctr->medges, 0, 8, g->stream));
-        ++g->stats.launches;
-        k_ms_degree_sum<<<grid_for(nact, kBlock, num_sms() * 8), kBlock, 0, g->stream>>>(g->q[cur], (uint32_t)nact,
-                                                                                      nullptr, g->off, g->ctr);
-        sync_counters(g);
-        const bool pull = (double)g->h_ctr->medges * alpha > (double)g->E;
+        const bool pull = (double)level_edges * alpha > (double)g->E;
         const bool tracing = (g->flags & CGB_FLAG_TRACE) != 0;
-        const uint64_t level_edges = g->h_ctr->medges;
         if (tracing) CGB_CUDA_TRY(cudaEventRecord(g->ev_iter[0], g->stream));
         const int nxt = cur ^ 1;
         unsigned long long* fcur = b.front[cur];
         unsigned long long* fnxt = b.front[nxt];
-        CGB_CUDA_TRY(cudaMemsetAsync(&g->ctr->qlen[nxt], 0, 4, g->stream));
-        CGB_CUDA_TRY(cudaMemsetAsync(&g->ctr->alive, 0, 8, g->stream));
+        ++g->stats.launches;
+        k_ms_level_reset<<<1, 1, 0, g->stream>>>(g->ctr, nxt);
         if (pull) {
             MsBuArgs ba{V, g->in_off, g->in_src, fcur, b.seen, fnxt, b.next, live, level_out, lvl + 1, g->nz,
                         g->q[nxt], &g->ctr->qlen[nxt], V, g->ctr, nullptr, &g->ctr->alive, b.heavy_w, b.heavy_b,
                         b.heavy_len, b.cap_b, b.hub_chunks, b.cap_c};
             ms_bottom_up(ba, g->stream, &g->stats.launches);
+            ++g->stats.launches;
+            k_ms_degree_sum<<<gridV, kBlock, 0, g->stream>>>(g->q[nxt], 0, &g->ctr->qlen[nxt], g->off, g->ctr);
             g->stats.pulls_bu++;
         } else {
             // expansion into next[]: touched vertices are queued once in stamp[]
-            CGB_CUDA_TRY(cudaMemsetAsync(&g->ctr->found, 0, 4, g->stream));
-            CGB_CUDA_TRY(cudaMemsetAsync(&g->ctr->chunk_len, 0, 4, g->stream));
             MsTdOp op{g->off, g->dst, fcur, b.seen, b.next, g->stamp, &g->ctr->found, V, g->ctr};
             launch_push(g, g->q[cur], (uint32_t)nact, op, false);
-            sync_counters(g);
-            CGB_REQUIRE(!g->h_ctr->overflow, CGB_EOVERFLOW, "multi-root BFS queue overflow");
-            const uint32_t touched = g->h_ctr->found;
-            if (touched) {
-                ++g->stats.launches;
-                k_ms_finalize<<<grid_for(touched, kBlock, num_sms() * 8), kBlock, 0, g->stream>>>(
-                    g->stamp, touched, nullptr, b.seen, b.next, fnxt, level_out, V, lvl + 1, g->nz, g->q[nxt],
-                    &g->ctr->qlen[nxt], V, g->ctr, nullptr, &g->ctr->alive);
-            }
+            ++g->stats.launches;
+            // at most one touched vertex per out-edge
+            k_ms_finalize<<<grid_for(std::min<uint64_t>(V, level_edges), kBlock, num_sms() * 8), kBlock, 0,
+                            g->stream>>>(g->stamp, 0, &g->ctr->found, b.seen, b.next, fnxt, level_out, V, lvl + 1,
+                                         g->nz, g->q[nxt], &g->ctr->qlen[nxt], V, g->ctr, nullptr, &g->ctr->alive,
+                                         g->off);
             g->stats.pushes_td++;
         }
         ++g->stats.launches;
@@ -491,6 +503,7 @@ void run_msbfs(cgb_graph* g, const uint32_t* d_roots, uint32_t n, uint32_t* leve
         }
         nact = g->h_ctr->qlen[nxt];
         live = g->h_ctr->alive;
+        level_edges = g->h_ctr->medges;
         cur = nxt;
         lvl++;
     }

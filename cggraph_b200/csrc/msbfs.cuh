@@ -95,12 +95,14 @@ struct MsTdOp {
     __device__ __forceinline__ void block_end() const { stage_end(qout, qlen, cap, &ctr->overflow); }
 };
 
-// n_ptr (optional) replaces n by a device-resident count.
+// n_ptr (optional) replaces n by a device-resident count; off (optional):
+// the next frontier's out-edges are added to ctr->medges.
 __global__ void k_ms_finalize(const uint32_t* __restrict__ q, uint32_t n, const uint32_t* n_ptr,
                               unsigned long long* seen,
                               unsigned long long* next, unsigned long long* fnext, uint32_t* level_out, uint32_t V,
                               uint32_t lvl, uint32_t nz, uint32_t* qact, uint32_t* qact_len, uint32_t cap,
-                              DevCounters* ctr, const uint32_t* start, unsigned long long* alive);
+                              DevCounters* ctr, const uint32_t* start, unsigned long long* alive,
+                              const uint32_t* __restrict__ off);
 __global__ void k_ms_clear(const uint32_t* __restrict__ q, uint32_t n, unsigned long long* f);
 __global__ void k_ms_fill(uint64_t n, uint32_t* a, uint32_t value);
 __global__ void k_ms_degree_sum(const uint32_t* __restrict__ q, uint32_t n, const uint32_t* n_ptr,

@@ -184,7 +184,32 @@ static MsspCounters mssp_sync(cgb_graph* g)
     return *b.h;
 }
 
-__global__ void k_mssp_set(uint32_t* a, uint32_t value) { *a = value; }
+// Before a near round: the queue that was built becomes the one to expand.
+__global__ void k_mssp_round_begin(MsspCounters* c)
+{
+    c->nq_in = c->nq_out;
+    c->nq_out = 0;
+    c->ndesc = 0;
+    if (c->nq_in) c->rounds++;
+}
+
+// Before and after a split of the far list.
+__global__ void k_mssp_split_begin(MsspCounters* c)
+{
+    c->nq_out = 0;
+    c->min_far = kValueMax;
+    c->nfar_next = 0;
+}
+
+__global__ void k_mssp_split_end(MsspCounters* c) { c->nfar_live = c->nfar_next; }
+
+// On graphs without hubs, whose queues grow slowly, several near rounds are
+// queued between two read-backs while the queue is small: a round without
+// work is three empty kernels, a read-back with its synchronisation costs
+// more than that.
+constexpr uint32_t kMsspSmall = 16384;  // vertices queued
+constexpr int kMsspAhead = 4;
+constexpr uint32_t kMsspMeshDeg = 64;   // longest list of such a graph is below this
 
 uint32_t mssp_default_delta(cgb_graph* g)
 {
@@ -208,63 +233,61 @@ void run_mssp(cgb_graph* g, const uint32_t* d_roots, uint32_t n, uint32_t* out, 
     ++g->stats.launches;
     k_mssp_roots<<<1, kMsRoots, 0, g->stream>>>(d_roots, n, b.dist, b.pend, g->q[0], b.c);
     uint32_t nq = mssp_sync(g).nq_out, nfar = 0;
-    CGB_CUDA_TRY(cudaMemcpyAsync(&b.c->nq_in, &b.c->nq_out, 4, cudaMemcpyDeviceToDevice, g->stream));
     int cur = 0, fcur = 0;  // near queue / far list holding the live entries
     uint64_t thr = delta;
     bool last_split_empty = false;
     uint32_t min_far = kValueMax;
-    uint64_t rounds = 0;
+    uint64_t splits = 0, rounds = 0;
     while (nq > 0 || nfar > 0) {
-        CGB_REQUIRE(++rounds <= 4ull * V + 64, CGB_ETIMEOUT, "multi-root SSSP round bound exceeded");
-        const int nxt = cur ^ 1;
-        CGB_CUDA_TRY(cudaMemsetAsync(&b.c->nq_out, 0, 4, g->stream));
+        CGB_REQUIRE(splits + rounds <= 4ull * V + 64, CGB_ETIMEOUT, "multi-root SSSP round bound exceeded");
         if (nq > 0) {
-            // near round at threshold thr: q[cur] -> q[nxt]
+            // near rounds at threshold thr: q[cur] -> q[cur ^ 1], the counts kept on the device
             const uint32_t t32 = (uint32_t)std::min<uint64_t>(thr, 0xFFFFFFFFull);
-            CGB_CUDA_TRY(cudaMemsetAsync(&b.c->ndesc, 0, 4, g->stream));
-            ++g->stats.launches;
-            k_mssp_desc<<<grid_for(nq, kBlock, num_sms() * 8), kBlock, 0, g->stream>>>(g->q[cur], &b.c->nq_in, g->off,
-                                                                                    b.pend, b.maskq, b.desc,
-                                                                                    b.desc_cap, b.c,
-                                                                                    g->tune.ms_edges);
-            ++g->stats.launches;
-            mssp_expand(g->w != nullptr, num_sms() * 8, g->stream, b.desc, b.c, b.maskq, g->dst, g->w, b.dist, b.pend,
-                        b.farm, g->q[nxt], &b.c->nq_out, b.far_list[fcur], &b.c->nfar_live, V, t32, nullptr,
-                        nullptr);
+            const bool ahead = nq <= kMsspSmall && g->max_degree < kMsspMeshDeg;
+            const uint32_t grid = num_sms() * (ahead ? 4 : 8);
+            for (int k = 0; k < (ahead ? kMsspAhead : 1); k++) {
+                g->stats.launches += 3;
+                k_mssp_round_begin<<<1, 1, 0, g->stream>>>(b.c);
+                k_mssp_desc<<<ahead ? grid : grid_for(nq, kBlock, grid), kBlock, 0, g->stream>>>(
+                    g->q[cur], &b.c->nq_in, g->off, b.pend, b.maskq, b.desc, b.desc_cap, b.c, g->tune.ms_edges);
+                mssp_expand(g->w != nullptr, grid, g->stream, b.desc, b.c, b.maskq, g->dst, g->w, b.dist, b.pend,
+                            b.farm, g->q[cur ^ 1], &b.c->nq_out, b.far_list[fcur], &b.c->nfar_live, V, t32, nullptr,
+                            nullptr);
+                cur ^= 1;
+            }
             const MsspCounters h = mssp_sync(g);
             nq = h.nq_out;
             nfar = h.nfar_live;
+            g->stats.pushes_td += h.rounds - rounds;
+            rounds = h.rounds;
             last_split_empty = false;
-            g->stats.pushes_td++;
         } else {
-            // split of the far list at the next bucket [thr, hi): far_list[fcur] -> q[nxt] + far_list[fcur ^ 1]
+            // split of the far list at the next bucket [thr, hi): far_list[fcur] -> q[cur] + far_list[fcur ^ 1]
             uint64_t hi = thr + delta;
             if (last_split_empty && min_far != kValueMax)
                 hi = std::max<uint64_t>(hi, ((uint64_t)min_far / delta + 1) * delta);
             const uint32_t lo32 = (uint32_t)std::min<uint64_t>(thr, 0xFFFFFFFFull);
             const uint32_t hi32 = (uint32_t)std::min<uint64_t>(hi, 0xFFFFFFFFull);
-            k_mssp_set<<<1, 1, 0, g->stream>>>(&b.c->min_far, kValueMax);
-            CGB_CUDA_TRY(cudaMemsetAsync(&b.c->nfar_next, 0, 4, g->stream));
-            ++g->stats.launches;
+            g->stats.launches += 3;
+            k_mssp_split_begin<<<1, 1, 0, g->stream>>>(b.c);
             k_mssp_split<<<grid_for(nfar, kBlock / 32, num_sms() * 8), kBlock, 0, g->stream>>>(
-                b.far_list[fcur], &b.c->nfar_live, b.dist, b.pend, b.farm, g->q[nxt], &b.c->nq_out,
+                b.far_list[fcur], &b.c->nfar_live, b.dist, b.pend, b.farm, g->q[cur], &b.c->nq_out,
                 b.far_list[fcur ^ 1], &b.c->nfar_next, V, lo32, hi32, nullptr, nullptr, ~0ull, nullptr, nullptr, b.c);
+            k_mssp_split_end<<<1, 1, 0, g->stream>>>(b.c);
             const MsspCounters h = mssp_sync(g);
             nq = h.nq_out;
             nfar = h.nfar_next;
             min_far = h.min_far;
             fcur ^= 1;
-            k_mssp_set<<<1, 1, 0, g->stream>>>(&b.c->nfar_live, nfar);
             thr = hi;
             last_split_empty = nq == 0;
+            splits++;
         }
-        cur = nxt;
-        CGB_CUDA_TRY(cudaMemcpyAsync(&b.c->nq_in, &b.c->nq_out, 4, cudaMemcpyDeviceToDevice, g->stream));
     }
     ++g->stats.launches;
     CGB_CUDA_TRY(cudaMemsetAsync(&g->ctr->reached_edges, 0, 8, g->stream));
     k_mssp_out<<<num_sms() * 16, kBlock, 0, g->stream>>>(b.dist, V, n, out, g->off, g->ctr);
-    g->stats.iterations = rounds;
+    g->stats.iterations = rounds + splits;
     g->stats.sssp_delta = delta;
 }
 

@@ -17,6 +17,7 @@ struct MsspCounters {
     uint32_t ndesc;        // descriptors of the round
     uint32_t min_far;      // smallest far distance >= hi seen by a split
     uint32_t overflow;
+    uint32_t rounds;       // near rounds that had work
     unsigned long long relax;  // relaxations (root, edge) that lowered the distance read
 };
 

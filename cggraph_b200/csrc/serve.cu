@@ -774,7 +774,7 @@ static void bfs_issue(cgb_server* s, Group& G)
         k_ms_finalize<<<num_sms() * 8, kBlock, 0, st>>>(G.touched, 0, &g->ctr->found, G.mb->seen, G.mb->next,
                                                      G.mb->front[nxt], G.region, V, lvl, g->nz, G.q[nxt],
                                                      &g->ctr->qlen[nxt], V, g->ctr, G.d_up->start,
-                                                     &G.d_stats->alive[0]);
+                                                     &G.d_stats->alive[0], nullptr);
     }
     k_ms_clear<<<grid_for(G.nact, kBlock, num_sms() * 8), kBlock, 0, st>>>(G.q[cur], G.nact, G.mb->front[cur]);
     k_ms_degree_sum<<<num_sms() * 4, kBlock, 0, st>>>(G.q[nxt], 0, &g->ctr->qlen[nxt], g->off, g->ctr);
