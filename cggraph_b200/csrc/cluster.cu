@@ -42,14 +42,14 @@ constexpr int kClBatch = 4;
 
 // What a CTA tells the others about the level it has built.  `word` packs
 // the entries (at most kClQueue, so that the cluster's sum stays below 2^20)
-// and the flags, one count each, so that one reduction adds them all.
-constexpr uint32_t kEntryMask = (1u << 20) - 1, kSpill = 1u << 20, kSpillMask = 31u << 20, kFar = 1u << 25;
+// and the spill flag, so that one reduction adds both.
+constexpr uint32_t kEntryMask = (1u << 20) - 1, kSpill = 1u << 20;
 
 struct __align__(16) ClCounts {
-    uint32_t word;     // entries, spill, far
+    uint32_t word;     // entries, spill
     uint32_t medges;   // out-edges of the next frontier
     uint32_t min_far;  // SSSP split: smallest distance left in the far bitmap,
-    uint32_t kept;     // and the vertices left
+    uint32_t far;      // and the vertices left; SSSP round: far bits set (a vertex may count twice)
 };
 
 struct ClShared {
@@ -57,13 +57,13 @@ struct ClShared {
     uint32_t v[2][kClQueue];
     ClCounts from[2][kClMaxCtas];
     uint64_t arrived[2];  // mbarriers: the counts of a level have come from every CTA
-    uint32_t entries, medges, far, min_far, kept;  // of the level being built
+    uint32_t entries, medges, far, min_far;  // of the level being built
     uint32_t gave_up;
 };
 
 __device__ __forceinline__ void cl_reset(ClShared& s)
 {
-    s.entries = s.medges = s.far = s.kept = 0;
+    s.entries = s.medges = s.far = 0;
     s.min_far = kValueMax;
 }
 
@@ -181,8 +181,7 @@ __device__ __forceinline__ bool cl_next_level(cooperative_groups::cluster_group&
     const uint32_t mbar = (uint32_t)__cvta_generic_to_shared(&s.arrived[buf]);
     if (threadIdx.x < 32) {
         const uint32_t n = s.entries;
-        const ClCounts c{min(n, kClQueue) | (n > kClQueue ? kSpill : 0) | (s.far ? kFar : 0), s.medges, s.min_far,
-                         s.kept};
+        const ClCounts c{min(n, kClQueue) | (n > kClQueue ? kSpill : 0), s.medges, s.min_far, s.far};
         __syncwarp();
         if (threadIdx.x == 0) {
             cl_reset(s);
@@ -199,7 +198,7 @@ __device__ __forceinline__ bool cl_next_level(cooperative_groups::cluster_group&
             asm("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(to_bar) : "r"(mbar), "r"(threadIdx.x));
             asm volatile(
                 "st.async.shared::cluster.mbarrier::complete_tx::bytes.v4.b32 [%0], {%1, %2, %3, %4}, [%5];" ::"r"(to),
-                "r"(c.word), "r"(c.medges), "r"(c.min_far), "r"(c.kept), "r"(to_bar)
+                "r"(c.word), "r"(c.medges), "r"(c.min_far), "r"(c.far), "r"(to_bar)
                 : "memory");
         }
     }
@@ -326,7 +325,7 @@ __global__ void __launch_bounds__(kClThreads, 1)
         const ClCounts c = lane_id() < ctas ? s.from[buf][lane_id()] : ClCounts{};
         word = __reduce_add_sync(0xffffffffu, c.word);
         scout = __reduce_add_sync(0xffffffffu, c.medges);
-        if (!ok || (word & kEntryMask) == 0 || (word & kSpillMask) || (word & kEntryMask) > nf_exit || scout > scout_exit ||
+        if (!ok || (word & kEntryMask) == 0 || (word & ~kEntryMask) || (word & kEntryMask) > nf_exit || scout > scout_exit ||
             it >= max_levels)
             break;
         scouts += scout;
@@ -399,7 +398,7 @@ __global__ void __launch_bounds__(kClThreads, 1)
                    uint32_t* dist, uint32_t* stamp, uint32_t* far_bm, uint32_t words, const uint32_t* q_in,
                    uint32_t* q_out, uint32_t cap, uint32_t nz, uint32_t nf, unsigned long long thr, uint32_t nfar,
                    unsigned long long bucket_lo, uint32_t delta, uint32_t nf_exit, uint32_t scout_exit,
-                   uint32_t max_rounds, uint32_t* far_len_out, ClusterState* st, ClusterState* host)
+                   uint32_t far_exit, uint32_t max_rounds, uint32_t* far_len_out, ClusterState* st, ClusterState* host)
 {
     extern __shared__ __align__(16) unsigned char smem[];
     ClShared& s = *reinterpret_cast<ClShared*>(smem);
@@ -412,22 +411,24 @@ __global__ void __launch_bounds__(kClThreads, 1)
     // a vertex goes to the global queue once (its short list may be queued twice)
     const uint32_t kLeft = 0xFFFFFFFFu;
     auto take = [&](uint32_t v) { return atomicExch(stamp + v, kLeft) != kLeft; };
-    bool any_far = nfar > 0, after_split = false;
+    uint32_t far = nfar;  // at least the far bitmap's population
+    bool after_split = false;
     for (;; it++) {
         const uint32_t buf = it & 1;
         ClCounts c{0, 0, kValueMax, 0};
         if (lane < ctas) c = s.from[buf][lane];
         word = __reduce_add_sync(0xffffffffu, c.word);
         scout = __reduce_add_sync(0xffffffffu, c.medges);
-        if (after_split) any_far = __any_sync(0xffffffffu, c.kept != 0);
-        else any_far = any_far || word >= kFar;
+        const uint32_t far_level = __reduce_add_sync(0xffffffffu, c.far);
+        far = after_split ? far_level : far + min(far_level, 0xFFFFFFFFu - far);
         const uint32_t entries = word & kEntryMask;
-        if (!ok || (entries == 0 && !any_far)) break;
-        if ((word & kSpillMask) || entries > nf_exit || scout > scout_exit || it >= max_rounds) break;
+        // a large far set is split by the whole machine
+        if (!ok || (entries == 0 && (far == 0 || far > far_exit))) break;
+        if ((word & ~kEntryMask) || entries > nf_exit || scout > scout_exit || it >= max_rounds) break;
         uint32_t edges = 0;
         if (entries) {
             const uint32_t bound = (uint32_t)min(thr, (unsigned long long)kValueMax);
-            bool far_set = false;
+            uint32_t far_set = 0;
             cl_for_entries(cluster, s, buf, [&](const uint32_t* entry, uint32_t start, uint32_t len, bool single) {
                 const uint32_t v = len ? *entry : 0u;
                 const uint32_t du = len ? __ldcg(dist + v) : 0u;
@@ -436,7 +437,7 @@ __global__ void __launch_bounds__(kClThreads, 1)
                 added += len && !again ? 1u : 0u;
                 for (uint32_t b = 0; __any_sync(0xffffffffu, b < len); b += kClBatch) {
                     uint32_t d[kClBatch], nd[kClBatch], old[kClBatch], lo[kClBatch], dg[kClBatch];
-                    bool near[kClBatch], far[kClBatch];
+                    bool near[kClBatch], to_far[kClBatch];
 #pragma unroll
                     for (int i = 0; i < kClBatch; i++) {
                         const bool in = b + i < len;
@@ -461,7 +462,7 @@ __global__ void __launch_bounds__(kClThreads, 1)
                     for (int i = 0; i < kClBatch; i++) {
                         const bool better = nd[i] < old[i] && d[i] < nz;
                         near[i] = better && nd[i] < bound;
-                        far[i] = better && !near[i];
+                        to_far[i] = better && !near[i];
                         dg[i] -= lo[i];
                         // the entries of a longer list do not know of one another: it is queued once
                         if (near[i] && dg[i] > kClPiece) {
@@ -471,13 +472,14 @@ __global__ void __launch_bounds__(kClThreads, 1)
                     }
 #pragma unroll
                     for (int i = 0; i < kClBatch; i++) {
-                        if (far[i]) atomicOr(far_bm + (d[i] >> 5), 1u << (d[i] & 31u));
-                        far_set |= far[i];
+                        if (to_far[i]) atomicOr(far_bm + (d[i] >> 5), 1u << (d[i] & 31u));
+                        far_set += to_far[i] ? 1u : 0u;
                     }
                     cl_push<kClBatch>(s, buf ^ 1, near, d, lo, dg, q_out, cap, st, edges, take);
                 }
             });
-            if (far_set) s.far = 1;
+            far_set = __reduce_add_sync(0xffffffffu, far_set);
+            if (lane == 0 && far_set) atomicAdd(&s.far, far_set);
             after_split = false;
         } else {
             // next bucket [thr, hi); after a split that found nothing, jump
@@ -534,7 +536,7 @@ __global__ void __launch_bounds__(kClThreads, 1)
             mn = __reduce_min_sync(0xffffffffu, mn);
             if (lane == 0) {
                 if (mn != kValueMax) atomicMin(&s.min_far, mn);
-                if (kept) atomicAdd(&s.kept, kept);
+                if (kept) atomicAdd(&s.far, kept);
             }
             after_split = true;
         }
@@ -543,7 +545,7 @@ __global__ void __launch_bounds__(kClThreads, 1)
     if (it > 0) cl_flush(s, it & 1, rank, off, q_out, cap, st, take);
     added = __reduce_add_sync(0xffffffffu, added);
     if (lane == 0 && added) atomicAdd(&st->found, added);
-    if (any_far) {
+    if (far) {
         uint32_t pop = 0;
         for (uint32_t i = rank * kClThreads + threadIdx.x; i < words; i += ctas * kClThreads)
             pop += __popc(__ldcg(far_bm + i));
@@ -657,14 +659,16 @@ PersistResult bfs_cluster(cgb_graph* g, uint32_t cur, uint32_t nf, uint32_t leve
 }
 
 SsspTail sssp_cluster(cgb_graph* g, uint32_t cur, uint32_t nf, uint64_t thr, uint32_t nfar, uint64_t bucket_lo,
-                      uint32_t* far_bm, uint32_t delta, uint32_t nf_exit, uint32_t scout_exit, uint32_t max_rounds)
+                      uint32_t* far_bm, uint32_t delta, uint32_t nf_exit, uint32_t scout_exit, uint32_t far_exit,
+                      uint32_t max_rounds)
 {
     CGB_CUDA_TRY(cudaMemsetAsync(g->stamp, 0, (size_t)g->V * 4, g->stream));
     const ClusterState h =
         run_cluster(g, g->w ? k_sssp_cluster<true> : k_sssp_cluster<false>, (const uint32_t*)g->off,
                     (const uint32_t*)g->dst, (const uint32_t*)g->w, g->value, g->stamp, far_bm, g->words(),
                     (const uint32_t*)g->q[cur], g->q[cur ^ 1], g->V, g->nz, nf, (unsigned long long)thr, nfar,
-                    (unsigned long long)bucket_lo, delta, nf_exit, scout_exit, max_rounds, &g->ctr->far_len[0]);
+                    (unsigned long long)bucket_lo, delta, nf_exit, scout_exit, far_exit, max_rounds,
+                    &g->ctr->far_len[0]);
     SsspTail t;
     t.r.levels = h.levels;
     t.r.cur = h.levels ? cur ^ 1 : cur;

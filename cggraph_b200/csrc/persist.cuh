@@ -32,6 +32,10 @@ constexpr uint32_t kBarrierSpins = 1u << 22;  // mostly x ~64 ns: gives up after
 // 5 M edges 0.70 / 0.68 / 0.64 / 0.66 / 0.65, 3000 x 4000 grid 114 / 111 /
 // 102 / 102 / 102; BFS on that grid 33 / 24 / 24 / 24 / 24 ms.
 constexpr uint32_t kClusterEnterEdges = 1u << 15, kClusterExitEdges = 1u << 16;
+// Vertices in the far bitmap above which SSSP buckets are not split in the
+// cluster: the split reads every far distance (RMAT-24 with a bucket width of
+// 16, millions of far vertices: 10.1 ms in the cluster, 4.0 ms without).
+constexpr uint32_t kClusterFar = 1u << 17;
 
 // Host-visible state of a device-resident loop.
 struct PersistState {
@@ -139,9 +143,10 @@ SsspTail sssp_device_tail(cgb_graph* g, uint32_t cur, uint32_t nf, uint32_t max_
 
 // The same in a cluster loop, which leaves when a frontier exceeds nf_exit
 // vertices or scout_exit out-edges (r.scout: the out-edges of the frontier it
-// returns).
+// returns), and before a split with more than far_exit far vertices.
 SsspTail sssp_cluster(cgb_graph* g, uint32_t cur, uint32_t nf, uint64_t thr, uint32_t nfar, uint64_t bucket_lo,
-                      uint32_t* far_bm, uint32_t delta, uint32_t nf_exit, uint32_t scout_exit, uint32_t max_rounds);
+                      uint32_t* far_bm, uint32_t delta, uint32_t nf_exit, uint32_t scout_exit, uint32_t far_exit,
+                      uint32_t max_rounds);
 
 // Warp-aggregated append into a device-resident loop's queue (every lane
 // calls it); past `cap` the loop's status records an overflow.

@@ -442,8 +442,9 @@ static void sssp_loop(cgb_graph* g, uint32_t root, uint32_t delta, const cgb_opt
     // run).  Both run near rounds and bucket splits until the run ends or a
     // frontier outgrows their bounds (then the rounds below take over again),
     // and keep the current delta for the buckets they split.  Under the
-    // learned schedule they wait for the first bucket boundary, so that the
-    // network picks that delta.
+    // learned schedule the network picks that delta at the first bucket
+    // boundary: until then the cluster loop returns there, and the grid loop
+    // waits.
     const bool tail_allowed = !tracing && o.schedule != CGB_SCHED_FIXED && g->tune.persist_enter > 0;
     const bool grid_fits = tail_allowed && g->max_degree < g->tune.persist_deg;
     const bool cluster_fits = tail_allowed && g->tune.cluster_enter > 0 && cluster_loop_ctas() > 0;
@@ -452,9 +453,9 @@ static void sssp_loop(cgb_graph* g, uint32_t root, uint32_t delta, const cgb_opt
     enum { kNoTail, kClusterTail, kGridTail };
     auto tail_kind = [&]() {
         if (cluster_fits && nnear <= std::min(g->tune.cluster_enter, g->tune.persist_enter) &&
-            near_edges <= kClusterEnterEdges)
+            near_edges <= kClusterEnterEdges && (nnear > 0 || nfar <= kClusterFar))
             return kClusterTail;
-        if (grid_fits && nnear <= g->tune.persist_enter && near_maxdeg < g->tune.persist_deg) return kGridTail;
+        if (grid_fits && tail_delta_chosen && nnear <= g->tune.persist_enter && near_maxdeg < g->tune.persist_deg) return kGridTail;
         return kNoTail;
     };
     // Runs the loop that takes the near queue (or, when it is empty, the next
@@ -468,7 +469,8 @@ static void sssp_loop(cgb_graph* g, uint32_t root, uint32_t delta, const cgb_opt
         const SsspTail t =
             kind == kClusterTail
                 ? sssp_cluster(g, cur, (uint32_t)nnear, thr, (uint32_t)nfar, bucket_lo, far_bm, delta,
-                               std::min(g->tune.persist_enter, 2 * g->tune.cluster_enter), kClusterExitEdges, max_rounds)
+                               std::min(g->tune.persist_enter, 2 * g->tune.cluster_enter), kClusterExitEdges,
+                               tail_delta_chosen ? kClusterFar : 0, max_rounds)
                 : sssp_device_tail(g, cur, (uint32_t)nnear, near_maxdeg, thr, (uint32_t)nfar, bucket_lo, far_bm, delta,
                                    g->tune.persist_enter, g->tune.persist_deg, max_rounds);
         if (timing) ktimer_end(g);
@@ -547,7 +549,7 @@ static void sssp_loop(cgb_graph* g, uint32_t root, uint32_t delta, const cgb_opt
     auto near_rounds = [&]() {
         while (nnear > 0) {
             CGB_REQUIRE(iters < max_iters, CGB_ETIMEOUT, "SSSP iteration budget exhausted");
-            if (!collect && tail_delta_chosen && device_tail()) {
+            if (!collect && device_tail()) {
                 have_round_out = false;
                 continue;
             }
@@ -804,7 +806,17 @@ uint32_t sssp_delta_for(const cgb_graph* g, double c)
     return (uint32_t)d;
 }
 
-uint32_t sssp_default_delta(const cgb_graph* g) { return sssp_delta_for(g, 128.0); }
+// Meshes (no list of kMeshDeg edges) of kMeshLarge vertices or more take c =
+// 64: their near sets grow with the bucket and the graph's width, and the
+// cluster loop's 16 SMs are full from a few thousand vertices on.  c = 128 /
+// 64: 500^2 grid 3.8 / 3.9 ms, 700 x 901 6.84 / 6.69, 1000^2 8.7 / 7.8, 2000^2
+// 29.9 / 26.2, 3000^2 73.9 / 44.3, 4800 x 5000 139.5 / 138.1.
+constexpr uint32_t kMeshDeg = 64, kMeshLarge = 1u << 19;
+
+uint32_t sssp_default_delta(const cgb_graph* g)
+{
+    return sssp_delta_for(g, g->max_degree < kMeshDeg && g->V >= kMeshLarge ? 64.0 : 128.0);
+}
 
 void run_sssp(cgb_graph* g, uint32_t root, const cgb_options& o)
 {

@@ -70,7 +70,8 @@ typedef struct cgb_options {
     uint32_t struct_size;   /* sizeof(cgb_options); 0 = all defaults */
     int32_t schedule;       /* cgb_schedule */
     int32_t variant;        /* cgb_variant, for CGB_SCHED_FIXED */
-    uint32_t sssp_delta;    /* 0 = heuristic: 128 * mean weight / mean degree (64 x for multi-root passes) */
+    uint32_t sssp_delta;    /* 0 = heuristic: 128 * mean weight / mean degree (64 x for multi-root passes and
+                               for meshes of 2^19 vertices or more) */
     double bfs_alpha;       /* Beamer alpha, 0 = 15 */
     double bfs_beta;        /* Beamer beta, 0 = 18 */
     uint64_t max_iterations;/* 0 = unlimited (V + 1 levels bound BFS anyway) */

@@ -42,6 +42,7 @@ def ladder(degrees):
 @pytest.mark.parametrize("graph", [
     lambda: star(100_000, 9),     # the queues spill
     lambda: star(65_000, 8),      # one piece a leaf, a queue nearly full
+    lambda: star(160_000, 2),     # more far vertices than the cluster splits
     lambda: star(3, 2),
     lambda: ladder([0, 1, 6, 7, 8, 9, 14, 15, 16, 17, 30, 31, 32, 33, 255, 256, 257, 5000] * 3),
 ])
