@@ -25,6 +25,7 @@ namespace cgb {
 // Per-CTA accumulators of the top-down op (flushed once per CTA).
 __shared__ unsigned long long s_td_medges;
 __shared__ uint32_t s_td_maxdeg;
+__shared__ uint32_t s_bu_found;  // bottom-up
 
 struct BfsTdOp {
     const uint32_t* __restrict__ off;
@@ -144,6 +145,11 @@ __global__ void __launch_bounds__(kBlock) k_bfs_bu(uint32_t V, const uint32_t* _
     const uint32_t warps = gridDim.x * (kBlock / 32);
     uint32_t medges = 0, found_cnt = 0, mx = 0;
     stage_begin();
+    if (threadIdx.x == 0) {
+        s_td_medges = 0;
+        s_td_maxdeg = 0;
+        s_bu_found = 0;
+    }
     __syncthreads();
     for (uint32_t wi = blockIdx.x * (kBlock / 32) + (threadIdx.x >> 5); wi < words; wi += warps) {
         const uint32_t v = wi * 32 + lane;
@@ -180,15 +186,21 @@ __global__ void __launch_bounds__(kBlock) k_bfs_bu(uint32_t V, const uint32_t* _
             if (fm) visited[wi] = vis | fm;
         }
     }
-    __syncthreads();
-    stage_end(qout, qlen, cap, &ctr->overflow);
+    // one set of counter atomics per CTA: per warp, they were 38 us of a level
     const uint32_t warp_edges = __reduce_add_sync(0xffffffffu, medges);  // at most E < 2^32
     found_cnt = __reduce_add_sync(0xffffffffu, found_cnt);
     mx = __reduce_max_sync(0xffffffffu, mx);
     if (lane == 0 && found_cnt) {
-        atomicAdd(&ctr->medges, (unsigned long long)warp_edges);
-        atomicAdd(&ctr->found, found_cnt);
-        atomicMax(&ctr->max_deg, mx);
+        atomicAdd(&s_td_medges, (unsigned long long)warp_edges);
+        atomicAdd(&s_bu_found, found_cnt);
+        atomicMax(&s_td_maxdeg, mx);
+    }
+    __syncthreads();
+    stage_end(qout, qlen, cap, &ctr->overflow);
+    if (threadIdx.x == 0 && s_bu_found) {
+        atomicAdd(&ctr->medges, s_td_medges);
+        atomicAdd(&ctr->found, s_bu_found);
+        atomicMax(&ctr->max_deg, s_td_maxdeg);
     }
 }
 

@@ -98,6 +98,20 @@ __device__ __forceinline__ unsigned long long warp_or(unsigned long long v)
     return v;
 }
 
+// Adds v of every thread of the CTA to *counter with one atomic (every
+// thread calls it; it synchronises the CTA).
+__device__ __forceinline__ void cta_add(unsigned long long v, unsigned long long* counter)
+{
+    __shared__ unsigned long long s_part[32];
+    v = warp_sum(v);
+    if (lane_id() == 0) s_part[threadIdx.x >> 5] = v;
+    __syncthreads();
+    if (threadIdx.x < 32) {
+        v = warp_sum(threadIdx.x < blockDim.x / 32 ? s_part[threadIdx.x] : 0ull);
+        if (threadIdx.x == 0 && v) atomicAdd(counter, v);
+    }
+}
+
 __device__ __forceinline__ uint32_t warp_max(uint32_t v)
 {
 #pragma unroll

@@ -88,13 +88,10 @@ __global__ void __launch_bounds__(kBlock) k_ms_finalize(const uint32_t* __restri
         }
         warp_append(act, u, qact, qact_len, cap, &ctr->overflow);
     }
-    if (off) {
-        edges = warp_sum(edges);
-        if (lane_id() == 0 && edges) atomicAdd(&ctr->medges, edges);
-    }
+    if (off) cta_add(edges, &ctr->medges);
     if (alive) {
         live = warp_or(live);
-        if (lane_id() == 0 && live) atomicOr(alive, live);
+        if (lane_id() == 0 && (live & ~*(volatile unsigned long long*)alive)) atomicOr(alive, live);
     }
 }
 
@@ -246,7 +243,7 @@ __global__ void __launch_bounds__(kBlock) k_ms_bu_light(MsBuArgs a)
     stage_end(a.qact, a.qact_len, a.cap, &a.ctr->overflow);
     if (a.alive) {
         live = warp_or(live);
-        if (lane_id() == 0 && live) atomicOr(a.alive, live);
+        if (lane_id() == 0 && (live & ~*(volatile unsigned long long*)a.alive)) atomicOr(a.alive, live);
     }
 }
 
@@ -293,7 +290,7 @@ __global__ void __launch_bounds__(kBlock) k_ms_bu_warp(MsBuArgs a)
     }
     if (a.alive) {
         live = warp_or(live);
-        if (lane == 0 && live) atomicOr(a.alive, live);
+        if (lane == 0 && (live & ~*(volatile unsigned long long*)a.alive)) atomicOr(a.alive, live);
     }
 }
 
@@ -365,7 +362,7 @@ __global__ void __launch_bounds__(kBlock) k_ms_bu_settle(MsBuArgs a)
     }
     if (a.alive) {
         live = warp_or(live);
-        if (lane_id() == 0 && live) atomicOr(a.alive, live);
+        if (lane_id() == 0 && (live & ~*(volatile unsigned long long*)a.alive)) atomicOr(a.alive, live);
     }
 }
 
@@ -388,8 +385,7 @@ __global__ void k_ms_degree_sum(const uint32_t* __restrict__ q, uint32_t n, cons
         const uint32_t v = q[i];
         s += off[v + 1] - off[v];
     }
-    s = warp_sum(s);
-    if (lane_id() == 0 && s) atomicAdd(&ctr->medges, s);
+    cta_add(s, &ctr->medges);
 }
 
 // Out-edges of the reached (root, vertex) pairs, from the seen masks.
@@ -399,8 +395,7 @@ __global__ void k_ms_reached(uint32_t V, const unsigned long long* __restrict__ 
     unsigned long long edges = 0;
     for (uint32_t v = blockIdx.x * blockDim.x + threadIdx.x; v < V; v += gridDim.x * blockDim.x)
         edges += (unsigned long long)__popcll(seen[v]) * (off[v + 1] - off[v]);
-    edges = warp_sum(edges);
-    if (lane_id() == 0 && edges) atomicAdd(&ctr->reached_edges, edges);
+    cta_add(edges, &ctr->reached_edges);
 }
 
 void count_reached_ms(cgb_graph* g)

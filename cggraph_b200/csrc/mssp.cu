@@ -109,7 +109,7 @@ __global__ void __launch_bounds__(kBlock) k_mssp_out(const uint32_t* __restrict_
         }
         __syncthreads();
     }
-    if (lane_id() == 0 && edges) atomicAdd(&ctr->reached_edges, edges);
+    cta_add(edges, &ctr->reached_edges);
 }
 
 void mssp_expand(bool weighted, uint32_t grid, cudaStream_t st, const uint4* desc, const MsspCounters* cc,

@@ -18,7 +18,6 @@ struct MsspCounters {
     uint32_t min_far;      // smallest far distance >= hi seen by a split
     uint32_t overflow;
     uint32_t rounds;       // near rounds that had work
-    unsigned long long relax;  // relaxations (root, edge) that lowered the distance read
 };
 
 struct MsspBuffers {
@@ -101,7 +100,7 @@ __device__ __forceinline__ void mssp_expand_body(const uint4* __restrict__ desc,
     const uint32_t lane = lane_id();
     const uint32_t warps = gridDim.x * (kBlock / 32);
     const uint32_t thr0 = thr_slot ? thr_slot[lane] : thr, thr1 = thr_slot ? thr_slot[lane + 32] : thr;
-    unsigned long long relax = 0, near_live = 0, far_live = 0;
+    unsigned long long near_live = 0, far_live = 0;
     for (uint32_t j = blockIdx.x * (kBlock / 32) + (threadIdx.x >> 5); j < ndesc; j += warps) {
         const uint4 d = desc[j];
         const unsigned long long m = maskq[d.w];
@@ -150,7 +149,6 @@ __device__ __forceinline__ void mssp_expand_body(const uint4* __restrict__ desc,
                     const unsigned long long nb =
                         (unsigned long long)__ballot_sync(0xffffffffu, m0 && c0 < thr0) |
                         ((unsigned long long)__ballot_sync(0xffffffffu, m1 && c1 < thr1) << 32);
-                    relax += __popcll(mb);
                     if (lane == t) {
                         my_nb = nb;
                         my_fb = mb & ~nb;
@@ -165,7 +163,6 @@ __device__ __forceinline__ void mssp_expand_body(const uint4* __restrict__ desc,
             warp_append(qf, my_u, far_out, far_len, cap, &c->overflow);
         }
     }
-    if (lane == 0 && relax) atomicAdd(&c->relax, relax);
     if (alive) {
         near_live = warp_or(near_live);
         far_live = warp_or(far_live);

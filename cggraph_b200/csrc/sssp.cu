@@ -218,6 +218,12 @@ __global__ void __launch_bounds__(kBlock) k_sssp_dense_scan(uint32_t V, const ui
     unsigned long long deg_sum = 0;
     uint32_t new_far = 0, touched = 0, max_deg = 0;
     stage_begin();
+    if (threadIdx.x == 0) {
+        s_sssp_newfar = 0;
+        s_sssp_medges = 0;
+        s_sssp_touched = 0;
+        s_sssp_maxdeg = 0;
+    }
     __syncthreads();
     for (uint64_t b0 = (uint64_t)blockIdx.x * kBlock * 4; b0 < V; b0 += (uint64_t)gridDim.x * kBlock * 4) {
         const uint32_t v0 = (uint32_t)b0 + 4 * threadIdx.x;
@@ -276,17 +282,24 @@ __global__ void __launch_bounds__(kBlock) k_sssp_dense_scan(uint32_t V, const ui
         }
         stage_append_n<4>(to_near, v, near_out, near_len, cap, &ctr->overflow);
     }
+    // one set of counter atomics per CTA
+    deg_sum = warp_sum(deg_sum);
+    touched = __reduce_add_sync(0xffffffffu, touched);
+    new_far = __reduce_add_sync(0xffffffffu, new_far);
+    max_deg = __reduce_max_sync(0xffffffffu, max_deg);
+    if (lane == 0) {
+        if (deg_sum) atomicAdd(&s_sssp_medges, deg_sum);
+        if (new_far) atomicAdd(&s_sssp_newfar, new_far);
+        if (touched) atomicAdd(&s_sssp_touched, touched);
+        if (max_deg) atomicMax(&s_sssp_maxdeg, max_deg);
+    }
     __syncthreads();
     stage_end(near_out, near_len, cap, &ctr->overflow);
-    deg_sum = warp_sum(deg_sum);
-    touched = warp_sum(touched);
-    new_far = warp_sum(new_far);
-    max_deg = warp_max(max_deg);
-    if (lane == 0) {
-        if (deg_sum) atomicAdd(&ctr->medges, deg_sum);
-        if (new_far) atomicAdd(&ctr->far_len[0], new_far);
-        if (touched) atomicAdd(&ctr->touched, touched);
-        if (max_deg) atomicMax(&ctr->max_deg, max_deg);
+    if (threadIdx.x == 0) {
+        if (s_sssp_medges) atomicAdd(&ctr->medges, s_sssp_medges);
+        if (s_sssp_newfar) atomicAdd(&ctr->far_len[0], s_sssp_newfar);
+        if (s_sssp_touched) atomicAdd(&ctr->touched, s_sssp_touched);
+        if (s_sssp_maxdeg) atomicMax(&ctr->max_deg, s_sssp_maxdeg);
     }
 }
 
