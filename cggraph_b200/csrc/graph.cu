@@ -820,7 +820,6 @@ static void stable_sort_u32(cgb_graph* g, const uint32_t* keys_in, uint32_t* key
     void* temp = dalloc<char>(tb, g->stream);
     cudaError_t err = cub::DeviceRadixSort::SortPairs(temp, tb, keys_in, keys_out, vals_in, vals_out, (uint64_t)n, 0,
                                                       bits, g->stream);
-    CGB_CUDA_TRY(cudaStreamSynchronize(g->stream));
     dfree(temp, g->stream);
     CGB_CUDA_TRY(err);
 }
@@ -1377,7 +1376,6 @@ void ensure_pr(cgb_graph* g)
         cudaError_t err = cub::DeviceRadixSort::SortPairs(temp, tb, kb, vb, (uint64_t)V, 0, 32, g->stream);
         k_pr_rank<<<grid_for(V, kBlock, num_sms() * 8), kBlock, 0, g->stream>>>(V, vb.Current(), g->off, g->pr_rank,
                                                                              g->pr_outdeg);
-        CGB_CUDA_TRY(cudaStreamSynchronize(g->stream));
         dfree(temp, g->stream);
         dfree(key, g->stream);
         dfree(key2, g->stream);
@@ -1399,7 +1397,6 @@ void ensure_pr(cgb_graph* g)
         CGB_CUDA_TRY(cub::DeviceScan::ExclusiveSum(nullptr, tb, od, src_off, (uint64_t)V + 1, g->stream));
         void* temp = dalloc<char>(tb, g->stream);
         cudaError_t err = cub::DeviceScan::ExclusiveSum(temp, tb, od, src_off, (uint64_t)V + 1, g->stream);
-        CGB_CUDA_TRY(cudaStreamSynchronize(g->stream));
         dfree(temp, g->stream);
         dfree(od, g->stream);
         CGB_CUDA_TRY(err);
@@ -1411,7 +1408,6 @@ void ensure_pr(cgb_graph* g)
             stable_sort_u32(g, key, kout, val, g->pr_src, E, (int)bits_for(V));
             k_offsets_from_u32<<<grid_for((uint64_t)V + 1, kBlock, num_sms() * 16), kBlock, 0, g->stream>>>(
                 V, E, kout, g->pr_off);
-            CGB_CUDA_TRY(cudaStreamSynchronize(g->stream));
             dfree(key, g->stream);
             dfree(val, g->stream);
             dfree(kout, g->stream);
@@ -1419,7 +1415,6 @@ void ensure_pr(cgb_graph* g)
             CGB_CUDA_TRY(cudaMemsetAsync(g->pr_off, 0, ((size_t)V + 1) * 4, g->stream));
         }
         dfree(src_off, g->stream);
-        CGB_CUDA_TRY(cudaStreamSynchronize(g->stream));
         dfree(order, g->stream);
     }
     // 3. the long rows' segments, and the sliced ELL
@@ -1471,8 +1466,7 @@ void ensure_pr(cgb_graph* g)
             dfree(key2, g->stream);
             dfree(id, g->stream);
         }
-        build_sell(g, seg);
-        CGB_CUDA_TRY(cudaStreamSynchronize(g->stream));
+        build_sell(g, seg);  // synchronises
         g->n_pr_hubs = h[3];
         // the columns hold every source: the relabelled CSC is not read again
         dfree(g->pr_src, g->stream);
