@@ -406,13 +406,6 @@ void count_reached_ms(cgb_graph* g)
     g->stats.traversed_edges = g->h_ctr->reached_edges;
 }
 
-unsigned long long* ms_alloc(size_t n)
-{
-    void* p = nullptr;
-    CGB_CUDA_TRY(cudaMalloc(&p, (n ? n : 1) * 8));
-    return (unsigned long long*)p;
-}
-
 // Runs one pass of up to 64 roots; level_out (device) receives n * V levels.
 void run_msbfs(cgb_graph* g, const uint32_t* d_roots, uint32_t n, uint32_t* level_out, double alpha)
 {
@@ -509,18 +502,25 @@ MsBuffers* ms_buffers_alloc(uint32_t V, uint64_t E)
 {
     auto* b = new MsBuffers();
     try {
-        b->seen = ms_alloc(V);
-        b->front[0] = ms_alloc(V);
-        b->front[1] = ms_alloc(V);
-        b->next = ms_alloc(V);
-        CGB_CUDA_TRY(cudaMemset(b->next, 0, (size_t)V * 8));  // zero between levels (bottom-up parks masks here)
-        CGB_CUDA_TRY(cudaMalloc((void**)&b->heavy_w, (size_t)V * 4));
         b->cap_b = (uint32_t)std::min<uint64_t>(E / kMsBlockDeg + 2, V);
-        CGB_CUDA_TRY(cudaMalloc((void**)&b->heavy_b, (size_t)b->cap_b * 4));
         // every hub's list past kMsLight in chunks: sum of ceil(deg / kMsHubChunk) <= E / kMsHubChunk + hubs
         b->cap_c = (uint32_t)(E / kMsHubChunk + b->cap_b + 1);
-        CGB_CUDA_TRY(cudaMalloc((void**)&b->hub_chunks, (size_t)b->cap_c * sizeof(uint2)));
-        CGB_CUDA_TRY(cudaMalloc((void**)&b->heavy_len, 12));
+        auto arrays = [&](Carve& c) {
+            c.take(b->seen, V);
+            c.take(b->front[0], V);
+            c.take(b->front[1], V);
+            c.take(b->next, V);
+            c.take(b->heavy_w, V);
+            c.take(b->heavy_b, b->cap_b);
+            c.take(b->hub_chunks, b->cap_c);
+            c.take(b->heavy_len, 3);
+        };
+        Carve size, place;
+        arrays(size);
+        CGB_CUDA_TRY(cudaMalloc(&b->block, size.bytes));
+        place.base = static_cast<char*>(b->block);
+        arrays(place);
+        CGB_CUDA_TRY(cudaMemset(b->next, 0, (size_t)V * 8));  // zero between levels (bottom-up parks masks here)
     } catch (...) {
         ms_buffers_free(b);
         throw;
@@ -531,14 +531,7 @@ MsBuffers* ms_buffers_alloc(uint32_t V, uint64_t E)
 void ms_buffers_free(MsBuffers* b)
 {
     if (!b) return;
-    cudaFree(b->seen);
-    cudaFree(b->front[0]);
-    cudaFree(b->front[1]);
-    cudaFree(b->next);
-    cudaFree(b->heavy_w);
-    cudaFree(b->heavy_b);
-    cudaFree(b->hub_chunks);
-    cudaFree(b->heavy_len);
+    cudaFree(b->block);
     delete b;
 }
 

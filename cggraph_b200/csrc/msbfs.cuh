@@ -7,7 +7,22 @@
 
 namespace cgb {
 
+// Several arrays in one device allocation (a cudaMalloc each cost more than
+// the first pass's kernels): sizes are added up by a first pass over the
+// arrays, pointers set by a second one.
+struct Carve {
+    char* base = nullptr;
+    size_t bytes = 0;
+    template <class T>
+    void take(T*& p, size_t n)
+    {
+        if (base) p = reinterpret_cast<T*>(base + bytes);
+        bytes += ((n ? n : 1) * sizeof(T) + 255) / 256 * 256;
+    }
+};
+
 struct MsBuffers {
+    void* block = nullptr;                  // the allocation that holds the arrays
     unsigned long long* seen = nullptr;
     unsigned long long* front[2] = {nullptr, nullptr};
     unsigned long long* next = nullptr;     // top-down scratch; bottom-up partial masks; zero between levels
@@ -107,6 +122,5 @@ __global__ void k_ms_clear(const uint32_t* __restrict__ q, uint32_t n, unsigned 
 __global__ void k_ms_fill(uint64_t n, uint32_t* a, uint32_t value);
 __global__ void k_ms_degree_sum(const uint32_t* __restrict__ q, uint32_t n, const uint32_t* n_ptr,
                                 const uint32_t* __restrict__ off, DevCounters* ctr);
-unsigned long long* ms_alloc(size_t n);
 
 }  // namespace cgb

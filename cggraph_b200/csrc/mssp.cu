@@ -132,15 +132,22 @@ MsspBuffers* mssp_buffers_alloc(uint32_t V, uint64_t E)
 {
     auto* b = new MsspBuffers();
     try {
-        CGB_CUDA_TRY(cudaMalloc((void**)&b->dist, (size_t)V * kMsRoots * 4));
-        CGB_CUDA_TRY(cudaMalloc((void**)&b->pend, (size_t)V * 8));
-        CGB_CUDA_TRY(cudaMalloc((void**)&b->farm, (size_t)V * 8));
-        CGB_CUDA_TRY(cudaMalloc((void**)&b->maskq, (size_t)V * 8));
-        CGB_CUDA_TRY(cudaMalloc((void**)&b->far_list[0], (size_t)V * 4));
-        CGB_CUDA_TRY(cudaMalloc((void**)&b->far_list[1], (size_t)V * 4));
         b->desc_cap = (uint64_t)V + E / kMinMsEdges + 1;  // any descriptor size cgb_tuning_set allows
-        CGB_CUDA_TRY(cudaMalloc((void**)&b->desc, b->desc_cap * sizeof(uint4)));
-        CGB_CUDA_TRY(cudaMalloc((void**)&b->c, sizeof(MsspCounters)));
+        auto arrays = [&](Carve& c) {
+            c.take(b->dist, (size_t)V * kMsRoots);
+            c.take(b->pend, V);
+            c.take(b->farm, V);
+            c.take(b->maskq, V);
+            c.take(b->far_list[0], V);
+            c.take(b->far_list[1], V);
+            c.take(b->desc, b->desc_cap);
+            c.take(b->c, 1);
+        };
+        Carve size, place;
+        arrays(size);
+        CGB_CUDA_TRY(cudaMalloc(&b->block, size.bytes));
+        place.base = static_cast<char*>(b->block);
+        arrays(place);
         CGB_CUDA_TRY(cudaMallocHost((void**)&b->h, sizeof(MsspCounters)));
     } catch (...) {
         mssp_buffers_free(b);
@@ -152,14 +159,7 @@ MsspBuffers* mssp_buffers_alloc(uint32_t V, uint64_t E)
 void mssp_buffers_free(MsspBuffers* b)
 {
     if (!b) return;
-    cudaFree(b->dist);
-    cudaFree(b->pend);
-    cudaFree(b->farm);
-    cudaFree(b->maskq);
-    cudaFree(b->far_list[0]);
-    cudaFree(b->far_list[1]);
-    cudaFree(b->desc);
-    cudaFree(b->c);
+    cudaFree(b->block);
     if (b->h) cudaFreeHost(b->h);
     delete b;
 }

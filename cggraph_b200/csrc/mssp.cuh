@@ -3,6 +3,7 @@
 #pragma once
 
 #include "engine.cuh"
+#include "msbfs.cuh"
 
 namespace cgb {
 
@@ -21,6 +22,7 @@ struct MsspCounters {
 };
 
 struct MsspBuffers {
+    void* block = nullptr;                  // the allocation that holds the arrays
     uint32_t* dist = nullptr;               // V * 64
     unsigned long long* pend = nullptr;     // V
     unsigned long long* farm = nullptr;     // V
