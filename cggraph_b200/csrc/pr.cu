@@ -103,8 +103,11 @@ __device__ __forceinline__ void pr_row_out(const PrIter& a, uint32_t r, double s
 // (cgb_tuning.pr_unroll) are issued before they are summed, in j order, so
 // each lane keeps kU gathers in flight.  Padding slots and the masked steps
 // of the last batch name vertex V, whose contribution is 0.
+// (The plain kernel is held to 32 registers, 8 CTAs an SM: at 34 registers, 6
+// CTAs, the 4800 x 5000 grid took 6.77 instead of 6.34 ms.  The hinted one
+// spills there: it has 6.)
 template <int kU, bool kHint>
-__global__ void __launch_bounds__(kBlock) k_pr_pull(PrIter a)
+__global__ void __launch_bounds__(kBlock, kHint ? 6 : 8) k_pr_pull(PrIter a)
 {
     const uint32_t lane = lane_id();
     const uint32_t nslices = a.n_seg_slices + (a.n_rows + 31) / 32;
