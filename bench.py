@@ -145,7 +145,7 @@ def pick_roots(offsets: np.ndarray, seed: int, n: int) -> list:
 # DRAM bytes (dram__bytes_read.sum + dram__bytes_write.sum) of one k_pr_pull
 # launch, from a one-pass ncu capture of this bench with --algorithms pr on the
 # same graph, keyed by (scale, edge factor, seed).
-PR_PULL_DRAM_BYTES = {(24, 16, 1): 1166656256 + 225822208, (22, 16, 1): 250001920 + 20899072}
+PR_PULL_DRAM_BYTES = {(24, 16, 1): 1230000000 + 73610000, (22, 16, 1): 287270000 + 5160000}
 
 
 def load_peaks() -> dict:
@@ -323,12 +323,12 @@ def bench_cgb200(args, d: Dist):
         bytes_per_launch = 12 * Ed + 20 * V + 4
         avg_s = pr_launch_ms / pr_launches / 1e3
         achieved = bytes_per_launch / avg_s / 1e9
-        roof.update({"kernel": "k_pr_pull (+ hub-row chunk kernels), one PageRank iteration",
+        roof.update({"kernel": "k_pr_pull + k_pr_combine, one PageRank iteration",
                      "alg_bytes_per_launch": bytes_per_launch, "avg_launch_ms": pr_launch_ms / pr_launches,
                      "achieved": achieved, "frac": achieved / peaks["hbm_gbs"],
                      "traffic": PR_PULL_DRAM_BYTES.get((args.scale, args.edge_factor, args.seed)),
                      "traffic_source": "dram__bytes_read.sum + dram__bytes_write.sum of one k_pr_pull launch, "
-                                       "ncu capture of this workload (hub-row chunk kernels not included)",
+                                       "ncu capture of this workload (k_pr_combine not included)",
                      "dominant_class": L.KERNEL_CLASS_NAMES[dom],
                      "class_share": {L.KERNEL_CLASS_NAMES[c]: round(kclass_ms[c] / max(1e-9, sum(kclass_ms)), 4)
                                      for c in range(8) if kclass_ms[c] > 0}})

@@ -334,8 +334,8 @@ typedef struct {
     uint32_t sssp_pull_alpha;  /* SSSP rounds pull (scan in-edges of unsettled vertices) when the near
                                   set's out-edges times this exceed E; 0 = always push (default; on
                                   RMAT-24 the pull kernels lose to the push, the autotuner may pick it) */
-    uint32_t cluster_enter;    /* BFS frontiers up to this size run their levels in one thread-block
-                                  cluster with a hardware barrier (0 = never, default 8192) */
+    uint32_t cluster_enter;    /* BFS and SSSP frontiers up to this size (and 2^15 out-edges) run their
+                                  levels in one thread-block cluster (0 = never, default 8192) */
     uint32_t sssp_dense_alpha; /* SSSP rounds use a dense frontier when the near set's out-edges times
                                   this times max(first touches per edge in the previous round, 1/8)
                                   exceed V (0 = never, default 4) */
