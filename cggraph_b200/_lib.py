@@ -35,7 +35,7 @@ EXPORTS = [
     "cgb_batch_info", "cgb_batch_stats", "cgb_server_create", "cgb_server_submit", "cgb_server_start",
     "cgb_server_wait", "cgb_server_poll", "cgb_server_stats", "cgb_server_destroy", "cgb_tuning_get",
     "cgb_tuning_set", "cgb_autotune", "cgb_memory_trim", "cgb_memory_info", "cgb_memory_reserve",
-    "cgb_check_barrier_timeout",
+    "cgb_check_barrier_timeout", "cgb_check_cluster_timeout",
 ]
 POLICY_FEATURES, POLICY_OUTPUTS, POLICY_PARAMS = 24, 14, 6670
 

@@ -72,6 +72,16 @@ cgb_status cgb_check_barrier_timeout(int device, uint32_t spin_limit)
     });
 }
 
+cgb_status cgb_check_cluster_timeout(int device, uint32_t limit_us)
+{
+    return guarded([&] {
+        CGB_REQUIRE(limit_us >= 1 && limit_us <= 1000000, CGB_EINVAL, "limit_us must be in [1, 1000000]");
+        CGB_CUDA_TRY(cudaSetDevice(device));
+        const cgb_status st = cluster_timeout_check(limit_us);
+        if (st != CGB_OK) throw Error{st, "cluster wait gave up after its time limit (the expected outcome)"};
+    });
+}
+
 const char* cgb_last_error_string(void) { return last_error().c_str(); }
 
 const char* cgb_status_string(cgb_status s)

@@ -13,10 +13,15 @@
 //   - the edges of a piece are visited kClBatch at a time, one atomicMin each
 //     that both tests and claims (no read before it);
 //   - the counts of a level go to every CTA as asynchronous stores that
-//     complete an mbarrier there, the only synchronisation between levels
-//     (its wait is bounded: status, CGB_ETIMEOUT).
+//     complete an mbarrier there, the only synchronisation between levels.
 // All exit decisions are taken by every thread from the same counts, so the
 // cluster leaves together.
+//
+// The wait for a level's counts ends after a time limit (cl_wait): the CTA
+// then drops what it has queued and leaves, and the run returns CGB_ETIMEOUT.
+// That covers counts which come late or not at all.  The cluster's hardware
+// barrier at either end of a loop has no limit of its own: it is reached by
+// every CTA, because nothing between the two waits for longer than that.
 //
 // Vertices without out-edges are claimed but not queued.  Vertices beyond a
 // CTA's queue spill to the global queue; the loop then returns
@@ -32,7 +37,9 @@ namespace {
 
 constexpr int kClThreads = 512;
 constexpr int kClWarps = kClThreads / 32;
-constexpr uint32_t kClSpins = 1u << 22;  // polls of a level's barrier before the loop gives up
+constexpr unsigned long long kClWaitNs = 1000000000ull;  // a level's counts take longer: the loop gives up
+constexpr uint32_t kClSpins = 1u << 28;  // and after so many polls, whatever the clock says
+constexpr uint32_t kClPollNs = 10000, kClEarly = 1u << 16;
 constexpr uint32_t kClMaxCtas = 16;
 constexpr uint32_t kClQueue = 8192;  // entries per CTA and buffer
 constexpr uint32_t kClPiece = 8;     // edges per entry
@@ -161,6 +168,47 @@ __device__ __forceinline__ void stage(uint32_t (&x)[N])
     for (int i = 0; i < N; i++) asm volatile("" : "+r"(x[i])::"memory");
 }
 
+// One poll of phase `parity` of an mbarrier of this CTA.  It may suspend the
+// thread until the phase completes, kClPollNs at most.
+__device__ __forceinline__ bool cl_poll(uint32_t mbar, uint32_t parity)
+{
+    uint32_t done;
+    asm volatile(
+        "{\n\t.reg .pred p;\n\t"
+        "mbarrier.try_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], %2, %3;\n\t"
+        "selp.u32 %0, 1, 0, p;\n\t}"
+        : "=r"(done)
+        : "r"(mbar), "r"(parity), "r"(kClPollNs)
+        : "memory");
+    return done != 0;
+}
+
+// The rest of a wait that has polled a while: at most wait_ns by the clock
+// and kClSpins polls.
+__device__ __forceinline__ bool cl_wait_late(uint32_t mbar, uint32_t parity, unsigned long long wait_ns)
+{
+    unsigned long long t0, t;
+    asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t0));
+    for (uint32_t spin = 0; spin < kClSpins; spin++) {
+        if (cl_poll(mbar, parity)) return true;
+        asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t));
+        if (t - t0 > wait_ns) return false;
+    }
+    return false;
+}
+
+// Waits for phase `parity` of an mbarrier of this CTA; false after kClEarly
+// polls (0.7 s if each is suspended) and wait_ns.  The clock is not looked at
+// while the early polls run: where it was, a level took 2 to 3 % longer (1200
+// x 1250 grid BFS 6.91 ms without a limit by the clock, 7.01 as it is, 7.13
+// with a look every 64 polls).
+__device__ __forceinline__ bool cl_wait(uint32_t mbar, uint32_t parity, unsigned long long wait_ns)
+{
+    bool done = false;
+    for (uint32_t spin = 0; !done && spin < kClEarly; spin++) done = cl_poll(mbar, parity);
+    return done || cl_wait_late(mbar, parity, wait_ns);
+}
+
 // Ends level `level`: sends this CTA's counts to every CTA (buffer level &
 // 1) and waits for theirs.  The counts travel as asynchronous stores that
 // complete the receiver's mbarrier, so a level costs one trip over the
@@ -168,9 +216,12 @@ __device__ __forceinline__ void stage(uint32_t (&x)[N])
 // The fence orders the queue entries before the counts.  Buffers alternate,
 // and a CTA sends the counts of a level only after it has received all of
 // the level before, so no slot, queue or mbarrier phase is overtaken.
-// Returns false when the wait gave up (the same CTA-wide).
+// Returns false when the wait gave up (the same CTA-wide): the counts in
+// from[] are then not this level's.  send = false (the self-check) keeps this
+// CTA's counts back.
 __device__ __forceinline__ bool cl_next_level(cooperative_groups::cluster_group& cluster, ClShared& s, uint32_t level,
-                                              uint32_t edges, ClusterState* st)
+                                              uint32_t edges, ClusterState* st, unsigned long long wait_ns,
+                                              bool send = true)
 {
     const uint32_t buf = level & 1, ctas = cluster.num_blocks();
     if (__any_sync(0xffffffffu, edges != 0)) {
@@ -189,7 +240,7 @@ __device__ __forceinline__ bool cl_next_level(cooperative_groups::cluster_group&
                          "r"(ctas * (uint32_t)sizeof(ClCounts))
                          : "memory");
         }
-        if (threadIdx.x < ctas) {
+        if (threadIdx.x < ctas && send) {
             asm volatile("fence.acq_rel.cluster;" ::: "memory");
             uint32_t to, to_bar;
             asm("mapa.shared::cluster.u32 %0, %1, %2;"
@@ -202,21 +253,25 @@ __device__ __forceinline__ bool cl_next_level(cooperative_groups::cluster_group&
                 : "memory");
         }
     }
-    uint32_t done = 0;
-    for (uint32_t spin = 0; !done && spin < kClSpins; spin++)
-        asm volatile(
-            "{\n\t.reg .pred p;\n\t"
-            "mbarrier.try_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], %2;\n\t"
-            "selp.u32 %0, 1, 0, p;\n\t}"
-            : "=r"(done)
-            : "r"(mbar), "r"((level >> 1) & 1)
-            : "memory");
-    if (!done) {
+    if (!cl_wait(mbar, (level >> 1) & 1, wait_ns)) {
         s.gave_up = 1;
         atomicOr(&st->status, 2u);
     }
     __syncthreads();  // the counts were reset, and all threads agree on gave_up
     return !s.gave_up;
+}
+
+// Ends the loop at level `level`: every CTA passes the cluster's barrier, so
+// none leaves while another may read its queue.  One that gave up may still
+// have that level's counts on their way to it: all CTAs have sent what they
+// send, and it waits for them once more before its shared memory goes.
+__device__ __forceinline__ void cl_leave(cooperative_groups::cluster_group& cluster, ClShared& s, uint32_t level,
+                                         unsigned long long wait_ns)
+{
+    __threadfence();
+    cluster.sync();
+    if (s.gave_up)
+        cl_wait((uint32_t)__cvta_generic_to_shared(&s.arrived[level & 1]), (level >> 1) & 1, wait_ns);
 }
 
 __device__ __forceinline__ void cl_setup(cooperative_groups::cluster_group& cluster, ClShared& s, ClusterState* st)
@@ -304,7 +359,7 @@ __global__ void __launch_bounds__(kClThreads, 1)
     k_bfs_cluster(const uint32_t* __restrict__ off, const uint32_t* __restrict__ dst, uint32_t* level,
                   uint32_t* visited, const uint32_t* q_in, uint32_t* q_out, uint32_t cap, uint32_t nz,
                   uint32_t start_level, uint32_t nf, uint32_t nf_exit, uint32_t scout_exit, uint32_t max_levels,
-                  ClusterState* st, ClusterState* host)
+                  unsigned long long wait_ns, ClusterState* st, ClusterState* host)
 {
     extern __shared__ __align__(16) unsigned char smem[];
     ClShared& s = *reinterpret_cast<ClShared*>(smem);
@@ -312,7 +367,7 @@ __global__ void __launch_bounds__(kClThreads, 1)
     const uint32_t ctas = cluster.num_blocks(), rank = cluster.block_rank();
     const bool leader = rank == 0 && threadIdx.x == 0;
     cl_setup(cluster, s, st);
-    bool ok = cl_next_level(cluster, s, 0, cl_load(cluster, s, off, q_in, nf, q_out, cap, st), st);
+    bool ok = cl_next_level(cluster, s, 0, cl_load(cluster, s, off, q_in, nf, q_out, cap, st), st, wait_ns);
     uint32_t it = 0, found = 0, word, scout;
     // a vertex that leaves for the global queue gets its visited bit now
     auto mark = [&](uint32_t v) {
@@ -366,13 +421,12 @@ __global__ void __launch_bounds__(kClThreads, 1)
                 cl_push<kClBatch>(s, buf ^ 1, enq, d, lo, dg, q_out, cap, st, edges, mark);
             }
         });
-        ok = cl_next_level(cluster, s, it + 1, edges, st);
+        ok = cl_next_level(cluster, s, it + 1, edges, st, wait_ns);
     }
     found = __reduce_add_sync(0xffffffffu, found);
     if (lane_id() == 0 && found) atomicAdd(&st->found, found);
-    if (it > 0) cl_flush(s, it & 1, rank, off, q_out, cap, st, mark);
-    __threadfence();
-    cluster.sync();  // also: no CTA leaves while another may read its queue
+    if (ok && it > 0) cl_flush(s, it & 1, rank, off, q_out, cap, st, mark);
+    cl_leave(cluster, s, it, wait_ns);
     if (leader) {
         ClusterState h{};
         h.qlen = __ldcg(&st->qlen);
@@ -398,7 +452,8 @@ __global__ void __launch_bounds__(kClThreads, 1)
                    uint32_t* dist, uint32_t* stamp, uint32_t* far_bm, uint32_t words, const uint32_t* q_in,
                    uint32_t* q_out, uint32_t cap, uint32_t nz, uint32_t nf, unsigned long long thr, uint32_t nfar,
                    unsigned long long bucket_lo, uint32_t delta, uint32_t nf_exit, uint32_t scout_exit,
-                   uint32_t far_exit, uint32_t max_rounds, uint32_t* far_len_out, ClusterState* st, ClusterState* host)
+                   uint32_t far_exit, uint32_t max_rounds, uint32_t* far_len_out, unsigned long long wait_ns,
+                   ClusterState* st, ClusterState* host)
 {
     extern __shared__ __align__(16) unsigned char smem[];
     ClShared& s = *reinterpret_cast<ClShared*>(smem);
@@ -406,7 +461,7 @@ __global__ void __launch_bounds__(kClThreads, 1)
     const uint32_t ctas = cluster.num_blocks(), rank = cluster.block_rank(), lane = lane_id();
     const bool leader = rank == 0 && threadIdx.x == 0;
     cl_setup(cluster, s, st);
-    bool ok = cl_next_level(cluster, s, 0, cl_load(cluster, s, off, q_in, nf, q_out, cap, st), st);
+    bool ok = cl_next_level(cluster, s, 0, cl_load(cluster, s, off, q_in, nf, q_out, cap, st), st, wait_ns);
     uint32_t it = 0, word, scout, added = 0;
     // a vertex goes to the global queue once (its short list may be queued twice)
     const uint32_t kLeft = 0xFFFFFFFFu;
@@ -540,20 +595,19 @@ __global__ void __launch_bounds__(kClThreads, 1)
             }
             after_split = true;
         }
-        ok = cl_next_level(cluster, s, it + 1, edges, st);
+        ok = cl_next_level(cluster, s, it + 1, edges, st, wait_ns);
     }
-    if (it > 0) cl_flush(s, it & 1, rank, off, q_out, cap, st, take);
+    if (ok && it > 0) cl_flush(s, it & 1, rank, off, q_out, cap, st, take);
     added = __reduce_add_sync(0xffffffffu, added);
     if (lane == 0 && added) atomicAdd(&st->found, added);
-    if (far) {
+    if (ok && far) {
         uint32_t pop = 0;
         for (uint32_t i = rank * kClThreads + threadIdx.x; i < words; i += ctas * kClThreads)
             pop += __popc(__ldcg(far_bm + i));
         pop = __reduce_add_sync(0xffffffffu, pop);
         if (lane == 0 && pop) atomicAdd(&st->far_left, pop);
     }
-    __threadfence();
-    cluster.sync();
+    cl_leave(cluster, s, it, wait_ns);
     if (leader) {
         ClusterState h{};
         h.qlen = __ldcg(&st->qlen);
@@ -566,6 +620,27 @@ __global__ void __launch_bounds__(kClThreads, 1)
         h.thr = thr;
         h.bucket_lo = bucket_lo;
         *far_len_out = h.far_left;
+        *host = h;
+    }
+}
+
+// Self-check of the time limit: level 0 completes; at level 1 CTA 0 sends
+// nothing, so every CTA's wait runs out, and all meet at the last barrier.
+__global__ void __launch_bounds__(kClThreads, 1)
+    k_cluster_timeout(unsigned long long wait_ns, ClusterState* st, ClusterState* host)
+{
+    extern __shared__ __align__(16) unsigned char smem[];
+    ClShared& s = *reinterpret_cast<ClShared*>(smem);
+    cooperative_groups::cluster_group cluster = cooperative_groups::this_cluster();
+    cl_setup(cluster, s, st);
+    uint32_t it = 0;
+    bool ok = cl_next_level(cluster, s, 0, 0, st, wait_ns);
+    if (ok) ok = cl_next_level(cluster, s, ++it, 0, st, wait_ns, cluster.block_rank() != 0);
+    cl_leave(cluster, s, it, wait_ns);
+    if (cluster.block_rank() == 0 && threadIdx.x == 0) {
+        ClusterState h{};
+        h.status = __ldcg(&st->status);
+        h.levels = it;
         *host = h;
     }
 }
@@ -609,18 +684,17 @@ uint32_t cluster_loop_ctas()
     int c = cache[dev].load(std::memory_order_acquire);
     if (!c) {
         c = 1 + (int)std::min({cluster_ctas(k_bfs_cluster), cluster_ctas(k_sssp_cluster<true>),
-                               cluster_ctas(k_sssp_cluster<false>)});
+                               cluster_ctas(k_sssp_cluster<false>), cluster_ctas(k_cluster_timeout)});
         cache[dev].store(c, std::memory_order_release);
     }
     return (uint32_t)(c - 1);
 }
 
-// Launches a cluster loop on the graph's stream and returns what it reports
-// (through pinned host memory; synchronises the stream).
+// Launches a cluster loop on stream st and returns what it reports (through
+// pinned host memory; synchronises the stream).
 template <class... P, class... A>
-static ClusterState run_cluster(cgb_graph* g, void (*kern)(P...), A... args)
+static ClusterState launch_cluster(cudaStream_t st, void (*kern)(P...), A... args)
 {
-    if (!g->cluster) g->cluster = pool_alloc(sizeof(ClusterState), g->stream);
     PinnedArray<ClusterState> h(1);
     cudaLaunchAttribute attr[1];
     attr[0].id = cudaLaunchAttributeClusterDimension;
@@ -629,15 +703,45 @@ static ClusterState run_cluster(cgb_graph* g, void (*kern)(P...), A... args)
     cfg.gridDim = dim3(attr[0].val.clusterDim.x);
     cfg.blockDim = dim3(kClThreads);
     cfg.dynamicSmemBytes = sizeof(ClShared);
-    cfg.stream = g->stream;
+    cfg.stream = st;
     cfg.attrs = attr;
     cfg.numAttrs = 1;
-    ++g->stats.launches;
-    CGB_CUDA_TRY(cudaLaunchKernelEx(&cfg, kern, args..., (ClusterState*)g->cluster, h.data()));
-    CGB_CUDA_TRY(cudaStreamSynchronize(g->stream));
-    CGB_REQUIRE(!(h[0].status & 2u), CGB_ETIMEOUT, "cluster loop: a level's barrier gave up");
-    CGB_REQUIRE(!h[0].status, CGB_EOVERFLOW, "cluster loop: queue overflow");
+    CGB_CUDA_TRY(cudaLaunchKernelEx(&cfg, kern, args..., h.data()));
+    CGB_CUDA_TRY(cudaStreamSynchronize(st));
     return h[0];
+}
+
+// The same for a graph's run.
+template <class... P, class... A>
+static ClusterState run_cluster(cgb_graph* g, void (*kern)(P...), A... args)
+{
+    if (!g->cluster) g->cluster = pool_alloc(sizeof(ClusterState), g->stream);
+    ++g->stats.launches;
+    const ClusterState h = launch_cluster(g->stream, kern, args..., kClWaitNs, (ClusterState*)g->cluster);
+    CGB_REQUIRE(!(h.status & 2u), CGB_ETIMEOUT, "cluster loop: a level's counts did not come in time");
+    CGB_REQUIRE(!h.status, CGB_EOVERFLOW, "cluster loop: queue overflow");
+    return h;
+}
+
+cgb_status cluster_timeout_check(uint32_t limit_us)
+{
+    CGB_REQUIRE(cluster_loop_ctas() > 0, CGB_EUNSUPPORTED, "the device schedules no cluster of 8 CTAs");
+    ClusterState* st = nullptr;
+    CGB_CUDA_TRY(cudaMalloc((void**)&st, sizeof(ClusterState)));
+    cudaStream_t stream = nullptr;
+    ClusterState h{};
+    try {
+        CGB_CUDA_TRY(cudaStreamCreateWithFlags(&stream, cudaStreamNonBlocking));
+        h = launch_cluster(stream, k_cluster_timeout, limit_us * 1000ull, st);
+    } catch (...) {
+        if (stream) cudaStreamDestroy(stream);
+        cudaFree(st);
+        throw;
+    }
+    cudaStreamDestroy(stream);
+    cudaFree(st);
+    CGB_REQUIRE(h.levels == 1, CGB_ECUDA, "cluster self-check: the first level did not complete");
+    return (h.status & 2u) ? CGB_ETIMEOUT : CGB_OK;
 }
 
 PersistResult bfs_cluster(cgb_graph* g, uint32_t cur, uint32_t nf, uint32_t level, uint32_t nf_exit,

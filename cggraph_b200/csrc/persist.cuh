@@ -76,7 +76,7 @@ struct PersistBlock {
 // What a cluster loop reports on exit.
 struct ClusterState {
     uint32_t qlen;      // frontier vertices left in the global queue
-    uint32_t status;    // 1 = queue overflow, 2 = a barrier gave up
+    uint32_t status;    // 1 = queue overflow, 2 = a wait gave up
     uint32_t levels;    // levels (rounds) run
     uint32_t max_deg;   // longest list of the frontier
     uint32_t found;     // BFS: vertices reached; SSSP: list pieces expanded
@@ -112,6 +112,9 @@ PersistResult bfs_persistent(cgb_graph* g, uint32_t cur, uint32_t nf, unsigned l
 // The cluster loops.  CTAs of a cluster on the current device (0: the device
 // schedules none, and the loops must not be called).
 uint32_t cluster_loop_ctas();
+// Launches a cluster in which one CTA keeps a level's counts back;
+// CGB_ETIMEOUT when the wait for them ended after limit_us (a self-check).
+cgb_status cluster_timeout_check(uint32_t limit_us);
 // BFS levels from q[cur][0, nf) (level `level`): bounds as bfs_persistent.
 // Vertices without out-edges are reached but not part of a frontier.
 PersistResult bfs_cluster(cgb_graph* g, uint32_t cur, uint32_t nf, uint32_t level, uint32_t nf_exit,

@@ -541,6 +541,12 @@ cgb_status cgb_policy_loss_grad(const float* params, const float* features, cons
  * when the others gave up as they should (the context stays usable). */
 cgb_status cgb_check_barrier_timeout(int device, uint32_t spin_limit);
 
+/* The same for the loops that run in one thread-block cluster, whose CTAs
+ * wait for one another's counts after each level for at most a time limit:
+ * one CTA keeps its counts back, with a limit of 1 .. 1000000 microseconds.
+ * CGB_ETIMEOUT when every wait ended and the kernel returned. */
+cgb_status cgb_check_cluster_timeout(int device, uint32_t limit_us);
+
 const char* cgb_last_error_string(void);
 const char* cgb_status_string(cgb_status s);
 int cgb_abi_version(void);

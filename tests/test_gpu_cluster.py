@@ -62,3 +62,25 @@ def test_cluster_loops(graph, wmax, delta):
         np.testing.assert_array_equal(g.run(SSSP, 1, opts)[0], O.sssp(off, dst, w, 1))
     with cg.Graph.from_csr(off, dst) as g:  # unit weights
         np.testing.assert_array_equal(g.run(SSSP, 0)[0], O.bfs(off, dst, 0))
+
+
+@pytest.mark.gpu
+def test_wait_for_counts_ends():
+    """A CTA that keeps its counts back ends the others' waits after their time limit, and the context stays usable."""
+    import ctypes
+    import time
+    from cggraph_b200 import _lib as L
+    f = L.lib().cgb_check_cluster_timeout
+    f.argtypes = [ctypes.c_int, ctypes.c_uint32]
+    f.restype = ctypes.c_int
+    assert f(0, 0) == L.EINVAL and f(0, 1_000_001) == L.EINVAL
+    assert f(0, 100) == L.ETIMEOUT
+    t0 = time.monotonic()
+    assert f(0, 200_000) == L.ETIMEOUT
+    # the wait and, before the cluster leaves, once more as long
+    assert 0.2 <= time.monotonic() - t0 < 5
+    V, src, dst = ladder([3] * 40)
+    off, dst, w = csr(V, src, dst, 5, 9)
+    with cg.Graph.from_csr(off, dst, w) as g:
+        np.testing.assert_array_equal(g.run(BFS, 0)[0], O.bfs(off, dst, 0))
+        np.testing.assert_array_equal(g.run(SSSP, 0)[0], O.sssp(off, dst, w, 0))
