@@ -445,6 +445,9 @@ __global__ void __launch_bounds__(kClThreads, 1)
 // last expanded a vertex: one that several edges improve in a round is queued
 // as often, and its later entries are skipped (checking when it is queued
 // would lengthen the round's chain; only lists of several pieces pay that).
+// Rounds only grow and kLeft is above them all, so marks are set by
+// atomicMax: an entry expanded later in the round leaves the mark of a vertex
+// that has gone to the global queue.
 // far_len_out receives the far bitmap's population on exit.
 template <bool kHasW>
 __global__ void __launch_bounds__(kClThreads, 1)
@@ -488,7 +491,7 @@ __global__ void __launch_bounds__(kClThreads, 1)
                 const uint32_t v = len ? *entry : 0u;
                 const uint32_t du = len ? __ldcg(dist + v) : 0u;
                 // a vertex queued twice: the second entry is skipped
-                const bool again = len && single && atomicExch(stamp + v, it + 1) == it + 1;
+                const bool again = len && single && atomicMax(stamp + v, it + 1) == it + 1;
                 added += len && !again ? 1u : 0u;
                 for (uint32_t b = 0; __any_sync(0xffffffffu, b < len); b += kClBatch) {
                     uint32_t d[kClBatch], nd[kClBatch], old[kClBatch], lo[kClBatch], dg[kClBatch];
@@ -521,7 +524,7 @@ __global__ void __launch_bounds__(kClThreads, 1)
                         dg[i] -= lo[i];
                         // the entries of a longer list do not know of one another: it is queued once
                         if (near[i] && dg[i] > kClPiece) {
-                            const uint32_t was = atomicExch(stamp + d[i], it + 2);
+                            const uint32_t was = atomicMax(stamp + d[i], it + 2);
                             near[i] = was != it + 2 && was != kLeft;
                         }
                     }

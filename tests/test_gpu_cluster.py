@@ -84,3 +84,33 @@ def test_wait_for_counts_ends():
     with cg.Graph.from_csr(off, dst, w) as g:
         np.testing.assert_array_equal(g.run(BFS, 0)[0], O.bfs(off, dst, 0))
         np.testing.assert_array_equal(g.run(SSSP, 0)[0], O.sssp(off, dst, w, 0))
+
+
+def spill_twice(members, longs, long_deg):
+    """A round that queues nearly every vertex again, more than the cluster's queues hold.  The root reaches `members`
+    vertices with short lists at random distances and a hub at distance 1; a member's list names one vertex with a long
+    list first (these fill the queues), then three members; the hub's list, expanded last, improves every member."""
+    rng = np.random.default_rng(7)
+    V = 1 + longs + members + 1
+    first, hub = 1 + longs, V - 1
+    m = np.arange(first, hub)
+    a, b = np.repeat(m, 3), first + rng.integers(0, members, 3 * members)
+    ls = np.repeat(np.arange(1, first), long_deg)
+    ld = first + (np.arange(longs * long_deg) * 13) % members
+    src = np.concatenate([np.zeros(members + 1, np.int64), m, a, ls, np.full(members, hub)])
+    dst = np.concatenate([np.arange(first, V), 1 + np.arange(members) % longs, b, ld, m])
+    return V, src[src != dst], dst[src != dst]
+
+
+@pytest.mark.gpu
+def test_spilled_vertex_leaves_once():
+    """All vertices but two are in one round's next frontier, so a queue of V entries has no room for one of them twice."""
+    V, src, dst = spill_twice(12_000, 4_096, 1_024)
+    off, dd, _ = csr(V, src, dst, 5, 1)
+    w = np.ones(dd.size, np.uint32)
+    w[:off[1]] = np.random.default_rng(3).integers(1 << 16, 1 << 20, off[1])  # the root's edges,
+    w[off[1] - 1] = 1                                                         # but for the hub's
+    exp = O.sssp(off, dd, w, 0)
+    with cg.Graph.from_csr(off, dd, w) as g:
+        for _ in range(5):
+            np.testing.assert_array_equal(g.run(SSSP, 0, cg.make_options(sssp_delta=1 << 30))[0], exp)
