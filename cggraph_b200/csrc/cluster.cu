@@ -78,7 +78,7 @@ __device__ __forceinline__ void cl_reset(ClShared& s)
 // of this CTA and adds their out-edges to `edges` (per thread; cl_next_level
 // collects it); warp-collective.  Vertices without edges are skipped; a
 // vertex for which the queue has no room spills to the global queue if
-// take(v) holds.
+// take(v) holds, and its list counts for the frontier's longest.
 template <int N, class Take>
 __device__ __forceinline__ void cl_push(ClShared& s, uint32_t buf, const bool (&pred)[N], const uint32_t (&v)[N],
                                         const uint32_t (&start)[N], const uint32_t (&deg)[N], uint32_t* spill_q,
@@ -91,9 +91,12 @@ __device__ __forceinline__ void cl_push(ClShared& s, uint32_t buf, const bool (&
         big |= pred[i] && deg[i] > kClPiece;
         edges += pred[i] ? deg[i] : 0;
     }
-    auto spill = [&](bool pred, uint32_t vv) {  // warp-collective
+    auto spill = [&](bool pred, uint32_t vv, uint32_t dd) {  // warp-collective
         if (!__any_sync(0xffffffffu, pred)) return;
-        warp_append(pred && take(vv), vv, spill_q, &st->qlen, cap, &st->status);
+        const bool taken = pred && take(vv);
+        warp_append(taken, vv, spill_q, &st->qlen, cap, &st->status);
+        const uint32_t mx = __reduce_max_sync(0xffffffffu, taken ? dd : 0u);
+        if (lane == 0 && mx) atomicMax(&st->max_deg, mx);
     };
     if (!__any_sync(0xffffffffu, big)) {
         // one entry per vertex
@@ -116,7 +119,7 @@ __device__ __forceinline__ void cl_push(ClShared& s, uint32_t buf, const bool (&
                 s.v[buf][at] = v[i];
             }
             pos += __popc(m[i]);
-            if (pos > kClQueue) spill(mine && at >= kClQueue, v[i]);
+            if (pos > kClQueue) spill(mine && at >= kClQueue, v[i], deg[i]);
         }
         return;
     }
@@ -142,7 +145,7 @@ __device__ __forceinline__ void cl_push(ClShared& s, uint32_t buf, const bool (&
             s.v[buf][at] = vv;
         };
         const bool fits = pos + n[i] <= kClQueue;
-        spill(n[i] && !fits, v[i]);
+        spill(n[i] && !fits, v[i], deg[i]);
         if (n[i] <= 4)
             for (uint32_t k = 0; k < n[i]; k++) put(pos + k, k, v[i], start[i], deg[i], fits);
         for (uint32_t todo = __ballot_sync(0xffffffffu, n[i] > 4); todo; todo &= todo - 1) {
@@ -350,6 +353,18 @@ __device__ __forceinline__ void cl_flush(ClShared& s, uint32_t buf, uint32_t ran
     if (lane_id() == 0 && mx) atomicMax(&st->max_deg, mx);
 }
 
+// The longest list of the frontier given in q[0, nf), when no level ran.
+__device__ __forceinline__ void cl_given_max_deg(cooperative_groups::cluster_group& cluster,
+                                                 const uint32_t* __restrict__ off, const uint32_t* q, uint32_t nf,
+                                                 ClusterState* st)
+{
+    uint32_t mx = 0;
+    for (uint32_t i = cluster.block_rank() * kClThreads + threadIdx.x; i < nf; i += kClThreads * cluster.num_blocks())
+        mx = max(mx, off[q[i] + 1] - off[q[i]]);
+    mx = __reduce_max_sync(0xffffffffu, mx);
+    if (lane_id() == 0 && mx) atomicMax(&st->max_deg, mx);
+}
+
 }  // namespace
 
 // BFS levels from q_in[0, nf), the vertices of level start_level.  Stops
@@ -426,6 +441,7 @@ __global__ void __launch_bounds__(kClThreads, 1)
     found = __reduce_add_sync(0xffffffffu, found);
     if (lane_id() == 0 && found) atomicAdd(&st->found, found);
     if (ok && it > 0) cl_flush(s, it & 1, rank, off, q_out, cap, st, mark);
+    if (ok && it == 0) cl_given_max_deg(cluster, off, q_in, nf, st);
     cl_leave(cluster, s, it, wait_ns);
     if (leader) {
         ClusterState h{};
@@ -601,6 +617,7 @@ __global__ void __launch_bounds__(kClThreads, 1)
         ok = cl_next_level(cluster, s, it + 1, edges, st, wait_ns);
     }
     if (ok && it > 0) cl_flush(s, it & 1, rank, off, q_out, cap, st, take);
+    if (ok && it == 0) cl_given_max_deg(cluster, off, q_in, nf, st);
     added = __reduce_add_sync(0xffffffffu, added);
     if (lane == 0 && added) atomicAdd(&st->found, added);
     if (ok && far) {

@@ -114,3 +114,26 @@ def test_spilled_vertex_leaves_once():
     with cg.Graph.from_csr(off, dd, w) as g:
         for _ in range(5):
             np.testing.assert_array_equal(g.run(SSSP, 0, cg.make_options(sssp_delta=1 << 30))[0], exp)
+
+
+@pytest.mark.gpu
+def test_spilled_hub_is_the_longest_list():
+    """A frontier whose longest list left for the global queue is kept from the grid loop, which takes lists below
+    persist_deg: seven hubs found by one thread, six fill a CTA's queue and the seventh, the longest, spills."""
+    hubs = [9_600] * 6 + [20_000]
+    leaves, each = sum(hubs), 62
+    first, V = 1 + len(hubs), 1 + len(hubs) + leaves
+    leaf = np.arange(first, V)
+    src = np.concatenate([np.zeros(len(hubs), np.int64), np.repeat(np.arange(1, first), hubs), np.repeat(leaf, each)])
+    dst = np.concatenate([np.arange(1, first), leaf, first + (np.arange(leaves * each) * 17 + 5) % leaves])
+    off, dd, _ = csr(V, src, dst, 1, 1)
+    assert np.diff(off[1:first + 1].astype(np.int64)).tolist() == hubs
+    # the hubs' lists stay far from the direction switch, so that the grid loop is in question
+    assert 4 * 15 * leaves < dd.size
+    exp, launches = O.bfs(off, dd, 0), {}
+    with cg.Graph.from_csr(off, dd) as g:
+        for deg in (8_000, 16_000, 65_536):
+            g.set_tuning({"persist_deg": deg})
+            np.testing.assert_array_equal(g.run(BFS, 0)[0], exp)
+            launches[deg] = g.stats().launches
+    assert launches[8_000] == launches[16_000] != launches[65_536]
