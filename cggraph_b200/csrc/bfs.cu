@@ -348,7 +348,8 @@ void run_bfs(cgb_graph* g, uint32_t root, const cgb_options& o)
                                              scout_exit, g->tune.persist_deg, max_levels);
             if (timing) ktimer_end(g);
             scout = r.scout;
-            maxdeg = r.max_deg;
+            if (r.levels > 0) maxdeg = r.max_deg;
+            else if (nf == 1) maxdeg = (uint32_t)scout;
             if (r.levels > 0) {
                 visited_cnt += r.found;
                 edges_to_check -= (int64_t)r.scouts;

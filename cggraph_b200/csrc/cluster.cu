@@ -78,7 +78,7 @@ __device__ __forceinline__ void cl_reset(ClShared& s)
 // of this CTA and adds their out-edges to `edges` (per thread; cl_next_level
 // collects it); warp-collective.  Vertices without edges are skipped; a
 // vertex for which the queue has no room spills to the global queue if
-// take(v) holds, and its list counts for the frontier's longest.
+// take(v) holds.
 template <int N, class Take>
 __device__ __forceinline__ void cl_push(ClShared& s, uint32_t buf, const bool (&pred)[N], const uint32_t (&v)[N],
                                         const uint32_t (&start)[N], const uint32_t (&deg)[N], uint32_t* spill_q,
@@ -91,12 +91,9 @@ __device__ __forceinline__ void cl_push(ClShared& s, uint32_t buf, const bool (&
         big |= pred[i] && deg[i] > kClPiece;
         edges += pred[i] ? deg[i] : 0;
     }
-    auto spill = [&](bool pred, uint32_t vv, uint32_t dd) {  // warp-collective
+    auto spill = [&](bool pred, uint32_t vv) {  // warp-collective
         if (!__any_sync(0xffffffffu, pred)) return;
-        const bool taken = pred && take(vv);
-        warp_append(taken, vv, spill_q, &st->qlen, cap, &st->status);
-        const uint32_t mx = __reduce_max_sync(0xffffffffu, taken ? dd : 0u);
-        if (lane == 0 && mx) atomicMax(&st->max_deg, mx);
+        warp_append(pred && take(vv), vv, spill_q, &st->qlen, cap, &st->status);
     };
     if (!__any_sync(0xffffffffu, big)) {
         // one entry per vertex
@@ -119,7 +116,7 @@ __device__ __forceinline__ void cl_push(ClShared& s, uint32_t buf, const bool (&
                 s.v[buf][at] = v[i];
             }
             pos += __popc(m[i]);
-            if (pos > kClQueue) spill(mine && at >= kClQueue, v[i], deg[i]);
+            if (pos > kClQueue) spill(mine && at >= kClQueue, v[i]);
         }
         return;
     }
@@ -145,7 +142,7 @@ __device__ __forceinline__ void cl_push(ClShared& s, uint32_t buf, const bool (&
             s.v[buf][at] = vv;
         };
         const bool fits = pos + n[i] <= kClQueue;
-        spill(n[i] && !fits, v[i], deg[i]);
+        spill(n[i] && !fits, v[i]);
         if (n[i] <= 4)
             for (uint32_t k = 0; k < n[i]; k++) put(pos + k, k, v[i], start[i], deg[i], fits);
         for (uint32_t todo = __ballot_sync(0xffffffffu, n[i] > 4); todo; todo &= todo - 1) {
@@ -353,18 +350,6 @@ __device__ __forceinline__ void cl_flush(ClShared& s, uint32_t buf, uint32_t ran
     if (lane_id() == 0 && mx) atomicMax(&st->max_deg, mx);
 }
 
-// The longest list of the frontier given in q[0, nf), when no level ran.
-__device__ __forceinline__ void cl_given_max_deg(cooperative_groups::cluster_group& cluster,
-                                                 const uint32_t* __restrict__ off, const uint32_t* q, uint32_t nf,
-                                                 ClusterState* st)
-{
-    uint32_t mx = 0;
-    for (uint32_t i = cluster.block_rank() * kClThreads + threadIdx.x; i < nf; i += kClThreads * cluster.num_blocks())
-        mx = max(mx, off[q[i] + 1] - off[q[i]]);
-    mx = __reduce_max_sync(0xffffffffu, mx);
-    if (lane_id() == 0 && mx) atomicMax(&st->max_deg, mx);
-}
-
 }  // namespace
 
 // BFS levels from q_in[0, nf), the vertices of level start_level.  Stops
@@ -441,13 +426,13 @@ __global__ void __launch_bounds__(kClThreads, 1)
     found = __reduce_add_sync(0xffffffffu, found);
     if (lane_id() == 0 && found) atomicAdd(&st->found, found);
     if (ok && it > 0) cl_flush(s, it & 1, rank, off, q_out, cap, st, mark);
-    if (ok && it == 0) cl_given_max_deg(cluster, off, q_in, nf, st);
     cl_leave(cluster, s, it, wait_ns);
     if (leader) {
         ClusterState h{};
         h.qlen = __ldcg(&st->qlen);
         h.status = __ldcg(&st->status);
-        h.max_deg = __ldcg(&st->max_deg);
+        // (kept where vertices spill, the longest list cost SSSP rounds 5 to 12 %)
+        h.max_deg = word & ~kEntryMask ? 0xFFFFFFFFu : __ldcg(&st->max_deg);
         h.found = __ldcg(&st->found);
         h.levels = it;
         h.scout = scout;
@@ -617,7 +602,6 @@ __global__ void __launch_bounds__(kClThreads, 1)
         ok = cl_next_level(cluster, s, it + 1, edges, st, wait_ns);
     }
     if (ok && it > 0) cl_flush(s, it & 1, rank, off, q_out, cap, st, take);
-    if (ok && it == 0) cl_given_max_deg(cluster, off, q_in, nf, st);
     added = __reduce_add_sync(0xffffffffu, added);
     if (lane == 0 && added) atomicAdd(&st->found, added);
     if (ok && far) {
@@ -633,7 +617,8 @@ __global__ void __launch_bounds__(kClThreads, 1)
         h.qlen = __ldcg(&st->qlen);
         h.status = __ldcg(&st->status);
         h.far_left = __ldcg(&st->far_left);
-        h.max_deg = __ldcg(&st->max_deg);
+        // (kept where vertices spill, the longest list cost SSSP rounds 5 to 12 %)
+        h.max_deg = word & ~kEntryMask ? 0xFFFFFFFFu : __ldcg(&st->max_deg);
         h.found = __ldcg(&st->found);
         h.levels = it;
         h.scout = scout;
@@ -776,7 +761,7 @@ PersistResult bfs_cluster(cgb_graph* g, uint32_t cur, uint32_t nf, uint32_t leve
     r.cur = h.levels ? cur ^ 1 : cur;
     r.nf = h.levels ? h.qlen : nf;
     r.scout = h.scout;
-    r.max_deg = h.max_deg;
+    r.max_deg = std::min(h.max_deg, g->max_degree);
     r.found = h.found;
     r.scouts = h.scouts;
     return r;
@@ -798,7 +783,7 @@ SsspTail sssp_cluster(cgb_graph* g, uint32_t cur, uint32_t nf, uint64_t thr, uin
     t.r.cur = h.levels ? cur ^ 1 : cur;
     t.r.nf = h.levels ? h.qlen : nf;
     t.r.scout = h.scout;
-    t.r.max_deg = h.max_deg;
+    t.r.max_deg = std::min(h.max_deg, g->max_degree);
     t.r.added = h.found;
     t.thr = h.thr;
     t.nfar = h.far_left;

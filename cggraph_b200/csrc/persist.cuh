@@ -78,7 +78,7 @@ struct ClusterState {
     uint32_t qlen;      // frontier vertices left in the global queue
     uint32_t status;    // 1 = queue overflow, 2 = a wait gave up
     uint32_t levels;    // levels (rounds) run
-    uint32_t max_deg;   // longest list of the frontier
+    uint32_t max_deg;   // longest list of the frontier, if a level ran (0xFFFFFFFF: not known, vertices spilled)
     uint32_t found;     // BFS: vertices reached; SSSP: list pieces expanded
     uint32_t far_left;  // SSSP: vertices left in the far bitmap
     unsigned long long scout;   // out-edges of the frontier
@@ -90,7 +90,7 @@ struct PersistResult {
     uint32_t levels = 0;       // levels (rounds) run
     uint32_t cur = 0;          // queue index holding the frontier on exit
     uint32_t nf = 0;           // frontier size on exit
-    uint32_t max_deg = 0;      // its max out-degree
+    uint32_t max_deg = 0;      // its max out-degree, if a level ran (a bound: the graph's, where it is not known)
     uint32_t found = 0;        // vertices reached (BFS)
     unsigned long long scout = 0;   // its out-edges (BFS, cluster loops)
     unsigned long long added = 0;   // sum of the frontier sizes run

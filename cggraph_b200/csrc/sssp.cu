@@ -490,7 +490,7 @@ static void sssp_loop(cgb_graph* g, uint32_t root, uint32_t delta, const cgb_opt
         iters += t.r.levels;
         expanded += t.r.added;
         nnear = t.r.nf;
-        near_maxdeg = t.r.max_deg;
+        if (t.r.levels > 0) near_maxdeg = t.r.max_deg;
         nfar = t.nfar;
         thr = t.thr;
         bucket_lo = t.bucket_lo;
