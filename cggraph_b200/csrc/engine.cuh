@@ -157,6 +157,7 @@ struct cgb_graph {
     uint32_t* aux_bm = nullptr;           // 3 bitmaps: device-resident SSSP near dedup
     void* persist = nullptr;              // state of the device-resident loops
     void* cluster = nullptr;              // state of the cluster loops
+    uint32_t cluster_rounds = 1u << 30;   // SSSP rounds and splits of one cluster launch
     cgb::MsBuffers* ms = nullptr;         // multi-root BFS masks
     cgb::MsspBuffers* mssp = nullptr;     // multi-root SSSP distances and masks
 

@@ -1139,15 +1139,23 @@ static void group_retire(cgb_server* s, Group& G, unsigned long long fin, unsign
 // retires as a batched one does.
 constexpr uint32_t kLoneMaxDue = 4;
 
+// Rounds after which the cluster loop of an SSSP run without the
+// cooperative-launch lock returns to the host: a millisecond or two (3 to 6
+// us a round on road-like frontiers).
+constexpr uint32_t kSharedRounds = 256;
+
 static void lone_run(cgb_server* s, Group& G, int a, uint32_t k)
 {
     cgb_graph* g = (a == 1 && s->shadow) ? s->shadow : s->g;
-    // the engine's device-resident loops are cooperative launches, as the
-    // groups' are, so a run that may start one takes the cooperative-launch
-    // lock: any BFS run (its small-frontier levels), and an SSSP run only
-    // where its device-resident tail can run (no list of persist_deg edges or
-    // more; on power-law graphs it never does, and SSSP runs then overlap
-    // BFS runs and ticks)
+    // the engine's grid loops are cooperative launches, as the groups' are, so
+    // a run that may start one takes the cooperative-launch lock: any BFS run
+    // (its small-frontier levels), and an SSSP run where its grid loop can run
+    // (no list of persist_deg edges or more).  Elsewhere SSSP runs overlap BFS
+    // runs and ticks.  Their cluster loop holds 16 SMs, with 196 KB of shared
+    // memory and 45 k registers each: a BFS group's loop needs one small CTA on
+    // every SM and its grid barrier waits 0.3 s for the last, so without the
+    // lock the cluster loop leaves after kSharedRounds and never comes near
+    // that, whatever fits beside it.
     const cgb_tuning& t = g->tune_alg[CGB_SSSP];
     const bool coop_needed = a == 0 || (t.persist_enter > 0 && g->max_degree < t.persist_deg);
     Clock::time_point t0;
@@ -1163,6 +1171,12 @@ static void lone_run(cgb_server* s, Group& G, int a, uint32_t k)
         cgb_options o;
         memset(&o, 0, sizeof(o));
         o.struct_size = sizeof(o);
+        struct Rounds {
+            cgb_graph* g;
+            uint32_t was;
+            Rounds(cgb_graph* gr, uint32_t n) : g(gr), was(gr->cluster_rounds) { g->cluster_rounds = n; }
+            ~Rounds() { g->cluster_rounds = was; }
+        } rounds(g, coop_needed ? g->cluster_rounds : kSharedRounds);
         run_one(g, G.alg, G.root[k], o, nullptr);
         CGB_CUDA_TRY(cudaMemcpyAsync(G.region + (size_t)k * g->V, g->value, (size_t)g->V * 4,
                                      cudaMemcpyDeviceToDevice, g->stream));

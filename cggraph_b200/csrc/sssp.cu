@@ -483,7 +483,7 @@ static void sssp_loop(cgb_graph* g, uint32_t root, uint32_t delta, const cgb_opt
             kind == kClusterTail
                 ? sssp_cluster(g, cur, (uint32_t)nnear, thr, (uint32_t)nfar, bucket_lo, far_bm, delta,
                                std::min(g->tune.persist_enter, 2 * g->tune.cluster_enter), kClusterExitEdges,
-                               tail_delta_chosen ? kClusterFar : 0, max_rounds)
+                               tail_delta_chosen ? kClusterFar : 0, std::min(max_rounds, g->cluster_rounds))
                 : sssp_device_tail(g, cur, (uint32_t)nnear, near_maxdeg, thr, (uint32_t)nfar, bucket_lo, far_bm, delta,
                                    g->tune.persist_enter, g->tune.persist_deg, max_rounds);
         if (timing) ktimer_end(g);

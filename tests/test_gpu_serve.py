@@ -145,3 +145,30 @@ def test_server_memory_budget_caps_slots(oracle):
                 srv.submit(SSSP, 0)
             with pytest.raises(cg.CgbError):
                 srv.submit(BFS, V)
+
+
+@pytest.mark.parametrize("flags", [0, L.SERVER_BATCH_ONLY])
+def test_server_hub_and_long_path(oracle, flags):
+    """A list of persist_deg edges or more (SSSP runs without the
+    cooperative-launch lock) beside thousands of thin levels (their cluster
+    loop runs for most of the query), BFS and SSSP served together."""
+    path, hub = 20_000, 3_000
+    V = path + hub
+    rng = np.random.default_rng(11)
+    src = np.concatenate([np.arange(path - 1), np.arange(1, path), np.zeros(hub, np.int64), np.arange(path, V)])
+    dst = np.concatenate([np.arange(1, path), np.arange(path - 1), np.arange(path, V), np.zeros(hub, np.int64)])
+    order = np.lexsort((dst, src))
+    src, dst = src[order], dst[order].astype(np.uint32)
+    off = np.zeros(V + 1, np.uint32)
+    off[1:] = np.cumsum(np.bincount(src, minlength=V))
+    w = rng.integers(1, 65, dst.size).astype(np.uint32)
+    queries = [(i % 2, int(r)) for i, r in enumerate(rng.integers(0, V, 12))]
+    with cg.Graph.from_csr(off, dst, w) as g:
+        g._host_off = off
+        assert int(np.diff(off.astype(np.int64)).max()) >= g.get_tuning(SSSP)["persist_deg"]
+        recs, _ = _serve_and_check(g, queries, np.arange(12) * 2_000.0, bfs_slots=4, sssp_slots=4, flags=flags)
+        assert len(recs) == 12
+    for alg, root in queries[:4]:
+        exp = oracle.bfs(off, dst, root) if alg == BFS else oracle.sssp(off, dst, w, root)
+        with cg.Graph.from_csr(off, dst, w) as g:
+            np.testing.assert_array_equal(g.run(alg, root)[0], exp)
