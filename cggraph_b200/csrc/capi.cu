@@ -332,7 +332,13 @@ void run_one(cgb_graph* g, int alg, uint32_t root_or_iters, const cgb_options& o
     }
     const uint64_t V = g->V, E = g->E;
     if (alg != CGB_PR) g->result = g->value;
-    if (out) copy_any(out, g->result, (size_t)V * (alg == CGB_PR ? 8 : 4), g->stream);
+    g->result_alg = alg;  // with the pointer: its element size
+    // a copy that is refused ends the call with its error, but only after the
+    // run's own end: the graph keeps the result and its statistics
+    const cudaError_t copied =
+        out ? cudaMemcpyAsync(out, g->result, (size_t)V * (alg == CGB_PR ? 8 : 4), cudaMemcpyDefault, g->stream)
+            : cudaSuccess;
+    if (copied != cudaSuccess) cudaGetLastError();
     if (alg == CGB_BFS || alg == CGB_SSSP) count_reached(g);
     else CGB_CUDA_TRY(cudaStreamSynchronize(g->stream));
     CGB_CUDA_TRY(cudaGetLastError());
@@ -352,7 +358,7 @@ void run_one(cgb_graph* g, int alg, uint32_t root_or_iters, const cgb_options& o
         g->stats.reached = V;
         g->stats.alg_bytes = (12 * E + 20 * V + 4) * g->stats.iterations;
     }
-    g->result_alg = alg;
+    CGB_CUDA_TRY(copied);
 }
 }  // namespace cgb
 

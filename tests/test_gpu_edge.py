@@ -502,3 +502,36 @@ def test_device_barrier_gives_up_and_context_survives(oracle):
     with cg.Graph.from_csr(off, dst, w) as g:
         np.testing.assert_array_equal(g.run(BFS, root)[0], oracle.bfs(off, dst, root))
         np.testing.assert_array_equal(g.run(SSSP, root)[0], oracle.sssp(off, dst, w, root))
+
+
+def test_refused_result_copy_leaves_a_consistent_graph(oracle):
+    """A run whose result copy the driver refuses (a host buffer of which only
+    the first part is registered) returns an error, and the graph still holds
+    that run's result, with its element size, and statistics: the run before
+    it had 8-byte elements."""
+    import ctypes
+    import mmap
+    import torch
+    off, dst, w = oracle.rmat_graph(14, 8, seed=3)
+    V = off.size - 1
+    root = int(np.diff(off.astype(np.int64)).argmax())
+    exp = oracle.bfs(off, dst, root)
+    mem = mmap.mmap(-1, 4 * V)
+    buf = np.frombuffer(mem, np.uint32)
+    rt = torch.cuda.cudart()
+    with cg.Graph.from_csr(off, dst, w) as g:
+        g.run(PR, 2)
+        assert int(rt.cudaHostRegister(buf.ctypes.data, 2 * V, 0)) == 0
+        try:
+            with pytest.raises(CgbError) as e:
+                g.run(BFS, root, out=buf)
+        finally:
+            assert int(rt.cudaHostUnregister(buf.ctypes.data)) == 0
+        assert e.value.status == L.ECUDA
+        got = np.full(2 * V, 5, np.uint32)
+        assert L.lib().cgb_graph_result_download(ctypes.c_void_p(g.handle.value), got.ctypes.data) == L.OK
+        np.testing.assert_array_equal(got[:V], exp)
+        assert np.all(got[V:] == 5)
+        s = g.stats()
+        assert s.reached == np.count_nonzero(exp != VMAX) and s.alg_bytes > 0
+        np.testing.assert_array_equal(g.run(SSSP, root, out=buf)[0], oracle.sssp(off, dst, w, root))
