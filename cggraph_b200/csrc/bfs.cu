@@ -320,6 +320,7 @@ void run_bfs(cgb_graph* g, uint32_t root, const cgb_options& o)
         return in;
     };
 
+    bool cluster_passed = false;  // the cluster loop ran no level of this frontier
     while (nf > 0) {
         CGB_REQUIRE(iters < max_iters, CGB_ETIMEOUT, "BFS iteration budget exhausted");
         // ----- direction decision
@@ -331,7 +332,8 @@ void run_bfs(cgb_graph* g, uint32_t root, const cgb_options& o)
         const bool far_off = !heur && (double)scout * alpha * 4.0 <= (double)edges_to_check;
         const uint64_t scout_exit = (uint64_t)std::max(0.0, (double)edges_to_check / alpha / 4.0);
         const uint32_t max_levels = (uint32_t)std::min<uint64_t>(max_iters - iters, 1u << 20);
-        const bool use_cluster = cluster_ok && nf <= std::min(g->tune.cluster_enter, g->tune.persist_enter) &&
+        const bool use_cluster = cluster_ok && !cluster_passed &&
+                                 nf <= std::min(g->tune.cluster_enter, g->tune.persist_enter) &&
                                  (whole || (far_off && scout <= kClusterEnterEdges));
         const bool use_grid = persist_ok && !use_cluster && far_off && nf <= g->tune.persist_enter &&
                               maxdeg < g->tune.persist_deg && scout > 0;
@@ -363,7 +365,14 @@ void run_bfs(cgb_graph* g, uint32_t root, const cgb_options& o)
                 have_policy_out = false;
                 continue;
             }
+            if (use_cluster) {
+                // the direction is decided again, now that the loop has counted
+                // the frontier's out-edges (a root's were not known before)
+                cluster_passed = true;
+                continue;
+            }
         }
+        cluster_passed = false;
         const int out = cur ^ 1;
         // the heuristic's expansion of a push level: every list of 32 edges or
         // more chunked for small frontiers, else the degree-binned tiers

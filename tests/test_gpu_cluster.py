@@ -137,3 +137,22 @@ def test_spilled_hub_is_the_longest_list():
             np.testing.assert_array_equal(g.run(BFS, 0)[0], exp)
             launches[deg] = g.stats().launches
     assert launches[8_000] == launches[16_000] != launches[65_536]
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("leaves,degree", [(200_000, 6), (300_000, 4)])
+def test_root_beyond_the_cluster_pulls(leaves, degree):
+    """A root with more than a fifteenth of the edges is pulled from, as the direction rule has it, though the cluster
+    loop was asked first and its out-edges were not known then."""
+    V, src, dst = star(leaves, degree)
+    off, dd, _ = csr(V, src[src != dst], dst[src != dst], 5, 1)
+    root_edges = int(off[1])
+    assert dd.size > 1 << 20 and 15 * root_edges > dd.size  # not a whole run in the cluster; beyond the switch point
+    exp, pulls = O.bfs(off, dd, 0), []
+    with cg.Graph.from_csr(off, dd) as g:
+        for tuning in ({}, {"cluster_enter": 0}):
+            g.set_tuning(tuning)
+            np.testing.assert_array_equal(g.run(BFS, 0)[0], exp)
+            s = g.stats()
+            pulls.append((s.pulls_bu, s.pushes_td))
+    assert pulls[0] == pulls[1] and pulls[0][0] > 0
