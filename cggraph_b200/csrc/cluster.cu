@@ -309,8 +309,9 @@ __device__ __forceinline__ uint32_t cl_load(cooperative_groups::cluster_group& c
     return edges;
 }
 
-// Visits every entry of buffer buf: visit(entry, start, len, single) is
-// warp-collective (len 0 on idle lanes), entry a pointer to the vertex.  A
+// Visits every entry of buffer buf: visit(entry, start, len, flags) is
+// warp-collective (len 0 on idle lanes), entry a pointer to the vertex, flags
+// kClFirst and kClSingle (0 on idle lanes).  A
 // CTA takes the entries j = rank mod ctas of every queue, neighbouring lanes
 // from neighbouring CTAs' queues, so that all CTAs have equal shares and a
 // small frontier fills few warps.
@@ -326,7 +327,7 @@ __device__ __forceinline__ void cl_for_entries(cooperative_groups::cluster_group
         if (!__any_sync(0xffffffffu, j < n)) break;
         const uint64_t list = j < n ? r->list[buf][j] : 0;
         const uint32_t len = (uint32_t)(list >> 32);
-        visit(&r->v[buf][j], (uint32_t)list, len & (kClSingle - 1), (len & kClSingle) != 0);
+        visit(&r->v[buf][j], (uint32_t)list, len & (kClSingle - 1), len & (kClFirst | kClSingle));
     }
 }
 
@@ -353,7 +354,7 @@ __device__ __forceinline__ void cl_flush(ClShared& s, uint32_t buf, uint32_t ran
 }  // namespace
 
 // BFS levels from q_in[0, nf), the vertices of level start_level.  Stops
-// before a level whose frontier exceeds nf_exit vertices or scout_exit
+// before a level whose frontier exceeds nf_exit queue entries or scout_exit
 // out-edges, after a spill or max_levels levels.
 __global__ void __launch_bounds__(kClThreads, 1)
     k_bfs_cluster(const uint32_t* __restrict__ off, const uint32_t* __restrict__ dst, uint32_t* level,
@@ -386,7 +387,7 @@ __global__ void __launch_bounds__(kClThreads, 1)
         scouts += scout;
         const uint32_t next_level = start_level + it + 1;
         uint32_t edges = 0;
-        cl_for_entries(cluster, s, buf, [&](const uint32_t* entry, uint32_t start, uint32_t len, bool) {
+        cl_for_entries(cluster, s, buf, [&](const uint32_t* entry, uint32_t start, uint32_t len, uint32_t) {
             // the visited bit of a queued vertex, off the level's chain
             if (len) {
                 const uint32_t v = *entry;
@@ -488,12 +489,12 @@ __global__ void __launch_bounds__(kClThreads, 1)
         if (entries) {
             const uint32_t bound = (uint32_t)min(thr, (unsigned long long)kValueMax);
             uint32_t far_set = 0;
-            cl_for_entries(cluster, s, buf, [&](const uint32_t* entry, uint32_t start, uint32_t len, bool single) {
+            cl_for_entries(cluster, s, buf, [&](const uint32_t* entry, uint32_t start, uint32_t len, uint32_t flags) {
                 const uint32_t v = len ? *entry : 0u;
                 const uint32_t du = len ? __ldcg(dist + v) : 0u;
                 // a vertex queued twice: the second entry is skipped
-                const bool again = len && single && atomicMax(stamp + v, it + 1) == it + 1;
-                added += len && !again ? 1u : 0u;
+                const bool again = (flags & kClSingle) && atomicMax(stamp + v, it + 1) == it + 1;
+                added += (flags & kClFirst) && !again ? 1u : 0u;  // a vertex counts with its first entry
                 for (uint32_t b = 0; __any_sync(0xffffffffu, b < len); b += kClBatch) {
                     uint32_t d[kClBatch], nd[kClBatch], old[kClBatch], lo[kClBatch], dg[kClBatch];
                     bool near[kClBatch], to_far[kClBatch];

@@ -25,7 +25,8 @@ constexpr uint32_t kBarrierSpins = 1u << 22;  // mostly x ~64 ns: gives up after
 
 // The cluster loops (cluster.cu) take frontiers of at most
 // cgb_tuning.cluster_enter vertices and kClusterEnterEdges out-edges, and
-// return once a frontier exceeds twice the entry size or kClusterExitEdges:
+// return once a frontier exceeds twice cluster_enter in queue entries (pieces
+// of at most 8 edges) or kClusterExitEdges:
 // beyond, 16 SMs take longer than a host round trip over all of them.  Entry
 // bounds of 8 k / 16 k / 32 k / 64 k / 128 k edges: SSSP RMAT-18 0.42 / 0.41
 // / 0.41 / 0.43 / 0.43 ms, RMAT-15 0.30 / 0.28 / 0.29 / 0.27 / 0.26, Chung-Lu
@@ -79,7 +80,7 @@ struct ClusterState {
     uint32_t status;    // 1 = queue overflow, 2 = a wait gave up
     uint32_t levels;    // levels (rounds) run
     uint32_t max_deg;   // longest list of the frontier, if a level ran (0xFFFFFFFF: not known, vertices spilled)
-    uint32_t found;     // BFS: vertices reached; SSSP: list pieces expanded
+    uint32_t found;     // BFS: vertices reached; SSSP: vertices expanded
     uint32_t far_left;  // SSSP: vertices left in the far bitmap
     unsigned long long scout;   // out-edges of the frontier
     unsigned long long scouts;  // BFS: sum of the out-edges of the levels run
@@ -115,7 +116,8 @@ uint32_t cluster_loop_ctas();
 // Launches a cluster in which one CTA keeps a level's counts back;
 // CGB_ETIMEOUT when the wait for them ended after limit_us (a self-check).
 cgb_status cluster_timeout_check(uint32_t limit_us);
-// BFS levels from q[cur][0, nf) (level `level`): bounds as bfs_persistent.
+// BFS levels from q[cur][0, nf) (level `level`): bounds as bfs_persistent, but
+// nf_exit counts queue entries, pieces of at most 8 edges.
 // Vertices without out-edges are reached but not part of a frontier.
 PersistResult bfs_cluster(cgb_graph* g, uint32_t cur, uint32_t nf, uint32_t level, uint32_t nf_exit,
                           uint32_t scout_exit, uint32_t max_levels);
@@ -145,7 +147,7 @@ SsspTail sssp_device_tail(cgb_graph* g, uint32_t cur, uint32_t nf, uint32_t max_
                           uint32_t max_rounds);
 
 // The same in a cluster loop, which leaves when a frontier exceeds nf_exit
-// vertices or scout_exit out-edges (r.scout: the out-edges of the frontier it
+// queue entries or scout_exit out-edges (r.scout: the out-edges of the frontier it
 // returns), and before a split with more than far_exit far vertices.
 SsspTail sssp_cluster(cgb_graph* g, uint32_t cur, uint32_t nf, uint64_t thr, uint32_t nfar, uint64_t bucket_lo,
                       uint32_t* far_bm, uint32_t delta, uint32_t nf_exit, uint32_t scout_exit, uint32_t far_exit,

@@ -156,3 +156,45 @@ def test_root_beyond_the_cluster_pulls(leaves, degree):
             s = g.stats()
             pulls.append((s.pulls_bu, s.pushes_td))
     assert pulls[0] == pulls[1] and pulls[0][0] > 0
+
+
+@pytest.mark.gpu
+def test_learned_delta_sees_vertices_not_pieces():
+    """At the first bucket boundary the network is told how many vertices have been expanded, in the cluster as by the
+    host's rounds: nine here (the root and eight hubs), whose lists are 2001 pieces.  A hand-made network picks four
+    times the width when they are more than a two-hundredth of the vertices."""
+    import torch
+    from cggraph_b200 import _lib as L, policy
+    hubs, leaves, fill, each = 8, 2_000, 1 << 16, 1 << 10  # the filler brings the edges to where the network is asked
+    first = 1 + hubs + hubs * leaves
+    V = first + fill
+    dev = dict(device="cuda", dtype=torch.int32)
+    deg = torch.tensor([hubs] + [leaves] * hubs + [0] * (hubs * leaves) + [each] * fill, **dev)
+    off = torch.zeros(V + 1, **dev)
+    off[1:] = deg.cumsum(0)
+    dst = torch.cat([torch.arange(1, first, **dev), (first + torch.arange(each, **dev)).repeat(fill)])
+    w = torch.full_like(dst, 64)
+    w[:hubs] = 1
+    w[hubs:hubs + hubs * leaves] = 1000
+    p = np.zeros(policy.NP, np.float32)
+    w1, w2, w3 = 0, 24 * 64 + 64, 24 * 64 + 64 + 64 * 64 + 64
+    p[w1 + 23 * 64] = 1000.0    # settled / V
+    p[24 * 64] = -5.0
+    p[w2] = 1.0
+    p[w3 + policy.SSSP_DELTA[4]] = -1.0
+    p[w3 + 64 * 14:] = 1.0
+    exp = np.full(V, cg.VALUE_MAX, np.uint32)
+    exp[0], exp[1:1 + hubs], exp[1 + hubs:first] = 0, 1, 1001
+    deltas = []
+    policy.load(p)
+    try:
+        with cg.Graph.from_csr(off, dst, w, vertexNum=V, edgeNum=dst.numel()) as g:
+            for tuning in ({"cluster_enter": 0}, {"cluster_enter": 8192}):
+                g.set_tuning(tuning)
+                np.testing.assert_array_equal(g.run(SSSP, 0, cg.make_options(schedule=L.SCHED_LEARNED))[0], exp)
+                deltas.append(g.stats().sssp_delta)
+            g.run(SSSP, 0)
+            deltas.append(g.stats().sssp_delta)
+    finally:
+        policy.load(None)
+    assert deltas[0] == deltas[1] == deltas[2] < 1000
