@@ -819,16 +819,30 @@ uint32_t sssp_delta_for(const cgb_graph* g, double c)
     return (uint32_t)d;
 }
 
-// Meshes (no list of kMeshDeg edges) of kMeshLarge vertices or more take c =
-// 64: their near sets grow with the bucket and the graph's width, and the
-// cluster loop's 16 SMs are full from a few thousand vertices on.  c = 128 /
-// 64: 500^2 grid 3.8 / 3.9 ms, 700 x 901 6.84 / 6.69, 1000^2 8.7 / 7.8, 2000^2
-// 29.9 / 26.2, 3000^2 73.9 / 44.3, 4800 x 5000 139.5 / 138.1.
+// Graphs without hubs (no list of kMeshDeg edges) of kMeshLarge vertices or
+// more whose edge lengths differ take c = 64: on meshes their near sets grow
+// with the bucket and the graph's width, and the cluster loop's 16 SMs are
+// full from a few thousand vertices on.  Where all lengths are equal a bucket
+// is a few whole levels, a wider one saves splits and relaxes no edge twice:
+// they keep 128, on meshes and random graphs alike.  (Equal lengths show in
+// the sum alone: a mean that is a whole number.  Lengths that differ and have
+// such a mean just keep 128.)  c = 128 / 64, ms:
+//                          lengths 1 .. 1000    all equal
+//   700 x 901 grid             5.61 /  5.16     3.67 / 3.81
+//   1000^2                     8.54 /  7.88     5.49 / 5.72
+//   3000^2                     80.9 /  45.0     25.2 / 27.9
+//   4800 x 5000                 154 /   145     57.1 / 66.4
+//   100 x 20000                91.2 /  96.3     60.3 / 62.5
+//   200^3                      17.8 /  17.1     9.99 / 11.2
+//   random, 2^19 x 16          3.02 /  3.17     0.63 / 0.80
+//   random, 2^23 x 4           5.38 /  5.45     1.96 / 2.00
+//   random, 2^23 x 8           8.52 /  8.54     2.16 / 3.12
 constexpr uint32_t kMeshDeg = 64, kMeshLarge = 1u << 19;
 
 uint32_t sssp_default_delta(const cgb_graph* g)
 {
-    return sssp_delta_for(g, g->max_degree < kMeshDeg && g->V >= kMeshLarge ? 64.0 : 128.0);
+    const bool lengths_differ = g->w && g->E && g->sum_w % g->E != 0;
+    return sssp_delta_for(g, g->max_degree < kMeshDeg && g->V >= kMeshLarge && lengths_differ ? 64.0 : 128.0);
 }
 
 void run_sssp(cgb_graph* g, uint32_t root, const cgb_options& o)

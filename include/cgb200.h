@@ -71,7 +71,8 @@ typedef struct cgb_options {
     int32_t schedule;       /* cgb_schedule */
     int32_t variant;        /* cgb_variant, for CGB_SCHED_FIXED */
     uint32_t sssp_delta;    /* 0 = heuristic: 128 * mean weight / mean degree (64 x for multi-root passes and
-                               for meshes of 2^19 vertices or more) */
+                               for graphs of 2^19 vertices or more with no list of 64 edges and lengths
+                               that differ) */
     double bfs_alpha;       /* Beamer alpha, 0 = 15 */
     double bfs_beta;        /* Beamer beta, 0 = 18 */
     uint64_t max_iterations;/* 0 = unlimited (V + 1 levels bound BFS anyway) */

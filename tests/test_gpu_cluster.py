@@ -198,3 +198,25 @@ def test_learned_delta_sees_vertices_not_pieces():
     finally:
         policy.load(None)
     assert deltas[0] == deltas[1] == deltas[2] < 1000
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("weight,factor", [(None, 128), (1, 128), (7, 128), ("mixed", 64)])
+def test_default_width_of_large_meshes(weight, factor):
+    """Graphs of 2^19 vertices or more without hubs: narrower default buckets only where edge lengths differ."""
+    rows, cols = 725, 724
+    with cg.Graph.grid(rows, cols, seed=1, wmax=1) as g:
+        off, dst, _ = g.download(False)
+    w = None
+    if weight == "mixed":
+        w = np.random.default_rng(2).integers(1, 1001, dst.size).astype(np.uint32)
+        w[0] += 1 if w.sum(dtype=np.uint64) % dst.size == 0 else 0
+    elif weight:
+        w = np.full(dst.size, weight, np.uint32)
+    mean = 1.0 if w is None else w.sum(dtype=np.uint64) / dst.size
+    root = rows * cols // 2
+    with cg.Graph.from_csr(off, dst, w) as g:
+        got, _ = g.run(SSSP, root)
+        assert g.stats().sssp_delta == int(factor * mean / (dst.size / (rows * cols)))
+    exp = O.bfs(off, dst, root) * (weight or 1) if weight != "mixed" else O.sssp(off, dst, w, root)
+    np.testing.assert_array_equal(got, exp)
