@@ -29,8 +29,9 @@ namespace cgb {
 // also provides
 //   template <int M> __device__ void edges(const bool (&valid)[M],
 //                                          const uint32_t (&e)[M],
-//                                          const uint32_t (&msg)[M]) const;
-// (warp-collective, like edge) which visits M edge slots per lane at once:
+//                                          const uint32_t (&msg)[M]);
+// (warp-collective, like edge; it may keep counts in the op, which is the
+// thread's own) which visits M edge slots per lane at once:
 // every load of the M slots is issued before any of them is used, so a lane
 // keeps M gathers in flight instead of one dependent chain per edge.  The
 // expansion loops below hand such ops N slots per lane (32 * N edges per
@@ -400,23 +401,36 @@ __global__ void __launch_bounds__(kBlk) k_push_binned(const uint32_t* __restrict
 
 // One warp per chunk descriptor, grid-stride over the chunk queue: warps
 // run ahead of one another, so that a few hundred edges per chunk keep many
-// chains of loads in flight.
+// chains of loads in flight.  Ops without batched visits take a chunk with the
+// whole CTA: one edge per lane at a time, a warp's chunk of 1024 edges is 32
+// chains of dependent loads one after the other.  Label propagation, a chunk
+// by a warp / by a CTA: RMAT-20 1.37 / 0.97 ms (and 6 rounds instead of 5: the
+// long lists' labels arrive late), RMAT-16 0.28 / 0.18.
 template <class Op, int kBlk>
 __global__ void __launch_bounds__(kBlk) k_push_chunks(const uint2* __restrict__ chunk_q, const uint32_t* chunk_len,
                                                         uint32_t chunk_cap, Op op, uint32_t chunk)
 {
     const uint32_t n = min(*chunk_len, chunk_cap);
-    // CTAs take the first chunks one warp each before any takes a second
-    const uint32_t w0 = (threadIdx.x >> 5) * gridDim.x + blockIdx.x, warps = gridDim.x * (kBlk / 32);
     if (blockIdx.x >= n) return;
     op.block_begin();
     __syncthreads();
-    for (uint32_t c = w0; c < n; c += warps) {
+    constexpr bool kByCta = op_batch<Op>::value == 1;
+    // (warps: CTAs take the first chunks one warp each before any takes a second)
+    const uint32_t c0 = kByCta ? blockIdx.x : (threadIdx.x >> 5) * gridDim.x + blockIdx.x;
+    const uint32_t step = kByCta ? gridDim.x : gridDim.x * (kBlk / 32);
+    for (uint32_t c = c0; c < n; c += step) {
         const uint2 d = chunk_q[c];
         uint32_t start, deg, msg;
         if (!op.load(d.x, start, deg, msg)) continue;
-        const uint32_t cs = d.y * chunk;
-        warp_range(op, start + cs, start + min(deg, cs + chunk), msg);
+        const uint32_t cs = d.y * chunk, ce = min(deg, cs + chunk);
+        if constexpr (kByCta) {
+            for (uint32_t k = cs; k < ce; k += kBlk) {
+                const uint32_t i = k + threadIdx.x;
+                op.edge(i < ce, i < ce ? start + i : 0u, msg);
+            }
+        } else {
+            warp_range(op, start + cs, start + ce, msg);
+        }
     }
     __syncthreads();
     op.block_end();
