@@ -14,8 +14,8 @@
 //      initialisation of ECL-CC, Jaiganesh and Burtscher 2018);
 //   2. one round that links v with its second neighbour, and with its first
 //      one where step 1 left it pointing at itself (first neighbour larger);
-//      on graphs with hubs it runs on a sample of the vertices first, and the
-//      full round skips the giant component that step 3 finds after that
+//      on graphs with hubs or long enough lists it runs on a sample of the
+//      vertices first, and the full round skips the giant component that step 3 finds after that
 //      sample and a compress; every find halves the path it walks, so no
 //      other compress pass runs before step 5;
 //   3. find the roots of 1024 hashed vertices and take the most frequent
@@ -481,8 +481,13 @@ static void cc_afforest(cgb_graph* g, bool weak)
     // walk again (RMAT-20 took as long as RMAT-23).  A hashed sample of the
     // vertices merges the large trees first, a compress points everyone at
     // the merged roots, and the full round then finds equal parents.
-    // (RMAT-20 weak: 0.46 -> 0.16 ms, RMAT-24: 1.0 -> 0.75 ms.)  Meshes have
-    // no such trees.
+    // (RMAT-20 weak: 0.46 -> 0.16 ms, RMAT-24: 1.0 -> 0.75 ms.)  Random graphs
+    // have them too, from some mean list length on: without / with the sample,
+    // weak components of 2^20 vertices of 1 / 2 / 3 / 4 out-edges 0.22 / 0.27,
+    // 0.45 / 0.27, 0.70 / 0.31 and 0.80 / 0.32 ms, 2^18 of 16 0.46 / 0.18;
+    // symmetric, mean length 8 / 10 / 12 / 14, 1.0 / 1.2, 0.39 / 0.22, 0.73 /
+    // 0.20 and 0.52 / 0.20, 2^18 of 32 0.56 / 0.14.  Meshes (lists below
+    // kSampleMinDeg) do not.
     constexpr uint32_t kNoGiant = 0xFFFFFFFFu;
     auto link_round = [&](uint32_t stride, uint32_t skip_giant) {
         ++g->stats.launches;
@@ -524,7 +529,9 @@ static void cc_afforest(cgb_graph* g, bool weak)
         return giant;
     };
     uint32_t giant = kNoGiant;
-    if (g->max_degree >= kProbeMaxDeg) {
+    constexpr uint32_t kSampleMinDeg = 8, kSampleMeanWeak = 2, kSampleMeanSym = 10;
+    const uint64_t sample_edges = (uint64_t)V * (weak ? kSampleMeanWeak : kSampleMeanSym);
+    if (g->max_degree >= kProbeMaxDeg || (g->max_degree >= kSampleMinDeg && g->E >= sample_edges)) {
         if (timing) ktimer_begin(g, CGB_K_HOOK);
         link_round(1024, kNoGiant);
         link_round(32, kNoGiant);

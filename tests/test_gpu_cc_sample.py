@@ -51,3 +51,31 @@ def test_components(sizes, extra):
         np.testing.assert_array_equal(g.run(CC, 0, cg.make_options(flags=WEAK))[0], exp)
     with cg.Graph.from_csr(soff, sdst) as g:
         np.testing.assert_array_equal(g.run(CC, 0)[0], exp)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("sizes,degree", [
+    ([1 << 18], 8),                    # one component, no vertex of 64 edges
+    ([40_000, 40_000, 17, 5], 4),
+    ([12] * 9_000, 7),                 # none that a sample would find often
+    ([1 << 18], 1),                    # trees and cycles
+    ([4_300_000], 3),                  # rounds above 2^22 vertices
+])
+def test_components_without_hubs(sizes, degree):
+    rng = np.random.default_rng(len(sizes) + degree)
+    V = sum(sizes) + 3
+    base = np.concatenate([[0], np.cumsum(sizes)])
+    ids = rng.permutation(V)
+    src = np.concatenate([np.repeat(np.arange(b, b + n), degree) for b, n in zip(base, sizes)])
+    dst = np.concatenate([b + rng.integers(0, n, n * degree) for b, n in zip(base, sizes)])
+    keep = src != dst
+    src, dst = ids[src[keep]], ids[dst[keep]]
+    off, dd = csr(V, src, dst)
+    soff, sdst = csr(V, np.concatenate([src, dst]), np.concatenate([dst, src]))
+    longest = int(np.diff(soff.astype(np.int64)).max())
+    assert longest < 64
+    exp = O.cc(soff, sdst)
+    with cg.Graph.from_csr(off, dd) as g:
+        np.testing.assert_array_equal(g.run(CC, 0, cg.make_options(flags=WEAK))[0], exp)
+    with cg.Graph.from_csr(soff, sdst) as g:
+        np.testing.assert_array_equal(g.run(CC, 0)[0], exp)
