@@ -221,8 +221,18 @@ static void reset_level_counters(cgb_graph* g, int out)
 }
 
 // A graph of at most this many edges runs in the cluster from start to end,
-// all levels pushed.
-constexpr uint32_t kClusterWholeEdges = 1u << 20;
+// all levels pushed: no host round trips, but 16 of the SMs and no pulls.
+// Bounds of 2^18 / 2^19 / 2^20 edges, mean of 5 roots, us:
+//   Chung-Lu, 280 k edges                         200 / 107 / 107
+//   random, 2^13 vertices of 60, 490 k edges      105 / 119 / 119
+//   random, 2^18 vertices of 2, 524 k             448 / 260 / 257
+//   Chung-Lu, 546 k                               225 / 229 / 158
+//   random, 2^10 vertices of 554, 568 k            81 /  82 / 120
+//   random, 2^11 vertices of 444, 908 k            85 /  87 / 156
+//   RMAT-16, 955 k                                149 / 147 / 191
+//   random, 2^16 vertices of 15, 983 k            184 / 176 / 203
+//   random, 2^18 vertices of 4, 1049 k            290 / 302 / 284
+constexpr uint32_t kClusterWholeEdges = 1u << 19;
 
 void run_bfs(cgb_graph* g, uint32_t root, const cgb_options& o)
 {

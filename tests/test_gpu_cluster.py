@@ -220,3 +220,27 @@ def test_default_width_of_large_meshes(weight, factor):
         assert g.stats().sssp_delta == int(factor * mean / (dst.size / (rows * cols)))
     exp = O.bfs(off, dst, root) * (weight or 1) if weight != "mixed" else O.sssp(off, dst, w, root)
     np.testing.assert_array_equal(got, exp)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("V,edges,pulls", [
+    (2048, (1 << 19), False),      # the largest graph that runs in the cluster from start to end
+    (2048, (1 << 19) + 1, True),   # and the smallest that does not: dense, most of it is pulled
+    (2048, 900_000, True),
+    (1 << 18, (1 << 19) + 1, None),
+])
+def test_whole_runs_in_the_cluster(V, edges, pulls):
+    rng = np.random.default_rng(V + edges)
+    key = np.unique(np.concatenate([np.arange(V, dtype=np.int64) * V + (np.arange(V) + 1) % V,
+                                    rng.integers(0, V, 2 * edges) * V + rng.integers(0, V, 2 * edges)]))
+    key = key[key // V != key % V]
+    key = np.sort(rng.permutation(key)[:edges])
+    off, dd, w = csr(V, key // V, key % V, 3, 20)
+    assert dd.size == edges
+    roots = np.nonzero(np.diff(off.astype(np.int64)))[0][[0, 7, -1]]
+    with cg.Graph.from_csr(off, dd, w) as g:
+        for r in map(int, roots):
+            np.testing.assert_array_equal(g.run(BFS, r)[0], O.bfs(off, dd, r))
+            if pulls is not None:
+                assert (g.stats().pulls_bu > 0) == pulls
+            np.testing.assert_array_equal(g.run(SSSP, r)[0], O.sssp(off, dd, w, r))
