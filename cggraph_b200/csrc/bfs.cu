@@ -39,6 +39,7 @@ struct BfsTdOp {
     uint32_t cap;
     DevCounters* ctr;
     uint32_t t_edges = 0, t_maxdeg = 0;  // of the vertices this thread claimed
+    static constexpr bool kStaged = true;
     static constexpr int kBatch = 4;  // edge slots per lane visited together (push.cuh)
 
     __device__ __forceinline__ bool load(uint32_t v, uint32_t& s, uint32_t& d, uint32_t& m) const
@@ -126,6 +127,13 @@ __global__ void k_q2bm(const uint32_t* __restrict__ q, uint32_t n, uint32_t* bm)
     }
 }
 
+// Few staged items a warp: what the stage takes of an SM's memory L1 lacks,
+// from which lanes read the lists that they walk.  Every level pulled, 2^20
+// vertices of 30 edges: 256 items 2.40 ms, 128 1.91, 64 1.75, 32 1.76 (with
+// a CTA's finds appended together, without a stage, 1.78); RMAT-20 12.7,
+// 12.1, 11.3, 11.3 (10.5).
+constexpr uint32_t kBuStage = 64;
+
 // One bottom-up level.  Reads front (current frontier bitmap), writes
 // next (all words, so it needs no clearing) and the next queue.  A warp takes
 // one bitmap word per step, and warps share nothing between steps (finds are
@@ -178,7 +186,7 @@ __global__ void __launch_bounds__(kBlock) k_bfs_bu(uint32_t V, const uint32_t* _
                 found_cnt += enq[0];
                 mx = max(mx, deg);
                 const uint32_t it[1] = {v};
-                stage_append_n<1>(enq, it, qout, qlen, cap, &ctr->overflow);
+                stage_append_n<1, kBuStage>(enq, it, qout, qlen, cap, &ctr->overflow);
             }
         }
         if (lane == 0) {
@@ -196,7 +204,7 @@ __global__ void __launch_bounds__(kBlock) k_bfs_bu(uint32_t V, const uint32_t* _
         atomicMax(&s_td_maxdeg, mx);
     }
     __syncthreads();
-    stage_end(qout, qlen, cap, &ctr->overflow);
+    stage_end<kBuStage>(qout, qlen, cap, &ctr->overflow);
     if (threadIdx.x == 0 && s_bu_found) {
         atomicAdd(&ctr->medges, s_td_medges);
         atomicAdd(&ctr->found, s_bu_found);
@@ -302,7 +310,7 @@ void run_bfs(cgb_graph* g, uint32_t root, const cgb_options& o)
             if (timing) ktimer_begin(g, CGB_K_PULL);
             const uint32_t grid = grid_for((uint64_t)words * 32, kBlock, num_sms() * 16);
             ++g->stats.launches;
-            k_bfs_bu<<<grid, kBlock, 0, g->stream>>>(V, g->in_off, g->in_src, g->off, g->value, g->visited, front,
+            k_bfs_bu<<<grid, kBlock, stage_bytes(kBlock, kBuStage), g->stream>>>(V, g->in_off, g->in_src, g->off, g->value, g->visited, front,
                                                      next, level + 1, g->nz, g->q[out], &g->ctr->qlen[out], V,
                                                      g->ctr);
             if (timing) ktimer_end(g);

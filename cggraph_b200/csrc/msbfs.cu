@@ -369,7 +369,7 @@ __global__ void __launch_bounds__(kBlock) k_ms_bu_settle(MsBuArgs a)
 void ms_bottom_up(const MsBuArgs& a, cudaStream_t st, uint64_t* launches)
 {
     CGB_CUDA_TRY(cudaMemsetAsync(a.heavy_len, 0, 12, st));
-    k_ms_bu_light<<<grid_for(a.V, kBlock, num_sms() * 8), kBlock, 0, st>>>(a);
+    k_ms_bu_light<<<grid_for(a.V, kBlock, num_sms() * 8), kBlock, stage_bytes(kBlock), st>>>(a);
     k_ms_bu_warp<<<num_sms() * 8, kBlock, 0, st>>>(a);
     k_ms_bu_chunks<<<num_sms() * 8, kBlock, 0, st>>>(a);
     k_ms_bu_settle<<<num_sms() * 4, kBlock, 0, st>>>(a);

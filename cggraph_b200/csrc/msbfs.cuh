@@ -75,6 +75,7 @@ struct MsTdOp {
     uint32_t cap;
     DevCounters* ctr;
 
+    static constexpr bool kStaged = true;
     static constexpr int kBatch = 4;  // edge slots per lane visited together (push.cuh)
 
     __device__ __forceinline__ bool load(uint32_t v, uint32_t& s, uint32_t& d, uint32_t& m) const

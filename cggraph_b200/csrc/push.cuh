@@ -110,32 +110,46 @@ __device__ __forceinline__ void warp_append_n(const bool (&pred)[N], const uint3
 // queued at its L2 slice (1.5 G same-address atomics a second on a B200): a
 // BFS level of 4.3 M edges with 1.4 M finds spent most of its 0.24 ms there.
 // stage_begin comes before a CTA barrier, stage_end after one, both called by
-// every thread; stage_append_n is warp-collective.
-constexpr uint32_t kStage = 256;         // items per warp
+// every thread; stage_append_n is warp-collective.  The items are in dynamic
+// shared memory, stage_bytes(threads, kItems) of it, kItems per warp.
+constexpr uint32_t kStage = 128;
 constexpr uint32_t kStageWarps = 512 / 32;  // largest CTA of the push kernels
 
-__shared__ uint32_t s_stage[kStageWarps][kStage];
+extern __shared__ uint32_t s_stage[];
 __shared__ uint32_t s_staged[kStageWarps];
+
+constexpr uint32_t stage_bytes(uint32_t threads, uint32_t items = kStage) { return threads / 32 * items * 4; }
+
+// An op that stages its finds declares `static constexpr bool kStaged = true`.
+template <class T, class = void>
+struct op_staged {
+    static constexpr bool value = false;
+};
+template <class T>
+struct op_staged<T, std::void_t<decltype(T::kStaged)>> {
+    static constexpr bool value = T::kStaged;
+};
 
 __device__ __forceinline__ void stage_begin()
 {
     if (threadIdx.x < kStageWarps) s_staged[threadIdx.x] = 0;
 }
 
+template <uint32_t kItems>
 __device__ __forceinline__ void stage_write(uint32_t warp, uint32_t n, uint32_t base, uint32_t* q, uint32_t cap,
                                             uint32_t* overflow)
 {
     for (uint32_t i = lane_id(); i < n; i += 32) {
-        if (base + i < cap) q[base + i] = s_stage[warp][i];
+        if (base + i < cap) q[base + i] = s_stage[warp * kItems + i];
         else atomicOr(overflow, 1u);
     }
 }
 
-template <int N>
+template <int N, uint32_t kItems = kStage>
 __device__ __forceinline__ void stage_append_n(const bool (&pred)[N], const uint32_t (&item)[N], uint32_t* q,
                                                uint32_t* ctr, uint32_t cap, uint32_t* overflow)
 {
-    static_assert(32 * N <= kStage, "one step must fit");
+    static_assert(32 * N <= kItems, "one step must fit");
     const uint32_t warp = threadIdx.x >> 5, lane = lane_id();
     uint32_t m[N], total = 0;
 #pragma unroll
@@ -146,22 +160,23 @@ __device__ __forceinline__ void stage_append_n(const bool (&pred)[N], const uint
     if (total == 0) return;
     uint32_t have = s_staged[warp];
     __syncwarp();
-    if (have + total > kStage) {
+    if (have + total > kItems) {
         uint32_t base = 0;
         if (lane == 0) base = atomicAdd(ctr, have);
-        stage_write(warp, have, __shfl_sync(0xffffffffu, base, 0), q, cap, overflow);
+        stage_write<kItems>(warp, have, __shfl_sync(0xffffffffu, base, 0), q, cap, overflow);
         have = 0;
         __syncwarp();
     }
     if (lane == 0) s_staged[warp] = have + total;
 #pragma unroll
     for (int i = 0; i < N; i++) {
-        if (pred[i]) s_stage[warp][have + __popc(m[i] & lanemask_lt())] = item[i];
+        if (pred[i]) s_stage[warp * kItems + have + __popc(m[i] & lanemask_lt())] = item[i];
         have += __popc(m[i]);
     }
     __syncwarp();
 }
 
+template <uint32_t kItems = kStage>
 __device__ __forceinline__ void stage_end(uint32_t* q, uint32_t* ctr, uint32_t cap, uint32_t* overflow)
 {
     __shared__ uint32_t s_base[kStageWarps];
@@ -175,7 +190,7 @@ __device__ __forceinline__ void stage_end(uint32_t* q, uint32_t* ctr, uint32_t c
         if (lane < warps) s_base[lane] = base + incl - n;
     }
     __syncthreads();
-    stage_write(warp, s_staged[warp], s_base[warp], q, cap, overflow);
+    stage_write<kItems>(warp, s_staged[warp], s_base[warp], q, cap, overflow);
 }
 
 // Chunk descriptors (v, 0 .. nch - 1) of every lane's vertex, written by the
@@ -450,13 +465,14 @@ inline void launch_push_blk(cgb_graph* g, const uint32_t* qin, uint32_t nin, con
                             uint32_t ctas, uint32_t big_deg, uint32_t chunk)
 {
     const uint32_t grid = grid_for(nin, kBlk, ctas);
+    constexpr uint32_t smem = op_staged<Op>::value ? stage_bytes(kBlk) : 0;
     if (identity)
-        k_push_binned<Op, true, kBlk><<<grid, kBlk, 0, g->stream>>>(qin, nin, op, g->chunk_q, &g->ctr->chunk_len,
-                                                                     g->chunk_cap, &g->ctr->overflow, big_deg, chunk);
+        k_push_binned<Op, true, kBlk><<<grid, kBlk, smem, g->stream>>>(
+            qin, nin, op, g->chunk_q, &g->ctr->chunk_len, g->chunk_cap, &g->ctr->overflow, big_deg, chunk);
     else
-        k_push_binned<Op, false, kBlk><<<grid, kBlk, 0, g->stream>>>(qin, nin, op, g->chunk_q, &g->ctr->chunk_len,
-                                                                      g->chunk_cap, &g->ctr->overflow, big_deg, chunk);
-    k_push_chunks<Op, kBlk><<<ctas, kBlk, 0, g->stream>>>(g->chunk_q, &g->ctr->chunk_len, g->chunk_cap, op, chunk);
+        k_push_binned<Op, false, kBlk><<<grid, kBlk, smem, g->stream>>>(
+            qin, nin, op, g->chunk_q, &g->ctr->chunk_len, g->chunk_cap, &g->ctr->overflow, big_deg, chunk);
+    k_push_chunks<Op, kBlk><<<ctas, kBlk, smem, g->stream>>>(g->chunk_q, &g->ctr->chunk_len, g->chunk_cap, op, chunk);
 }
 
 // Expansion variants of launch_push: the size rule (chunk every list of 32

@@ -50,6 +50,7 @@ struct SsspOp {
     uint32_t* far_bm;
     DevCounters* ctr;
     uint32_t t_newfar = 0, t_touched = 0, t_edges = 0, t_maxdeg = 0;  // this thread's counts
+    static constexpr bool kStaged = true;
     static constexpr int kBatch = 4;
 
     __device__ __forceinline__ bool load(uint32_t v, uint32_t& s, uint32_t& d, uint32_t& m) const
@@ -520,7 +521,8 @@ static void sssp_loop(cgb_graph* g, uint32_t root, uint32_t delta, const cgb_opt
             SsspDenseOp<kHasW> op{g->off, g->dst, g->w, g->value};
             launch_push(g, g->q[cur], (uint32_t)nnear, op, false);
             ++g->stats.launches;
-            k_sssp_dense_scan<<<grid_for(div_up(V, 4), kBlock, num_sms() * 8), kBlock, 0, g->stream>>>(
+            k_sssp_dense_scan<<<grid_for(div_up(V, 4), kBlock, num_sms() * 8), kBlock, stage_bytes(kBlock),
+                                g->stream>>>(
                 V, g->value, g->stamp, (uint32_t)std::min<uint64_t>(thr, kValueMax), g->nz, g->off, far_bm,
                 g->q[out], &g->ctr->qlen[out], V, g->ctr);
         } else {
