@@ -416,7 +416,9 @@ __global__ void __launch_bounds__(kBlk) k_push_binned(const uint32_t* __restrict
 
 // One warp per chunk descriptor, grid-stride over the chunk queue: warps
 // run ahead of one another, so that a few hundred edges per chunk keep many
-// chains of loads in flight.  Ops without batched visits take a chunk with the
+// chains of loads in flight.  With no more chunks than CTAs a chunk is cut once
+// more, over as many warps as a CTA has (10 levels of a 14 k-vertex Chung-Lu
+// graph: 10 us a launch otherwise, 6 cut).  Ops without batched visits take a chunk with the
 // whole CTA: one edge per lane at a time, a warp's chunk of 1024 edges is 32
 // chains of dependent loads one after the other.  Label propagation, a chunk
 // by a warp / by a CTA: RMAT-20 1.37 / 0.97 ms (and 6 rounds instead of 5: the
@@ -426,24 +428,25 @@ __global__ void __launch_bounds__(kBlk) k_push_chunks(const uint2* __restrict__ 
                                                         uint32_t chunk_cap, Op op, uint32_t chunk)
 {
     const uint32_t n = min(*chunk_len, chunk_cap);
-    if (blockIdx.x >= n) return;
+    constexpr bool kByCta = op_batch<Op>::value == 1;
+    const uint32_t parts = kByCta || n > gridDim.x ? 1 : min((uint32_t)kBlk / 32, chunk / 32);
+    if (blockIdx.x >= n * parts) return;
     op.block_begin();
     __syncthreads();
-    constexpr bool kByCta = op_batch<Op>::value == 1;
-    // (warps: CTAs take the first chunks one warp each before any takes a second)
-    const uint32_t c0 = kByCta ? blockIdx.x : (threadIdx.x >> 5) * gridDim.x + blockIdx.x;
+    // (warps: CTAs take the first pieces one warp each before any takes a second)
+    const uint32_t p0 = kByCta ? blockIdx.x : (threadIdx.x >> 5) * gridDim.x + blockIdx.x;
     const uint32_t step = kByCta ? gridDim.x : gridDim.x * (kBlk / 32);
-    for (uint32_t c = c0; c < n; c += step) {
-        const uint2 d = chunk_q[c];
+    for (uint32_t p = p0; p < n * parts; p += step) {
+        const uint2 d = chunk_q[p % n];
         uint32_t start, deg, msg;
         if (!op.load(d.x, start, deg, msg)) continue;
-        const uint32_t cs = d.y * chunk, ce = min(deg, cs + chunk);
+        const uint32_t len = chunk / parts, cs = d.y * chunk + p / n * len, ce = min(deg, cs + len);
         if constexpr (kByCta) {
             for (uint32_t k = cs; k < ce; k += kBlk) {
                 const uint32_t i = k + threadIdx.x;
                 op.edge(i < ce, i < ce ? start + i : 0u, msg);
             }
-        } else {
+        } else if (cs < ce) {
             warp_range(op, start + cs, start + ce, msg);
         }
     }

@@ -45,3 +45,22 @@ def test_push_edges(first, second, tuning):
         s = g.stats()
         assert s.reached == np.count_nonzero(exp_s != cg.VALUE_MAX)
         assert s.traversed_edges == int(np.diff(off.astype(np.int64))[exp_s != cg.VALUE_MAX].sum())
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("first,second", [
+    (1, [40_000]),                          # fewer chunks than CTAs: each is cut over a CTA's warps
+    (90, [255, 256, 257, 288, 289, 31, 32, 33]),
+    (1_183, [33, 64, 100, 256]),            # about as many chunks as CTAs (8 a SM), one below, one above
+    (1_184, [256]),
+    (1_185, [257]),
+])
+@pytest.mark.parametrize("block", [128, 256, 512])
+def test_few_chunks(first, second, block):
+    off, dst, w = fan(first, second, first + len(second))
+    exp_b, exp_s = O.bfs(off, dst, 0), O.sssp(off, dst, w, 0)
+    with cg.Graph.from_csr(off, dst, w) as g:
+        g.set_tuning({"persist_enter": 0, "cluster_enter": 0, "push_block": block})
+        np.testing.assert_array_equal(g.run(BFS, 0, cg.make_options(schedule=2, variant=3))[0], exp_b)
+        np.testing.assert_array_equal(g.run(SSSP, 0)[0], exp_s)
+        np.testing.assert_array_equal(g.run_batch(BFS, [0, 1])[0][0], exp_b)
