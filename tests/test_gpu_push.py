@@ -64,3 +64,21 @@ def test_few_chunks(first, second, block):
         np.testing.assert_array_equal(g.run(BFS, 0, cg.make_options(schedule=2, variant=3))[0], exp_b)
         np.testing.assert_array_equal(g.run(SSSP, 0)[0], exp_s)
         np.testing.assert_array_equal(g.run_batch(BFS, [0, 1])[0][0], exp_b)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("block", [128, 256, 512])
+def test_binned_tiers(block):
+    """A frontier above 2^19 vertices keeps the degree tiers: lists of up to 31 edges packed, up to push_big_deg - 1 by
+    a warp, longer ones in chunks of push_chunk edges; lists at each bound, with the smallest values of both."""
+    off, dst, w = fan(530_000, [1] * 60 + [31, 32, 33, 64, 127, 128, 129, 255, 256, 257, 400, 513], 9)
+    exp_b, exp_s = O.bfs(off, dst, 0), O.sssp(off, dst, w, 0)
+    with cg.Graph.from_csr(off, dst, w) as g:
+        g.set_tuning({"persist_enter": 0, "cluster_enter": 0, "push_block": block, "push_big_deg": 128,
+                      "push_chunk": 256})
+        np.testing.assert_array_equal(g.run(BFS, 0, cg.make_options(schedule=2, variant=3))[0], exp_b)
+        for alpha in (0, 1024):  # every round pushed, every round dense
+            g.set_tuning({"sssp_dense_alpha": alpha, "persist_enter": 0, "cluster_enter": 0, "push_block": block,
+                          "push_big_deg": 128, "push_chunk": 256})
+            np.testing.assert_array_equal(g.run(SSSP, 0, cg.make_options(sssp_delta=1 << 20))[0], exp_s)
+        np.testing.assert_array_equal(g.run_batch(BFS, [0, 5])[0][0], exp_b)
