@@ -487,7 +487,9 @@ static void cc_afforest(cgb_graph* g, bool weak)
     // 0.45 / 0.27, 0.70 / 0.31 and 0.80 / 0.32 ms, 2^18 of 16 0.46 / 0.18;
     // symmetric, mean length 8 / 10 / 12 / 14, 1.0 / 1.2, 0.39 / 0.22, 0.73 /
     // 0.20 and 0.52 / 0.20, 2^18 of 32 0.56 / 0.14.  Meshes (lists below
-    // kSampleMinDeg) do not.
+    // kSampleMinDeg) do not.  Below kSampleMinV vertices the sample costs more
+    // (its launches, 10 to 25 us) than it saves: weak, RMAT-8 0.078 / 0.101,
+    // RMAT-12 0.090 / 0.103, RMAT-13 0.109 / 0.104, RMAT-14 0.127 / 0.112 ms.
     constexpr uint32_t kNoGiant = 0xFFFFFFFFu;
     auto link_round = [&](uint32_t stride, uint32_t skip_giant) {
         ++g->stats.launches;
@@ -529,9 +531,10 @@ static void cc_afforest(cgb_graph* g, bool weak)
         return giant;
     };
     uint32_t giant = kNoGiant;
-    constexpr uint32_t kSampleMinDeg = 8, kSampleMeanWeak = 2, kSampleMeanSym = 10;
+    constexpr uint32_t kSampleMinV = 1u << 14, kSampleMinDeg = 8, kSampleMeanWeak = 2, kSampleMeanSym = 10;
     const uint64_t sample_edges = (uint64_t)V * (weak ? kSampleMeanWeak : kSampleMeanSym);
-    if (g->max_degree >= kProbeMaxDeg || (g->max_degree >= kSampleMinDeg && g->E >= sample_edges)) {
+    if (V >= kSampleMinV &&
+        (g->max_degree >= kProbeMaxDeg || (g->max_degree >= kSampleMinDeg && g->E >= sample_edges))) {
         if (timing) ktimer_begin(g, CGB_K_HOOK);
         link_round(1024, kNoGiant);
         link_round(32, kNoGiant);

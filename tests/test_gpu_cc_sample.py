@@ -79,3 +79,23 @@ def test_components_without_hubs(sizes, degree):
         np.testing.assert_array_equal(g.run(CC, 0, cg.make_options(flags=WEAK))[0], exp)
     with cg.Graph.from_csr(soff, sdst) as g:
         np.testing.assert_array_equal(g.run(CC, 0)[0], exp)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("V", [(1 << 14) - 1, 1 << 14, (1 << 14) + 1])
+def test_components_at_the_smallest_sampled_graph(V):
+    for hub in (0, 200):
+        rng = np.random.default_rng(V + hub)
+        src = np.concatenate([rng.integers(0, V, 2 * V), np.zeros(hub, np.int64)])
+        dst = np.concatenate([rng.integers(0, V, 2 * V), rng.integers(0, V, hub)])
+        keep = src != dst
+        off, dd = csr(V, src[keep], dst[keep])
+        soff, sdst = csr(V, np.concatenate([src[keep], dst[keep]]), np.concatenate([dst[keep], src[keep]]))
+        exp, launches = O.cc(soff, sdst), []
+        with cg.Graph.from_csr(off, dd) as g:
+            np.testing.assert_array_equal(g.run(CC, 0, cg.make_options(flags=WEAK))[0], exp)
+            launches.append(g.stats().launches)
+        if hub:
+            assert launches[0] == (8 if V < 1 << 14 else 11)
+        with cg.Graph.from_csr(soff, sdst) as g:
+            np.testing.assert_array_equal(g.run(CC, 0)[0], exp)
