@@ -240,6 +240,8 @@ static void reset_level_counters(cgb_graph* g, int out)
 //   RMAT-16, 955 k                                149 / 147 / 191
 //   random, 2^16 vertices of 15, 983 k            184 / 176 / 203
 //   random, 2^18 vertices of 4, 1049 k            290 / 302 / 284
+// A list beyond kClusterList ends the loop, and the run would come back to it
+// for nothing: such a graph takes the rule for small frontiers.
 constexpr uint32_t kClusterWholeEdges = 1u << 19;
 
 void run_bfs(cgb_graph* g, uint32_t root, const cgb_options& o)
@@ -346,7 +348,7 @@ void run_bfs(cgb_graph* g, uint32_t root, const cgb_options& o)
                                     : (double)scout > (double)edges_to_check / alpha;
         // small frontiers far from the switch point: run levels on the device;
         // a small graph's whole run, in the cluster
-        const bool whole = g->E <= kClusterWholeEdges && !bottom_up;
+        const bool whole = g->E <= kClusterWholeEdges && g->max_degree <= kClusterList && !bottom_up;
         const bool far_off = !heur && (double)scout * alpha * 4.0 <= (double)edges_to_check;
         const uint64_t scout_exit = (uint64_t)std::max(0.0, (double)edges_to_check / alpha / 4.0);
         const uint32_t max_levels = (uint32_t)std::min<uint64_t>(max_iters - iters, 1u << 20);

@@ -46,6 +46,7 @@ constexpr uint32_t kClPiece = 8;     // edges per entry
 constexpr uint32_t kClFirst = 0x80;  // marks a vertex's first entry,
 constexpr uint32_t kClSingle = 0x40; // and its only one
 constexpr int kClBatch = 4;
+static_assert(kClQueue * kClPiece == kClusterList, "the longest list that fits a queue");
 
 // What a CTA tells the others about the level it has built.  `word` packs
 // the entries (at most kClQueue, so that the cluster's sum stays below 2^20)

@@ -37,6 +37,9 @@ constexpr uint32_t kClusterEnterEdges = 1u << 15, kClusterExitEdges = 1u << 16;
 // cluster: the split reads every far distance (RMAT-24 with a bucket width of
 // 16, millions of far vertices: 10.1 ms in the cluster, 4.0 ms without).
 constexpr uint32_t kClusterFar = 1u << 17;
+// Edges of the longest list that a CTA's queue holds (8192 pieces of 8); a
+// longer one spills, and the loop ends with the level that found it.
+constexpr uint32_t kClusterList = 1u << 16;
 
 // Host-visible state of a device-resident loop.
 struct PersistState {

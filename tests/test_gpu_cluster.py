@@ -244,3 +244,25 @@ def test_whole_runs_in_the_cluster(V, edges, pulls):
             if pulls is not None:
                 assert (g.stats().pulls_bu > 0) == pulls
             np.testing.assert_array_equal(g.run(SSSP, r)[0], O.sssp(off, dd, w, r))
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("hub", [65_535, 65_536, 65_537, 150_000])
+def test_list_as_long_as_a_queue(hub):
+    """A hub with as many edges as a CTA's queue holds, and more, found from a leaf: the loop is asked once for a list
+    that it cannot hold, in a graph small enough to run there from start to end."""
+    V = hub + 1
+    src = np.concatenate([np.zeros(hub, np.int64), np.arange(1, V)])
+    dst = np.concatenate([np.arange(1, V), np.zeros(hub, np.int64)])
+    off, dd, w = csr(V, src, dst, 4, 50)
+    assert dd.size <= 1 << 19
+    with cg.Graph.from_csr(off, dd, w) as g:
+        for root in (5, 0):
+            np.testing.assert_array_equal(g.run(BFS, root)[0], O.bfs(off, dd, root))
+            np.testing.assert_array_equal(g.run(SSSP, root)[0], O.sssp(off, dd, w, root))
+        g.run(BFS, 5)
+        launches = g.stats().launches
+        g.set_tuning({"cluster_enter": 0})
+        g.run(BFS, 5)
+        # the loop's launch stands for the root's level (three launches) and is not followed by another
+        assert launches <= (g.stats().launches if hub > 1 << 16 else 2)
