@@ -99,10 +99,13 @@ __device__ __forceinline__ void pr_row_out(const PrIter& a, uint32_t r, double s
 }
 
 // One warp per slice: in step j every lane loads its row's j-th source (one
-// coalesced 128-byte load per warp) and gathers that contribution; kU steps
-// (cgb_tuning.pr_unroll) are issued before they are summed, in j order, so
-// each lane keeps kU gathers in flight.  Padding slots and the masked steps
-// of the last batch name vertex V, whose contribution is 0.
+// coalesced 128-byte load per warp) and gathers that contribution; the steps
+// go in batches of kU (cgb_tuning.pr_unroll), whose gathers are issued before
+// they are summed, in j order, as far as the registers reach: 32 (40 with
+// hints) do not hold 16 pending doubles, so at kU = 16 the compiler splits
+// the batch, and the three unrolls of a variant differ less than their names.
+// Padding slots and the masked steps of the last batch name vertex V, whose
+// contribution is 0.
 // (The plain kernel is held to 32 registers, 8 CTAs an SM: at 34 registers, 6
 // CTAs, the 4800 x 5000 grid took 6.77 instead of 6.34 ms.  The hinted one
 // spills there: it has 6.)
@@ -115,7 +118,6 @@ __global__ void __launch_bounds__(kBlock, kHint ? 6 : 8) k_pr_pull(PrIter a)
     uint64_t pol_hot, pol_cold;
     asm volatile("createpolicy.fractional.L2::evict_last.b64 %0, 1.0;" : "=l"(pol_hot));
     asm volatile("createpolicy.fractional.L2::evict_first.b64 %0, 1.0;" : "=l"(pol_cold));
-    asm volatile("griddepcontrol.launch_dependents;");
     asm volatile("griddepcontrol.wait;" ::: "memory");
     for (uint32_t s = blockIdx.x * (kBlock / 32) + (threadIdx.x >> 5); s < nslices; s += nwarps) {
         const uint32_t len = a.slice_len[s];
@@ -140,6 +142,7 @@ __global__ void __launch_bounds__(kBlock, kHint ? 6 : 8) k_pr_pull(PrIter a)
             if (r < a.n_rows && !((a.long_bm[rs] >> lane) & 1u)) pr_row_out(a, r, acc);
         }
     }
+    asm volatile("griddepcontrol.launch_dependents;");
 }
 
 // Adds the segments of the long rows: one CTA per hub row (more than
@@ -150,7 +153,6 @@ __global__ void __launch_bounds__(kBlock) k_pr_combine(PrIter a, const uint32_t*
                                                        const uint32_t* __restrict__ seg_base, uint32_t n,
                                                        const uint32_t* __restrict__ hubs, uint32_t n_hubs)
 {
-    asm volatile("griddepcontrol.launch_dependents;");
     const uint32_t lane = lane_id();
     if (blockIdx.x < n_hubs) {
         __shared__ double s_part[kBlock / 32];
@@ -167,6 +169,7 @@ __global__ void __launch_bounds__(kBlock) k_pr_combine(PrIter a, const uint32_t*
             t = warp_sum(lane < kBlock / 32 ? s_part[lane] : 0.0);
             if (lane == 0 && rows[i] < a.n_rows) pr_row_out(a, rows[i], t);
         }
+    asm volatile("griddepcontrol.launch_dependents;");
         return;
     }
     const uint32_t i = ((blockIdx.x - n_hubs) * kBlock + threadIdx.x) / 8;
@@ -183,6 +186,7 @@ __global__ void __launch_bounds__(kBlock) k_pr_combine(PrIter a, const uint32_t*
     t += __shfl_xor_sync(0xffffffffu, t, 2);
     t += __shfl_xor_sync(0xffffffffu, t, 4);
     if (mine && (lane & 7u) == 0 && row < a.n_rows) pr_row_out(a, row, t);
+    asm volatile("griddepcontrol.launch_dependents;");
 }
 
 // Back to the caller's vertex ids: out[v] = pr[rank[v]].
@@ -235,7 +239,13 @@ void run_pr(cgb_graph* g, uint32_t iters, const cgb_options& o)
         if (timing) ktimer_begin(g, CGB_K_PR);
         ++g->stats.launches;
         // programmatic dependent launches: a kernel's CTAs are placed while the last
-        // ones of the kernel before it run, and wait for its results there
+        // ones of the kernel before it run, and wait for its results there.  They
+        // may be placed only once a CTA's own work is done: placed earlier, the
+        // waiting CTAs of a grid that fits the machine at once crowd where there is
+        // room, and the next iteration runs with some SMs full and others idle
+        // (random graph, 2^17 vertices of 30 edges, 20 iterations: 0.60 ms placed
+        // at the start of a kernel, 0.36 at its end, 0.41 without such launches;
+        // RMAT-16 0.225, 0.194, 0.297; RMAT-24 13.64, 13.62; 4900^2 grid 6.5 each).
         cudaLaunchAttribute attr[1];
         attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
         attr[0].val.programmaticStreamSerializationAllowed = 1;

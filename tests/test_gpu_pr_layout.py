@@ -43,3 +43,25 @@ def test_row_bounds(V, degrees, extra, iters):
     # a sum of at most V terms, all positive: relative error below V * 2^-53 per iteration on either side
     np.testing.assert_allclose(got, exp, rtol=2 * iters * V * 2.0 ** -53 + 1e-14, atol=0)
     np.testing.assert_array_equal(got, again)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("V,degree,hub", [(5, 1, 0), (4_096, 8, 0), (131_072, 30, 0), (100_000, 3, 90_000)])
+def test_overlapped_iterations(V, degree, hub):
+    """Each iteration's kernels are placed while those before them run: many iterations of graphs that fit the machine
+    at once, with and without long rows, against the oracle and against launches without the overlap."""
+    rng = np.random.default_rng(V)
+    src = np.concatenate([np.repeat(np.arange(V), degree), 1 + rng.integers(0, V - 1, hub)])
+    dst = np.concatenate([rng.integers(0, V, V * degree), np.zeros(hub, np.int64)])
+    key = np.unique(src[src != dst].astype(np.int64) * V + dst[src != dst])
+    off = np.zeros(V + 1, np.uint32)
+    off[1:] = np.cumsum(np.bincount(key // V, minlength=V))
+    dd = (key % V).astype(np.uint32)
+    iters = 60
+    exp = O.pagerank(off, dd, iters)
+    with cg.Graph.from_csr(off, dd) as g:
+        got = [g.run(PR, iters)[0] for _ in range(3)]
+        plain, _ = g.run(PR, iters, cg.make_options(flags=0x1))  # timed launches are not overlapped
+    np.testing.assert_allclose(plain, exp, rtol=2 * iters * V * 2.0 ** -53 + 1e-14, atol=0)
+    for x in got:
+        np.testing.assert_array_equal(x, plain)
