@@ -36,7 +36,7 @@ struct MsBuffers {
 MsBuffers* ms_buffers_alloc(uint32_t V, uint64_t E);
 void ms_buffers_free(MsBuffers* b);
 
-// One bottom-up level (three kernels, see msbfs.cu).
+// One bottom-up level (four kernels, see msbfs.cu).
 struct MsBuArgs {
     uint32_t V;
     const uint32_t* in_off;
