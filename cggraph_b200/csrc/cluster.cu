@@ -39,7 +39,7 @@ constexpr int kClThreads = 512;
 constexpr int kClWarps = kClThreads / 32;
 constexpr unsigned long long kClWaitNs = 1000000000ull;  // a level's counts take longer: the loop gives up
 constexpr uint32_t kClSpins = 1u << 28;  // and after so many polls, whatever the clock says
-constexpr uint32_t kClPollNs = 10000, kClEarly = 1u << 16;
+constexpr uint32_t kClPollNs = 10000, kClEarly = 64;
 constexpr uint32_t kClMaxCtas = 16;
 constexpr uint32_t kClQueue = 8192;  // entries per CTA and buffer
 constexpr uint32_t kClPiece = 8;     // edges per entry
@@ -170,17 +170,28 @@ __device__ __forceinline__ void stage(uint32_t (&x)[N])
 }
 
 // One poll of phase `parity` of an mbarrier of this CTA.  It may suspend the
-// thread until the phase completes, kClPollNs at most.
+// thread until the phase completes, for a time that the device chooses or
+// (late) kClPollNs at most.
+template <bool kLate>
 __device__ __forceinline__ bool cl_poll(uint32_t mbar, uint32_t parity)
 {
     uint32_t done;
-    asm volatile(
-        "{\n\t.reg .pred p;\n\t"
-        "mbarrier.try_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], %2, %3;\n\t"
-        "selp.u32 %0, 1, 0, p;\n\t}"
-        : "=r"(done)
-        : "r"(mbar), "r"(parity), "r"(kClPollNs)
-        : "memory");
+    if (kLate)
+        asm volatile(
+            "{\n\t.reg .pred p;\n\t"
+            "mbarrier.try_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], %2, %3;\n\t"
+            "selp.u32 %0, 1, 0, p;\n\t}"
+            : "=r"(done)
+            : "r"(mbar), "r"(parity), "r"(kClPollNs)
+            : "memory");
+    else
+        asm volatile(
+            "{\n\t.reg .pred p;\n\t"
+            "mbarrier.try_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], %2;\n\t"
+            "selp.u32 %0, 1, 0, p;\n\t}"
+            : "=r"(done)
+            : "r"(mbar), "r"(parity)
+            : "memory");
     return done != 0;
 }
 
@@ -191,7 +202,7 @@ __device__ __forceinline__ bool cl_wait_late(uint32_t mbar, uint32_t parity, uns
     unsigned long long t0, t;
     asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t0));
     for (uint32_t spin = 0; spin < kClSpins; spin++) {
-        if (cl_poll(mbar, parity)) return true;
+        if (cl_poll<true>(mbar, parity)) return true;
         asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t));
         if (t - t0 > wait_ns) return false;
     }
@@ -199,14 +210,14 @@ __device__ __forceinline__ bool cl_wait_late(uint32_t mbar, uint32_t parity, uns
 }
 
 // Waits for phase `parity` of an mbarrier of this CTA; false after kClEarly
-// polls (0.7 s if each is suspended) and wait_ns.  The clock is not looked at
-// while the early polls run: where it was, a level took 2 to 3 % longer (1200
-// x 1250 grid BFS 6.91 ms without a limit by the clock, 7.01 as it is, 7.13
-// with a look every 64 polls).
+// polls and wait_ns.  The clock is not looked at, and no time is given to a
+// poll, while the early polls run: 1200 x 1250 grid BFS 6.88 ms without a
+// limit by the clock, 6.94 as it is, 6.97 with a time given to every poll,
+// 7.1 with a look at the clock every 64 polls.
 __device__ __forceinline__ bool cl_wait(uint32_t mbar, uint32_t parity, unsigned long long wait_ns)
 {
     bool done = false;
-    for (uint32_t spin = 0; !done && spin < kClEarly; spin++) done = cl_poll(mbar, parity);
+    for (uint32_t spin = 0; !done && spin < kClEarly; spin++) done = cl_poll<false>(mbar, parity);
     return done || cl_wait_late(mbar, parity, wait_ns);
 }
 
